@@ -55,7 +55,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     units = [
         ("kernels_fast.o", "kernels.cu", ["-DOPTX_NS=fast", "-DOPTX_EXACT=0"]),
         ("kernels_exact.o", "kernels.cu", ["-DOPTX_NS=exact", "-DOPTX_EXACT=1", "-fmad=false"]),
-        ("kernels_approx.o", "kernels.cu", ["-DOPTX_NS=approx", "-DOPTX_EXACT=0", "--use_fast_math"]),
+        ("kernels_approx.o", "kernels.cu", ["-DOPTX_NS=approx", "-DOPTX_EXACT=0", "-DOPTX_APPROX=1", "--use_fast_math"]),
         ("capi.o", "capi.cu", []),
     ]
     cmds, objs = [], []

@@ -96,6 +96,20 @@ int check_params(const optx_params* p, const optx_faces* f) {
   return OPTX_OK;
 }
 
+// True where the kernels' branch-free quotients are exact: the box exit's
+// numerators (+-h - p) are then 0 or at least 2^-66, its quotients normal, and the
+// Fresnel products in range. The bounds are far outside any detector (1e-12 to
+// 1e12 mm, indices 0.001 to 1000); records beyond them are transported with the IEEE
+// divisions, at the speed of those.
+bool ordinary_params(const optx_params& p) {
+  auto in = [](float v, float lo, float hi) { return v >= lo && v <= hi; };
+  bool ok = true;
+  for (float h : {p.hx, p.hy, p.hz}) ok = ok && in(h, 0x1p-40f, 0x1p40f);
+  for (float n : {p.n_scint, p.n_det, p.n_out}) ok = ok && in(n, 0x1p-10f, 0x1p10f);
+  for (float x : {p.src_x, p.src_y, p.src_z}) ok = ok && in(x, -kFarCoordinate, kFarCoordinate);
+  return ok;
+}
+
 // SimParams (+ optional per-face surfaces) -> the kernels' 112-byte record. The
 // derived quantities use the reference's float expressions: inv_speed =
 // n_scint / c (transport.hpp:74), eta = n1 / n2 and eta * eta (fresnel.hpp:32-33).
@@ -142,6 +156,7 @@ DevParams make_dev_params(const optx_params& p, const optx_faces* f) {
   volatile float two_hx = 2.0f * p.hx, two_hy = 2.0f * p.hy;
   d.inv2hx = 1.0f / two_hx;
   d.inv2hy = 1.0f / two_hy;
+  d.flags = ordinary_params(p) ? kOrdinary : 0u;
   return d;
 }
 
@@ -331,6 +346,10 @@ __global__ void genstep_records_kernel(const optx_genstep* __restrict__ gs, uint
 #pragma unroll
   for (int i = 0; i < 8; ++i) ok = ok && isfinite(v[i]);
   if (!ok) atomicOr(error, 1u);
+  bool far = false;
+#pragma unroll
+  for (int i = 0; i < 7; ++i) far = far || (i != 3 && fabsf(v[i]) > kFarCoordinate);
+  if (far) atomicOr(error, kFarGenstep);
   const uint32_t ev = ok ? s.event : 0u;
   DevParams d = phys[ev];
   d.source = kSourceSegment;
@@ -559,7 +578,11 @@ int engine_upload_args(optx_engine* e, int mode, int batch, int grid, cudaGraphC
   a.graph_handle = h;
   // Watchdog: no warp can iterate more than (photons + queue) x (max_steps + 2) times.
   uint32_t max_steps = 0;
-  for (const DevParams& p : e->h_params) max_steps = std::max(max_steps, p.max_steps);
+  a.flags = ~0u;
+  for (const DevParams& p : e->h_params) {
+    max_steps = std::max(max_steps, p.max_steps);
+    a.flags &= p.flags;
+  }
   a.iter_cap = (static_cast<unsigned long long>(e->total) + e->qcap + 64ull) *
                    (static_cast<unsigned long long>(max_steps) + 2ull) + 4096ull;
   // Every photon of a wave steps at least once, so a run needs at most about
@@ -1415,7 +1438,6 @@ static bool same_step_physics(DevParams a, DevParams b) {
     d->tau = 0.0f;
     d->src_x = d->src_y = d->src_z = 0.0f;
     d->source = 0u;
-    d->pad2 = 0u;
   }
   return std::memcmp(&a, &b, sizeof(DevParams)) == 0;
 }
@@ -1534,6 +1556,8 @@ int optx_engine_set_gensteps(optx_engine* e, const optx_params* events, const op
       if (!std::isfinite(f)) return fail(OPTX_ERR_INVALID_ARGUMENT, "genstep coordinates and times must be finite");
     if (gs.t1 < gs.t0) return fail(OPTX_ERR_INVALID_ARGUMENT, "genstep t1 must be >= t0");
     DevParams d = ev[gs.event];
+    for (int k : {0, 1, 2, 4, 5, 6})
+      if (std::fabs(v[k]) > kFarCoordinate) d.flags &= ~kOrdinary;
     d.source = kSourceSegment;
     d.src_x = gs.x0;
     d.src_y = gs.y0;
@@ -2231,6 +2255,7 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   std::memset(&a, 0, sizeof(a));
   a.n_events = 1;
   a.n_tallies = 1;
+  a.flags = P.flags;
   a.ev_shift = kEvShift;
   a.threshold = 28;
   a.cadence = 0;

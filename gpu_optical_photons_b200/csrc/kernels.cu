@@ -88,7 +88,7 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
       start_photon<false>(P, s, r, id, aux);
       uint32_t fate = kMaxSteps;
       for (uint32_t st = 0; st < P.max_steps; ++st) {
-        if (!step_photon<false>(P, s, r, id, fate, aux)) break;
+        if (!step_photon<false>(P, P.flags, s, r, id, fate, aux)) break;
       }
       done(i, s, fate);
     }
@@ -111,7 +111,7 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
       alive = true;
       ended = P.max_steps == 0u;
     } else {
-      ended = !step_photon<false>(P, s, r, first_id + cur, fate, aux);
+      ended = !step_photon<false>(P, P.flags, s, r, first_id + cur, fate, aux);
       if (!ended && ++step >= P.max_steps) ended = true;  // fate stays kMaxSteps
     }
     if (ended) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     const float4* qin;
     float4* qout;
     unsigned long long fresh_next, first_id, iter_cap;
-    uint32_t n_in, items, T, cadence, qcap, chunk, ev_shift, tail_steps, slot_cache;
+    uint32_t n_in, items, T, cadence, qcap, chunk, ev_shift, tail_steps, slot_cache, flags;
     const uint32_t* tally_of;
     TallyDev tc;
   };
@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     ws.ev_shift = A->ev_shift;
     ws.tail_steps = A->tail_steps < 1u ? 1u : A->tail_steps;
     ws.slot_cache = A->slot_cache;
+    ws.flags = (ctrl->gs_error & kFarGenstep) != 0u ? A->flags & ~kOrdinary : A->flags;
     ws.tc = A->tc;
   }
   __syncthreads();
@@ -717,7 +718,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     if (alive) {
       const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
       const bool still =
-          step_photon<kAdj, BATCH && !UNI>(P, s, r, first_id + pidx, fate, aux, smask);
+          step_photon<kAdj, BATCH && !UNI>(P, ws.flags, s, r, first_id + pidx, fate, aux, smask);
       ++wsteps;
       ended = !still || s.nb + s.ns >= P.max_steps;  // at max_steps fate stays kMaxSteps
     }
@@ -932,7 +933,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
     const uint64_t id = A.first_id + rel;
     if (seg < 3u) {
       const uint32_t m = __ballot_sync(kFull, valid);
-      if (valid) live = step_act<false>(P, s, r, id, fate, aux, hit, m);
+      if (valid) live = step_act<false>(P, P.flags, s, r, id, fate, aux, hit, m);
     }
 
     int next = -1;
@@ -940,7 +941,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
       // Last launch: the rest of each history in place (transport.hpp:151-159).
       while (live) {
         if (s.nb + s.ns >= P.max_steps) { fate = kMaxSteps; live = false; break; }
-        live = step_photon<false>(P, s, r, id, fate, aux);
+        live = step_photon<false>(P, P.flags, s, r, id, fate, aux);
       }
     } else if (live) {
       // Photons that have made max_steps steps end here (each live step counted
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         fate = kMaxSteps;
         live = false;
       } else {
-        hit = step_move(P, s, r);
+        hit = step_move(P, P.flags, s, r);
         if (hit == kHitAbsorb) {  // bulk absorption (transport.hpp:98-101)
           fate = kAbsorbedBulk;
           live = false;

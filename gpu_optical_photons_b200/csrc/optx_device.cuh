@@ -34,6 +34,9 @@
 #ifndef OPTX_EXACT
 #define OPTX_EXACT 0
 #endif
+#ifndef OPTX_APPROX  // 1: compiled with --use_fast_math
+#define OPTX_APPROX 0
+#endif
 
 namespace optx {
 
@@ -54,7 +57,7 @@ struct __align__(16) DevParams {
   uint32_t key_lo;
   uint32_t key_hi;
   float inv2hx, inv2hy;                    // 1 / (2 hx), 1 / (2 hy) rounded to nearest (xy_bin)
-  uint32_t pad2;
+  uint32_t flags;                          // kOrdinary
 };
 static_assert(sizeof(DevParams) == 112, "DevParams layout");
 // Indexed reads of a record in global memory (face_refl, step_act) rely on these
@@ -75,6 +78,11 @@ struct DevRecords {
   uint32_t* n_scatter;
   float *t, *x, *y, *z, *path;
 };
+
+// DevParams::flags. kOrdinary: sizes, indices and source lie where the branch-free
+// quotients below are exact (ordinary_params in capi.cu); a run with any other
+// record takes the IEEE divisions.
+enum : uint32_t { kOrdinary = 1u };
 
 enum : uint32_t { kPolished = 0, kBlack = 1, kSpecular = 2, kLambertian = 3 };
 enum : uint32_t { kDetected = 0, kAbsorbedBulk = 1, kAbsorbedSurface = 2, kEscaped = 3, kMaxSteps = 4 };
@@ -101,7 +109,8 @@ __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1) {
 
 // (bits >> 8) + 1 times 2^-24, in (0, 1], exact (philox.hpp:82-84).
 __device__ __forceinline__ float to_uniform(uint32_t bits) {
-  return __uint2float_rn((bits >> 8) + 1u) * (1.0f / 16777216.0f);
+  // One FMA for the addition and the scaling: the sum is at most 2^24, so exact.
+  return fmaf(__uint2float_rn(bits >> 8), 1.0f / 16777216.0f, 1.0f / 16777216.0f);
 }
 
 // The photon's random stream as a window of two consecutive Philox blocks.
@@ -159,6 +168,59 @@ struct Rng {
 };
 
 // ---------------------------------------------------------------------------
+// Correctly rounded quotient, reciprocal and square root without a branch: the
+// hardware's approximation, refined with FMA residuals (Markstein, IBM J. Res.
+// Dev. 34(1), 1990: with y the rounded reciprocal and q within an ulp of a / b,
+// q + (a - b q) y rounds to the quotient; the square root likewise from
+// g = x / sqrt(x) and its residual x - g^2). They equal the IEEE operations on the
+// ranges the step uses them on; tests/cuda/ieee_check.cu compares them with
+// __fdiv_rn, __frcp_rn and __fsqrt_rn. nvcc's own operators guard every range with a
+// check and a branch to a slow path: a step has about a dozen of them, one after
+// another, and the branches also keep the chains from overlapping. Measured against
+// the operators (1e7 photons, kernel time): Lambertian cube 1.90 -> 1.64 ms, polished
+// cube 1.36 -> 1.22 ms; 4096-event batch 9.81 -> 9.27 ms. The APPROX build keeps
+// the operators: --use_fast_math already turns them into the approximations.
+#if OPTX_APPROX
+__device__ __forceinline__ float m_rcp(float b) { return 1.0f / b; }
+__device__ __forceinline__ float m_div(float a, float b) { return a / b; }
+__device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
+#else
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float lg2_approx(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 1 / b for 2^-100 <= |b| <= 2^100; NaN for b = 0.
+__device__ __forceinline__ float m_rcp(float b) {
+  const float y = rcp_approx(b);
+  return fmaf(y, fmaf(-b, y, 1.0f), y);
+}
+// a / b for b as above and a = 0 or |a| >= 2^-100, when the quotient is normal (or
+// 0); NaN for b = 0.
+__device__ __forceinline__ float m_div(float a, float b) {
+  const float y = m_rcp(b);
+  const float q = a * y;
+  return fmaf(fmaf(-b, q, a), y, q);
+}
+// sqrt(x) for x = 0 or 2^-60 <= x <= 2^60.
+__device__ __forceinline__ float m_sqrt(float x) {
+  const float y = rsqrt_approx(fmaxf(x, 0x1p-60f));  // finite at 0, where g = 0 x y = 0
+  const float g = x * y;
+  return fmaf(fmaf(-g, g, x), 0.5f * y, g);
+}
+#endif
+
+// ---------------------------------------------------------------------------
 // Math policy (pmath.hpp:134-158). Fast: CUDA's library functions. Exact: the
 // portable functions built from correctly rounded operations only (the
 // reference's pmath.hpp:62-130 methods: atanh series for log, exact quarter-turn
@@ -173,7 +235,7 @@ __device__ __forceinline__ float m_log(float x) {
     m = 0.5f * m;
     ++e;
   }
-  const float s = (m - 1.0f) / (m + 1.0f);
+  const float s = m_div(m - 1.0f, m + 1.0f);
   const float s2 = s * s;
   const float poly = 1.0f + s2 * (1.0f / 3.0f + s2 * (1.0f / 5.0f + s2 * (1.0f / 7.0f +
                      s2 * (1.0f / 9.0f + s2 * (1.0f / 11.0f)))));
@@ -203,13 +265,19 @@ __device__ __forceinline__ void m_sincos_turns(float u, float& s, float& c) {
 __device__ __forceinline__ float m_cbrt(float x) {
   float y = __uint_as_float(__float_as_uint(x) / 3u + 0x2a514067u);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) y = y - (y * y * y - x) / (3.0f * y * y);
+  for (int i = 0; i < 4; ++i) y = y - m_div(y * y * y - x, 3.0f * y * y);
   return y;
 }
 #else
 __device__ __forceinline__ float m_log(float x) { return logf(x); }
 __device__ __forceinline__ void m_sincos_turns(float u, float& s, float& c) {
-  sincosf(6.28318530717958647692f * u, &s, &c);
+  const float a = 6.28318530717958647692f * u;
+#if !OPTX_APPROX
+  // u is in (0, 1]: without this the reduction of huge arguments is compiled in,
+  // with a 28-byte local array (measured: -2.6 % on the Lambertian cube).
+  __builtin_assume(fabsf(a) <= 7.0f);
+#endif
+  sincosf(a, &s, &c);
 }
 __device__ __forceinline__ float m_cbrt(float x) { return cbrtf(x); }
 #endif
@@ -245,18 +313,18 @@ __device__ __forceinline__ float face_refl(const DevParams& P, int face) {
 __device__ __forceinline__ void rotate_about(float ax, float ay, float az, float ct, float phi_u,
                                              float& ox, float& oy, float& oz) {
   const float sign = copysignf(1.0f, az);
-  const float a = -1.0f / (sign + az);
+  const float a = -m_rcp(sign + az);
   const float b = ax * ay * a;
   const float t1x = 1.0f + sign * ax * ax * a, t1y = sign * b, t1z = -sign * ax;
   const float t2x = b, t2y = sign + ay * ay * a, t2z = -ay;
-  const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+  const float st = m_sqrt(fmaxf(0.0f, 1.0f - ct * ct));
   float sp, cp;
   m_sincos_turns(phi_u, sp, cp);
   const float A = st * cp, B = st * sp;
   const float x = A * t1x + B * t2x + ct * ax;
   const float y = A * t1y + B * t2y + ct * ay;
   const float z = A * t1z + B * t2z + ct * az;
-  const float inv = 1.0f / sqrtf(x * x + y * y + z * z);
+  const float inv = m_rcp(m_sqrt(x * x + y * y + z * z));
   ox = inv * x;
   oy = inv * y;
   oz = inv * z;
@@ -266,24 +334,65 @@ __device__ __forceinline__ void rotate_about(float ax, float ay, float az, float
 // (sampling.hpp:39-44).
 __device__ __forceinline__ float rayleigh_cos(float u) {
   const float q = 4.0f * u - 2.0f;
-  const float s = sqrtf(q * q + 1.0f);
+  const float s = m_sqrt(q * q + 1.0f);
   // One cube-root call site: cbrt(q + s) for q >= 0, 1 / cbrt(s - q) otherwise.
   const bool pos = q >= 0.0f;
   const float c = m_cbrt(pos ? q + s : s - q);
-  const float a = pos ? c : 1.0f / c;
-  return fminf(1.0f, fmaxf(-1.0f, a - 1.0f / a));
+  const float a = pos ? c : m_rcp(c);
+  return fminf(1.0f, fmaxf(-1.0f, a - m_rcp(a)));
 }
 
 // Unpolarised Fresnel reflectance from n1 into n2 (fresnel.hpp:30-46);
 // eta2 = (n1 / n2)^2 precomputed with the same float operations.
 __device__ __forceinline__ float fresnel_R(float n1, float n2, float eta2, float cos_i) {
   if (n1 == n2) return 0.0f;
+#if OPTX_EXACT || OPTX_APPROX
   const float sin2_t = eta2 * fmaxf(0.0f, 1.0f - cos_i * cos_i);
+#else
+  const float sin2_t = __fmul_rn(eta2, fmaxf(0.0f, fmaf(-cos_i, cos_i, 1.0f)));
+#endif
   if (sin2_t >= 1.0f) return 1.0f;
   const float cos_t = sqrtf(1.0f - sin2_t);
+#if OPTX_EXACT || OPTX_APPROX
   const float rs = (n1 * cos_i - n2 * cos_t) / (n1 * cos_i + n2 * cos_t);
   const float rp = (n2 * cos_i - n1 * cos_t) / (n2 * cos_i + n1 * cos_t);
   return 0.5f * (rs * rs + rp * rp);
+#else
+  // nvcc's contraction of these expressions, spelled out: left to the compiler it
+  // would depend on what the caller computes beside them.
+  const float rs = fmaf(n1, cos_i, __fmul_rn(-n2, cos_t)) / fmaf(n1, cos_i, __fmul_rn(n2, cos_t));
+  const float rp = fmaf(n2, cos_i, __fmul_rn(-n1, cos_t)) / fmaf(n2, cos_i, __fmul_rn(n1, cos_t));
+  return 0.5f * fmaf(rs, rs, __fmul_rn(rp, rp));
+#endif
+}
+
+// u <= fresnel_R(...): the step needs only this outcome, never R itself, so the
+// comparison is made on approximate values, multiplied out (no division), and
+// fresnel_R decides where they leave it open. With p = n1 c + n2 ct and
+// q = n2 c + n1 ct, R = (v^2 + w^2) / (2 (p q)^2), v = (n1 c - n2 ct) q,
+// w = (n2 c - n1 ct) p. Both sides are off by less than 2^-17 (p q)^2 (the
+// approximate square root by 2^-22 of itself; fresnel_R's own rounding
+// included), a quarter of the margin; within 2^-10 of total internal
+// reflection, where sqrt(1 - sin2_t) magnifies the rounding of sin2_t, and outside
+// the ordinary range, fresnel_R decides too. Measured against calling it always:
+// batch 9.27 -> 9.09 ms, gradient run of 1e6 photons 0.272 -> 0.259 ms.
+__device__ __forceinline__ bool fresnel_reflects(float n1, float n2, float eta2, float cos_i, float u,
+                                                 uint32_t flags) {
+#if OPTX_APPROX
+  (void)flags;
+  return u <= fresnel_R(n1, n2, eta2, cos_i);
+#else
+  const float c2 = 1.0f - eta2 * fmaxf(0.0f, 1.0f - cos_i * cos_i);
+  const float ct = c2 * rsqrt_approx(fmaxf(c2, 0x1p-60f));
+  const float a = n1 * cos_i, b = n2 * ct, c = n2 * cos_i, d = n1 * ct;
+  const float p = a + b, q = c + d, pq = p * q, v = (a - b) * q, w = (c - d) * p;
+  const float den = pq * pq;
+  const float diff = fmaf(v, v, w * w) - 2.0f * u * den;
+  bool r = c2 < 0.0f || diff > 0.0f;
+  const bool open = !(fabsf(diff) > 0x1p-15f * den) && !(c2 <= -0x1p-10f);
+  if (open || fabsf(c2) < 0x1p-10f || !(flags & kOrdinary)) r = u <= fresnel_R(n1, n2, eta2, cos_i);
+  return r;
+#endif
 }
 
 // Emission (transport.hpp:55-67): position (3 draws, volume source only),
@@ -325,7 +434,7 @@ __device__ __forceinline__ void start_photon(const DevParams& P, Photon& s, Rng&
   }
   const float ua = r.uniform<0>(), ub = r.uniform<1>(), ue = r.uniform<2>();
   const float ct = 2.0f * ua - 1.0f;
-  const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+  const float st = m_sqrt(fmaxf(0.0f, 1.0f - ct * ct));
   float sp, cp;
   m_sincos_turns(ub, sp, cp);
   s.dx = st * cp;
@@ -345,21 +454,11 @@ __device__ __forceinline__ void start_photon(const DevParams& P, Photon& s, Rng&
 constexpr int kHitScatter = 6;
 constexpr int kHitAbsorb = 7;
 
-// First half of a step (transport.hpp:71-97): the exponential absorption and
-// scattering distances (window words 0 and 1), the box exit, and the move to the
-// nearest of the three. Returns the interaction; the window is not advanced.
-__device__ __forceinline__ int step_move(const DevParams& P, Photon& s, const Rng& r) {
-  const float u_abs = r.uniform<0>(), u_sca = r.uniform<1>();
-  const float s_abs = (P.abs_length == kInf) ? kInf : -P.abs_length * m_log(u_abs);
-  const float s_sca = (P.scat_length == kInf) ? kInf : -P.scat_length * m_log(u_sca);
-
-  // Distance to the box exit: per axis only the face the photon moves towards
-  // (geometry.hpp:25-46).
-  // All three quotients are computed and an axis the photon does not move along
-  // is then masked (its quotient, a division by zero, is never used): the same
-  // values as skipping it, without a branch per axis.
-  float dist = kInf;
-  int face = -1;
+// Distance to the box exit: per axis only the face the photon moves towards
+// (geometry.hpp:25-46), an axis it does not move along being skipped.
+__device__ __forceinline__ void box_exit_ieee(const DevParams& P, const Photon& s, float& dist, int& face) {
+  dist = kInf;
+  face = -1;
   {
     const bool pos = s.dx > 0.0f;
     const float tt = ((pos ? P.hx : -P.hx) - s.px) / s.dx;
@@ -375,8 +474,43 @@ __device__ __forceinline__ int step_move(const DevParams& P, Photon& s, const Rn
     const float tt = ((pos ? P.hz : -P.hz) - s.pz) / s.dz;
     if (s.dz != 0.0f && tt < dist) { dist = tt; face = pos ? 5 : 4; }
   }
+}
+
+// The same for ordinary records, where m_div is exact: the quotient of an axis the
+// photon does not move along is NaN and fminf passes over it; an earlier axis wins
+// a tie, as in the order of the comparisons above. (A direction component is 0 or
+// far above 2^-100: it comes out of sums of products of uniforms and sines.)
+__device__ __forceinline__ void box_exit(const DevParams& P, uint32_t flags, const Photon& s, float& dist,
+                                         int& face) {
+#if OPTX_APPROX
+  box_exit_ieee(P, s, dist, face);
+#else
+  if (!(flags & kOrdinary)) {
+    box_exit_ieee(P, s, dist, face);
+    return;
+  }
+  const float tx = m_div(copysignf(P.hx, s.dx) - s.px, s.dx);
+  const float ty = m_div(copysignf(P.hy, s.dy) - s.py, s.dy);
+  const float tz = m_div(copysignf(P.hz, s.dz) - s.pz, s.dz);
+  dist = fminf(fminf(tx, ty), tz);
+  const bool x = tx == dist, y = ty == dist;
+  const float along = x ? s.dx : (y ? s.dy : s.dz);
+  face = (x ? 0 : (y ? 2 : 4)) + (along > 0.0f ? 1 : 0);
+#endif
+}
+
+// First half of a step (transport.hpp:71-97): the exponential absorption and
+// scattering distances (window words 0 and 1), the box exit, and the move to the
+// nearest of the three. Returns the interaction; the window is not advanced.
+__device__ __forceinline__ int step_move(const DevParams& P, uint32_t flags, Photon& s, const Rng& r) {
+  const float u_abs = r.uniform<0>(), u_sca = r.uniform<1>();
+  float dist;
+  int face;
+  box_exit(P, flags, s, dist, face);
   dist = fmaxf(dist, 0.0f);
 
+  const float s_abs = (P.abs_length == kInf) ? kInf : -P.abs_length * m_log(u_abs);
+  const float s_sca = (P.scat_length == kInf) ? kInf : -P.scat_length * m_log(u_sca);
   const bool absorb = s_abs < dist && s_abs <= s_sca;
   const bool scatter = !absorb && s_sca < dist;
   const float d = absorb ? s_abs : (scatter ? s_sca : dist);
@@ -412,7 +546,7 @@ __device__ __forceinline__ uint32_t face_model(const DevParams& P, int face) {
 // runs once per warp step for all lanes that need one rather than once per
 // divergent group.
 template <bool AUX, bool GP = false>
-__device__ __forceinline__ bool step_act(const DevParams& P, Photon& s, Rng& r, uint64_t id,
+__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t flags, Photon& s, Rng& r, uint64_t id,
                                          uint32_t& fate, ScoreAux& aux, int hit,
                                          uint32_t sync_mask = 0u) {
   const int face = hit;
@@ -443,10 +577,9 @@ __device__ __forceinline__ bool step_act(const DevParams& P, Photon& s, Rng& r, 
       const bool readout = face == kReadoutFace;
       const int oi = readout ? 0 : 1;
       const float n2 = GP ? (&P.n_det)[oi] : (readout ? P.n_det : P.n_out);
-      const float R = fresnel_R(P.n_scint, n2, GP ? (&P.eta2_det)[oi] : (readout ? P.eta2_det : P.eta2_out),
-                                cos_i);
+      const float eta2 = GP ? (&P.eta2_det)[oi] : (readout ? P.eta2_det : P.eta2_out);
       k = 3u;
-      if (u2 <= R) {
+      if (fresnel_reflects(P.n_scint, n2, eta2, cos_i, u2, flags)) {
         flip = true;
       } else {
         fate = readout ? kDetected : kEscaped;
@@ -490,13 +623,14 @@ __device__ __forceinline__ bool step_act(const DevParams& P, Photon& s, Rng& r, 
   return live;
 }
 
-// One step (transport.hpp:71-145): move, then interact.
+// One step (transport.hpp:71-145): move, then interact. `flags`: those that hold for
+// every record of the run.
 template <bool AUX, bool GP = false>
-__device__ __forceinline__ bool step_photon(const DevParams& P, Photon& s, Rng& r, uint64_t id,
+__device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, Photon& s, Rng& r, uint64_t id,
                                             uint32_t& fate, ScoreAux& aux,
                                             uint32_t sync_mask = 0u) {
-  const int hit = step_move(P, s, r);
-  return step_act<AUX, GP>(P, s, r, id, fate, aux, hit, sync_mask);
+  const int hit = step_move(P, flags, s, r);
+  return step_act<AUX, GP>(P, flags, s, r, id, fate, aux, hit, sync_mask);
 }
 
 // Tally binning (transport.hpp:170-181); tscale = time_bins / time_max in float.

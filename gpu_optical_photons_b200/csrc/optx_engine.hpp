@@ -58,6 +58,7 @@ struct WaveArgs {
   uint32_t tail_steps;                  // steps a photon makes in a wave before it may be spilled at its end
   uint32_t slot_cache;                  // batched tallies: 1 = warps may cache events in shared-memory
                                         // slots (every record's max_steps < kSlotMaxAdd)
+  uint32_t flags;                       // DevParams::flags that every record has
   uint32_t keep_tally;                  // 1: the run adds to the tallies (no zeroing by the prep kernel)
   const uint32_t* tally_of;             // record -> event (null: the record's own index)
   const float4* seg;                    // genstep records: 2 float4 each (end x,y,z,t0), (dt,-,-,-)
@@ -78,7 +79,8 @@ struct WaveCtrl {
   unsigned int error;              // bit 0 queue overflow, bit 1 watchdog
   unsigned int spills;             // total photons spilled over the run
   unsigned int gs_error;           // device genstep upload: bit 0 an invalid genstep, bit 1 more
-                                   // photons than the engine holds (kept until the next upload)
+                                   // photons than the engine holds, kFarGenstep (no error) a
+                                   // genstep outside kFarCoordinate (kept until the next upload)
 };
 
 // kModeMoments: the adjoint replay that also fills the per-bin score moments
@@ -97,6 +99,9 @@ constexpr uint32_t kPantryBytesPerWarp = 32u * 112u;
 // for the kernels here).
 constexpr size_t kDynSmemOptIn = 47u * 1024u;
 constexpr unsigned kErrQueue = 1u, kErrWatchdog = 2u;
+// Sources beyond this (mm) are not kOrdinary.
+constexpr float kFarCoordinate = 0x1p40f;
+constexpr unsigned kFarGenstep = 4u;
 // Batched tallies: each warp caches the counters of two events in shared memory
 // (7 x u32 per event, padded to 8) and, when the tally has at most kSlotBins
 // histogram bins, their time / hit-map bins too (u32). A warp flushes both its
