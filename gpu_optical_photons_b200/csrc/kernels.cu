@@ -87,15 +87,14 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
       r.init(id, P.key_lo, P.key_hi, 0u);
       start_photon<false>(P, s, r, id, aux);
       uint32_t fate = kMaxSteps;
-      for (uint32_t st = 0; st < P.max_steps; ++st) {
-        if (!step_photon<false>(P, P.flags, s, r, id, fate, aux)) break;
+      if (P.max_steps != 0u) {
+        while (step_photon<false>(P, P.flags, s, r, id, fate, aux)) {}
       }
       done(i, s, fate);
     }
     return;
   }
   uint64_t cur = 0;
-  uint32_t step = 0;
   bool alive = false;
   for (;;) {
     uint32_t fate = kMaxSteps;
@@ -107,12 +106,10 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
       const uint64_t id = first_id + cur;
       r.init(id, P.key_lo, P.key_hi, 0u);
       start_photon<false>(P, s, r, id, aux);
-      step = 0;
       alive = true;
       ended = P.max_steps == 0u;
     } else {
       ended = !step_photon<false>(P, P.flags, s, r, first_id + cur, fate, aux);
-      if (!ended && ++step >= P.max_steps) ended = true;  // fate stays kMaxSteps
     }
     if (ended) {
       alive = false;
@@ -297,6 +294,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
   //  nwarps x 2 x n_bins u32 bins when n_bins <= kSlotBins]
   constexpr bool kSlots = BATCH && MODE == kModeTally;
   constexpr bool kAdj = MODE == kModeAdjoint || MODE == kModeMoments;  // replay modes
+  constexpr bool kPath = MODE != kModeTally;  // tallies do not use the path length
   float4* pantry = reinterpret_cast<float4*>(smem_raw + warp * kPantryBytesPerWarp);
   unsigned char* extra = smem_raw + nwarps * kPantryBytesPerWarp;
   uint32_t* s_hist = reinterpret_cast<uint32_t*>(extra);
@@ -664,7 +662,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
           const float4* e = pantry + (pc - 1u - rank) * 7u;
           const float4 a = e[0], b = e[1], c = e[2], d = e[3], f = e[4];
           s.px = a.x; s.py = a.y; s.pz = a.z; s.t = a.w;
-          s.dx = b.x; s.dy = b.y; s.dz = b.z; s.path = b.w;
+          s.dx = b.x; s.dy = b.y; s.dz = b.z;
+          if (kPath) s.path = b.w;
           s.nb = __float_as_uint(c.x);
           s.ns = __float_as_uint(c.y);
           pidx = __float_as_uint(c.z);
@@ -717,10 +716,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     bool ended = false;
     if (alive) {
       const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
-      const bool still =
-          step_photon<kAdj, BATCH && !UNI>(P, ws.flags, s, r, first_id + pidx, fate, aux, smask);
+      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, s, r, first_id + pidx, fate, aux, smask);
       ++wsteps;
-      ended = !still || s.nb + s.ns >= P.max_steps;  // at max_steps fate stays kMaxSteps
     }
     __syncwarp();
     if (ended) {
@@ -933,16 +930,17 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
     const uint64_t id = A.first_id + rel;
     if (seg < 3u) {
       const uint32_t m = __ballot_sync(kFull, valid);
-      if (valid) live = step_act<false>(P, P.flags, s, r, id, fate, aux, hit, m);
+      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, s, r, id, fate, aux, hit, m);
     }
 
     int next = -1;
     if (drain) {
       // Last launch: the rest of each history in place (transport.hpp:151-159).
-      while (live) {
-        if (s.nb + s.ns >= P.max_steps) { fate = kMaxSteps; live = false; break; }
-        live = step_photon<false>(P, P.flags, s, r, id, fate, aux);
+      if (live && s.nb + s.ns >= P.max_steps) {
+        fate = kMaxSteps;
+        live = false;
       }
+      while (live) live = step_photon<false>(P, P.flags, s, r, id, fate, aux);
     } else if (live) {
       // Photons that have made max_steps steps end here (each live step counted
       // one boundary or one scatter).
@@ -950,14 +948,14 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         fate = kMaxSteps;
         live = false;
       } else {
-        hit = step_move(P, P.flags, s, r);
+        hit = step_move(load_step<false>(P), P.flags, s, r);
         if (hit == kHitAbsorb) {  // bulk absorption (transport.hpp:98-101)
           fate = kAbsorbedBulk;
           live = false;
         } else if (hit == kHitScatter) {
           next = kQScatter;
         } else {
-          const uint32_t model = face_model(P, hit);
+          const uint32_t model = face_model(P.surf_bits, hit);
           if (model == kBlack) {  // black face: absorbed, no draw (transport.hpp:129-132)
             ++s.nb;
             fate = kAbsorbedSurface;

@@ -42,34 +42,34 @@ namespace optx {
 
 // ---------------------------------------------------------------------------
 // Parameters as the kernels see them (built by the host from optx_params and
-// optx_faces, see capi.cpp: make_dev_params). 112 bytes, 16-byte aligned so
-// that a table of them is read with 128-bit loads.
+// optx_faces, see capi.cu: make_dev_params). 112 bytes in 16-byte groups of what is
+// read together, so that a record in memory costs a step two 128-bit loads, a
+// polished face two 64-bit loads and a Philox block one (load_step, step_act): with
+// one 32-bit load per field the batch ran 19 of them per warp step and took 9.08 ms
+// against 8.9.
 struct __align__(16) DevParams {
   float hx, hy, hz, inv_speed;             // inv_speed = n_scint / c  (transport.hpp:74)
-  float n_scint, n_det, n_out, abs_length;
-  float scat_length, tau, src_x, src_y;
-  float src_z;
-  uint32_t surf_bits;                      // 2 bits per face 0..4: Polished/Black/Specular/Lambertian
+  float abs_length, scat_length;
   uint32_t max_steps;
-  uint32_t source;                         // 0 point, 1 uniform in the volume, 2 genstep segment
+  uint32_t surf_bits;                      // 2 bits per face 0..4: Polished/Black/Specular/Lambertian
+  float n_det, eta2_det, n_out, eta2_out;  // eta2 = (n_scint / n)^2 (fresnel.hpp:32-33)
+  float n_scint, tau;
+  uint32_t key_lo, key_hi;
   float refl0, refl1, refl2, refl3;        // reflectivity of faces 0..4
-  float refl4, eta2_det, eta2_out;         // (n_scint/n_det)^2, (n_scint/n_out)^2 (fresnel.hpp:32-33)
-  uint32_t key_lo;
-  uint32_t key_hi;
-  float inv2hx, inv2hy;                    // 1 / (2 hx), 1 / (2 hy) rounded to nearest (xy_bin)
+  float refl4;
   uint32_t flags;                          // kOrdinary
+  float inv2hx, inv2hy;                    // 1 / (2 hx), 1 / (2 hy) rounded to nearest (xy_bin)
+  float src_x, src_y, src_z;
+  uint32_t source;                         // 0 point, 1 uniform in the volume, 2 genstep segment
 };
 static_assert(sizeof(DevParams) == 112, "DevParams layout");
-// Indexed reads of a record in global memory (face_refl, step_act) rely on these
-// runs of consecutive floats: refl0..refl4, (n_det, n_out), (eta2_det, eta2_out).
-static_assert(offsetof(DevParams, refl1) == offsetof(DevParams, refl0) + 4 &&
-                  offsetof(DevParams, refl2) == offsetof(DevParams, refl0) + 8 &&
-                  offsetof(DevParams, refl3) == offsetof(DevParams, refl0) + 12 &&
+// The wide and the indexed reads of a record in memory rely on these places.
+static_assert(offsetof(DevParams, abs_length) == 16 && offsetof(DevParams, surf_bits) == 28 &&
+                  offsetof(DevParams, n_det) == 32 && offsetof(DevParams, n_out) == 40 &&
+                  offsetof(DevParams, key_lo) % 8 == 0 &&
+                  offsetof(DevParams, key_hi) == offsetof(DevParams, key_lo) + 4 &&
                   offsetof(DevParams, refl4) == offsetof(DevParams, refl0) + 16,
-              "DevParams reflectivities must be consecutive");
-static_assert(offsetof(DevParams, n_out) == offsetof(DevParams, n_det) + 4 &&
-                  offsetof(DevParams, eta2_out) == offsetof(DevParams, eta2_det) + 4,
-              "DevParams readout / outside pairs must be consecutive");
+              "DevParams layout");
 
 // Device-side structure-of-arrays photon records (29 bytes per photon).
 struct DevRecords {
@@ -294,18 +294,40 @@ struct ScoreAux {
   float t_emit;     // sampled emission time
 };
 
-// GP: P is a record in global memory, where an indexed load costs one
-// instruction; a kernel parameter is read with selects instead (indexing it
-// would copy the parameters to local memory).
+// GP: P is a record in global memory, read with wide or indexed loads; a kernel
+// parameter is read field by field and with selects instead (indexing it would copy
+// the parameters to local memory). Records do not change while a kernel that steps
+// photons runs.
 template <bool GP>
 __device__ __forceinline__ float face_refl(const DevParams& P, int face) {
-  if (GP) return (&P.refl0)[face];
+  if (GP) return __ldg(&P.refl0 + face);
   float r = P.refl0;
   r = (face == 1) ? P.refl1 : r;
   r = (face == 2) ? P.refl2 : r;
   r = (face == 3) ? P.refl3 : r;
   r = (face == 4) ? P.refl4 : r;
   return r;
+}
+
+// The parameters that every step reads.
+struct StepParams {
+  float hx, hy, hz, inv_speed, abs_length, scat_length;
+  uint32_t max_steps, surf_bits;
+};
+template <bool GP>
+__device__ __forceinline__ StepParams load_step(const DevParams& P) {
+  if (GP) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(&P)), b = __ldg(reinterpret_cast<const float4*>(&P) + 1);
+    return {a.x, a.y, a.z, a.w, b.x, b.y, __float_as_uint(b.z), __float_as_uint(b.w)};
+  }
+  return {P.hx, P.hy, P.hz, P.inv_speed, P.abs_length, P.scat_length, P.max_steps, P.surf_bits};
+}
+
+// The two words of the Philox key.
+template <bool GP>
+__device__ __forceinline__ uint2 load_key(const DevParams& P) {
+  if (GP) return __ldg(reinterpret_cast<const uint2*>(&P.key_lo));
+  return make_uint2(P.key_lo, P.key_hi);
 }
 
 // Branch-free orthonormal basis (Duff et al., JCGT 6(1) 2017) and rotation
@@ -456,7 +478,7 @@ constexpr int kHitAbsorb = 7;
 
 // Distance to the box exit: per axis only the face the photon moves towards
 // (geometry.hpp:25-46), an axis it does not move along being skipped.
-__device__ __forceinline__ void box_exit_ieee(const DevParams& P, const Photon& s, float& dist, int& face) {
+__device__ __forceinline__ void box_exit_ieee(const StepParams& P, const Photon& s, float& dist, int& face) {
   dist = kInf;
   face = -1;
   {
@@ -480,7 +502,7 @@ __device__ __forceinline__ void box_exit_ieee(const DevParams& P, const Photon& 
 // photon does not move along is NaN and fminf passes over it; an earlier axis wins
 // a tie, as in the order of the comparisons above. (A direction component is 0 or
 // far above 2^-100: it comes out of sums of products of uniforms and sines.)
-__device__ __forceinline__ void box_exit(const DevParams& P, uint32_t flags, const Photon& s, float& dist,
+__device__ __forceinline__ void box_exit(const StepParams& P, uint32_t flags, const Photon& s, float& dist,
                                          int& face) {
 #if OPTX_APPROX
   box_exit_ieee(P, s, dist, face);
@@ -501,8 +523,10 @@ __device__ __forceinline__ void box_exit(const DevParams& P, uint32_t flags, con
 
 // First half of a step (transport.hpp:71-97): the exponential absorption and
 // scattering distances (window words 0 and 1), the box exit, and the move to the
-// nearest of the three. Returns the interaction; the window is not advanced.
-__device__ __forceinline__ int step_move(const DevParams& P, uint32_t flags, Photon& s, const Rng& r) {
+// nearest of the three. Returns the interaction; the window is not advanced. Without
+// PATH the path length is left alone (tallies do not use it).
+template <bool PATH = true>
+__device__ __forceinline__ int step_move(const StepParams& P, uint32_t flags, Photon& s, const Rng& r) {
   const float u_abs = r.uniform<0>(), u_sca = r.uniform<1>();
   float dist;
   int face;
@@ -526,13 +550,13 @@ __device__ __forceinline__ int step_move(const DevParams& P, uint32_t flags, Pho
   s.py = ny;
   s.pz = nz;
   s.t = s.t + d * P.inv_speed;
-  s.path = s.path + d;
+  if (PATH) s.path = s.path + d;
   return absorb ? kHitAbsorb : (scatter ? kHitScatter : face);
 }
 
 // Surface model of face `face` (the readout face is always polished).
-__device__ __forceinline__ uint32_t face_model(const DevParams& P, int face) {
-  return (face == kReadoutFace) ? kPolished : ((P.surf_bits >> (2 * face)) & 3u);
+__device__ __forceinline__ uint32_t face_model(uint32_t surf_bits, int face) {
+  return (face == kReadoutFace) ? kPolished : ((surf_bits >> (2 * face)) & 3u);
 }
 
 // Second half of a step (transport.hpp:98-145): the interaction `hit` at the
@@ -540,97 +564,88 @@ __device__ __forceinline__ uint32_t face_model(const DevParams& P, int face) {
 // Returns true while the photon is alive; otherwise `fate` is set and the photon
 // sits at its final interaction. The window is advanced only for photons that
 // stay alive.
-// One exit: every outcome falls through to the shared tail (rotation, flip,
-// window advance). With sync_mask != 0 (the lanes of the warp that call this
-// step together) the warp reconverges before the advance, so the Philox block
+// The outcome of every interaction comes first, as a few predicates (kept,
+// scattered, mirrored, diffuse), then one pass each of the rotation, the mirror
+// flip and the advance for all lanes that need it: fewer branches than a body per
+// outcome (per warp step of the batch 47 of them, not 66; Lambertian cube 1e7
+// photons 1.63 -> 1.55 ms). With sync_mask != 0 (the lanes of the warp that call
+// this step together) the warp reconverges before the advance, so the Philox block
 // runs once per warp step for all lanes that need one rather than once per
 // divergent group.
 template <bool AUX, bool GP = false>
-__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t flags, Photon& s, Rng& r, uint64_t id,
-                                         uint32_t& fate, ScoreAux& aux, int hit,
+__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags, Photon& s, Rng& r,
+                                         uint64_t id, uint32_t& fate, ScoreAux& aux, int hit,
                                          uint32_t sync_mask = 0u) {
   const int face = hit;
   const int axis = face >> 1;
-  uint32_t k = 2u;           // words consumed by this step
-  bool live = true, rotate = false, flip = false;
-  float ax = s.dx, ay = s.dy, az = s.dz, ct = 0.0f, phi_u = 0.0f;
-  // The window's words 2..4 as uniforms, once for every outcome (each branch
-  // below uses its own subset; measured -2 % on the batch against drawing them
-  // inside the divergent branches).
+  // The window's words 2..4 as uniforms, once for every outcome (measured -2 % on
+  // the batch against drawing them where an outcome uses them).
   const float u2 = r.uniform<2>(), u3 = r.uniform<3>(), u4 = r.uniform<4>();
-  if (hit == kHitAbsorb) {
-    fate = kAbsorbedBulk;
-    live = false;
-  } else if (hit == kHitScatter) {
-    ++s.ns;
-    ct = rayleigh_cos(u2);
-    phi_u = u3;
-    rotate = true;
-    k = 4u;
-  } else {
-    ++s.nb;
-    const float cos_i = fabsf(axis == 0 ? s.dx : (axis == 1 ? s.dy : s.dz));
-    const uint32_t model = face_model(P, face);
+  const bool scattered = hit == kHitScatter, surface = hit < kHitScatter;
+  const uint32_t model = face_model(surf_bits, face);
+  bool kept = false;
+  if (surface) {
     if (model == kPolished) {
       // Readout face: interface to n_det, transmitted = detected; other faces:
       // interface to n_out, transmitted = escaped (transport.hpp:108-128).
       const bool readout = face == kReadoutFace;
-      const int oi = readout ? 0 : 1;
-      const float n2 = GP ? (&P.n_det)[oi] : (readout ? P.n_det : P.n_out);
-      const float eta2 = GP ? (&P.eta2_det)[oi] : (readout ? P.eta2_det : P.eta2_out);
-      k = 3u;
-      if (fresnel_reflects(P.n_scint, n2, eta2, cos_i, u2, flags)) {
-        flip = true;
-      } else {
-        fate = readout ? kDetected : kEscaped;
-        live = false;
-      }
-    } else if (model == kBlack) {
-      fate = kAbsorbedSurface;
-      live = false;
-    } else if (!(u2 <= face_refl<GP>(P, face))) {
-      // Painted reflector (transport.hpp:133-144): absorbed with 1 - R.
-      fate = kAbsorbedSurface;
-      live = false;
+      const float cos_i = fabsf(axis == 0 ? s.dx : (axis == 1 ? s.dy : s.dz));
+      float2 n2;  // index beyond the face, eta2
+      if (GP) n2 = __ldg(reinterpret_cast<const float2*>(&P.n_det) + (readout ? 0 : 1));
+      else n2 = readout ? make_float2(P.n_det, P.eta2_det) : make_float2(P.n_out, P.eta2_out);
+      kept = fresnel_reflects(GP ? __ldg(&P.n_scint) : P.n_scint, n2.x, n2.y, cos_i, u2, flags);
+      fate = readout ? kDetected : kEscaped;
     } else {
-      k = 3u;
-      if (AUX) ++aux.n_refl;
-      if (model == kSpecular) {
-        flip = true;
-      } else {
-        // Lambertian about the inward normal -n (signed zeros as in -face_normal()).
-        const float sg = (face & 1) ? -1.0f : 1.0f;
-        ax = (axis == 0) ? sg : -0.0f;
-        ay = (axis == 1) ? sg : -0.0f;
-        az = (axis == 2) ? sg : -0.0f;
-        ct = sqrtf(u3);
-        phi_u = u4;
-        rotate = true;
-        k = 5u;
-      }
+      // Painted reflector: absorbed with 1 - R; black: always (transport.hpp:129-144).
+      kept = model != kBlack && u2 <= face_refl<GP>(P, face);
+      fate = kAbsorbedSurface;
+      if (AUX && kept) ++aux.n_refl;
     }
+    ++s.nb;
+  } else {
+    fate = kAbsorbedBulk;
   }
-  if (rotate) {
+  if (scattered) ++s.ns;
+  const bool diffuse = kept && model == kLambertian, mirrored = kept && !diffuse;
+  const bool live = kept || scattered;
+  if (diffuse || scattered) {
+    float ax = s.dx, ay = s.dy, az = s.dz, ct, phi_u = u3;
+    if (scattered) {
+      ct = rayleigh_cos(u2);
+    } else {
+      // Lambertian about the inward normal -n (signed zeros as in -face_normal()).
+      const float sg = (face & 1) ? -1.0f : 1.0f;
+      ax = (axis == 0) ? sg : -0.0f;
+      ay = (axis == 1) ? sg : -0.0f;
+      az = (axis == 2) ? sg : -0.0f;
+      ct = m_sqrt(u3);
+      phi_u = u4;
+    }
     rotate_about(ax, ay, az, ct, phi_u, s.dx, s.dy, s.dz);
   }
-  if (flip) {
-    if (axis == 0) s.dx = -s.dx;
-    if (axis == 1) s.dy = -s.dy;
-    if (axis == 2) s.dz = -s.dz;
-  }
+  if (mirrored && axis == 0) s.dx = -s.dx;
+  if (mirrored && axis == 1) s.dy = -s.dy;
+  if (mirrored && axis == 2) s.dz = -s.dz;
   if (sync_mask != 0u) __syncwarp(sync_mask);
-  if (live) r.advance(k, id, P.key_lo, P.key_hi);
+  if (live) {
+    fate = kMaxSteps;
+    const uint2 key = load_key<GP>(P);
+    r.advance(scattered ? 4u : (diffuse ? 5u : 3u), id, key.x, key.y);
+  }
   return live;
 }
 
 // One step (transport.hpp:71-145): move, then interact. `flags`: those that hold for
-// every record of the run.
-template <bool AUX, bool GP = false>
+// every record of the run. False when the photon has ended, with its fate, or has
+// made max_steps steps (the fate is then kMaxSteps).
+template <bool AUX, bool GP = false, bool PATH = true>
 __device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, Photon& s, Rng& r, uint64_t id,
                                             uint32_t& fate, ScoreAux& aux,
                                             uint32_t sync_mask = 0u) {
-  const int hit = step_move(P, flags, s, r);
-  return step_act<AUX, GP>(P, flags, s, r, id, fate, aux, hit, sync_mask);
+  const StepParams q = load_step<GP>(P);
+  const int hit = step_move<PATH>(q, flags, s, r);
+  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, s, r, id, fate, aux, hit, sync_mask);
+  return live && s.nb + s.ns < q.max_steps;
 }
 
 // Tally binning (transport.hpp:170-181); tscale = time_bins / time_max in float.
