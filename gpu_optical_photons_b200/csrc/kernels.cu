@@ -195,11 +195,10 @@ __global__ void __launch_bounds__(1024, 1) history_tally_kernel(const DevParams 
 // (g >> shift) << shift; the scan moves past records that end before g (one or
 // two steps when records hold at least 2^shift photons; the host picks the
 // finest shift its table allocation allows).
-__device__ __forceinline__ uint32_t find_event(const WaveArgs* __restrict__ A, unsigned long long g,
-                                               uint32_t shift) {
-  uint32_t e = __ldg(A->ev_table + (g >> shift));
-  const unsigned long long* __restrict__ off = A->offsets;
-  while (e + 1u < A->n_events && __ldg(off + e + 1u) <= g) ++e;
+__device__ __forceinline__ uint32_t find_event(const WaveArgs& A, unsigned long long g) {
+  uint32_t e = __ldg(A.ev_table + (g >> A.ev_shift));
+  const unsigned long long* __restrict__ off = A.offsets;
+  while (e + 1u < A.n_events && __ldg(off + e + 1u) <= g) ++e;
   return e;
 }
 
@@ -231,11 +230,13 @@ __device__ __forceinline__ size_t qidx(uint32_t slot) {
   return static_cast<size_t>(slot >> 5) * 128u + (slot & 31u);
 }
 
-__global__ void wave_prep_kernel(const WaveArgs* __restrict__ A, WaveCtrl* __restrict__ ctrl) {
+__global__ void wave_prep_kernel(const __grid_constant__ WaveArgs A, WaveCtrl* __restrict__ ctrl) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned long long lo = A->item_lo < A->total ? A->item_lo : A->total;
-    unsigned long long fresh = A->total - lo < A->wave_quota ? A->total - lo : A->wave_quota;
-    if (A->cadence != 0u && fresh > A->qcap) fresh = A->qcap;
+    const unsigned long long total = A.total_ptr != nullptr ? *A.total_ptr : A.total;
+    const unsigned long long lo = A.item_lo < total ? A.item_lo : total;
+    unsigned long long fresh = total - lo < A.wave_quota ? total - lo : A.wave_quota;
+    if (A.cadence != 0u && fresh > A.qcap) fresh = A.qcap;
+    ctrl->total = total;
     ctrl->fresh_next = lo;
     ctrl->useful = 0ull;
     ctrl->issued = 0ull;
@@ -249,17 +250,17 @@ __global__ void wave_prep_kernel(const WaveArgs* __restrict__ A, WaveCtrl* __res
     ctrl->error = 0u;
     ctrl->spills = 0u;
   }
-  if (blockIdx.x == 0 && threadIdx.x < 4u && A->grad != nullptr) A->grad[threadIdx.x] = 0.0;
-  if (A->moments != nullptr) {
-    const uint32_t nm = 5u * (A->tc.time_bins + 1u);
+  if (blockIdx.x == 0 && threadIdx.x < 4u && A.grad != nullptr) A.grad[threadIdx.x] = 0.0;
+  if (A.moments != nullptr) {
+    const uint32_t nm = 5u * (A.tc.time_bins + 1u);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += gridDim.x * blockDim.x)
-      A->moments[i] = 0.0;
+      A.moments[i] = 0.0;
   }
-  if (A->tally != nullptr && A->keep_tally == 0u) {
-    const size_t total = static_cast<size_t>(A->n_tallies) * A->tc.len;
+  if (A.tally != nullptr && A.keep_tally == 0u) {
+    const size_t total = static_cast<size_t>(A.n_tallies) * A.tc.len;
     for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x)
-      A->tally[i] = 0ull;
+      A.tally[i] = 0ull;
   }
 }
 
@@ -269,8 +270,8 @@ __global__ void wave_prep_kernel(const WaveArgs* __restrict__ A, WaveCtrl* __res
 // records (events or gensteps) are read at emission only.
 template <bool BATCH, bool UNI>
 __device__ __forceinline__ const DevParams& params_of(const DevParams& P0,
-                                                      const WaveArgs* __restrict__ A, uint32_t ev) {
-  if (BATCH && !UNI) return A->phys[ev];
+                                                      const WaveArgs& A, uint32_t ev) {
+  if (BATCH && !UNI) return A.phys[ev];
   return P0;
 }
 
@@ -281,9 +282,9 @@ template <int MINB>
 constexpr int wave_max_threads() { return MINB >= 5 ? 128 : 256; }
 
 template <int MODE, bool BATCH, int MINB, bool UNI>
-__global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(const DevParams P0,
-                                                      const WaveArgs* __restrict__ A,
-                                                      WaveCtrl* __restrict__ ctrl) {
+__global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
+    wave_kernel(const __grid_constant__ DevParams P0, const __grid_constant__ WaveArgs A,
+                WaveCtrl* __restrict__ ctrl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = threadIdx.x >> 5;
@@ -299,18 +300,17 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
   unsigned char* extra = smem_raw + nwarps * kPantryBytesPerWarp;
   uint32_t* s_hist = reinterpret_cast<uint32_t*>(extra);
   double* s_w = reinterpret_cast<double*>(extra);
-  double* s_mom = s_w + (A->tc.time_bins + 1u);  // adjoint, moments_smem: [time_bins + 1][5]
+  double* s_mom = s_w + (A.tc.time_bins + 1u);  // adjoint, moments_smem: [time_bins + 1][5]
   uint32_t* s_evc = reinterpret_cast<uint32_t*>(extra) + warp * 16u;
   __shared__ double s_red[4][16];
 
-  // Wave-constant values live in shared memory, not in each thread's registers.
+  // What changes from wave to wave lives in shared memory, not in each thread's
+  // registers; the run's arguments are kernel parameters (the constant bank).
   struct WaveShared {
     const float4* qin;
     float4* qout;
-    unsigned long long fresh_next, first_id, iter_cap;
-    uint32_t n_in, items, T, cadence, qcap, chunk, ev_shift, tail_steps, slot_cache, flags;
-    const uint32_t* tally_of;
-    TallyDev tc;
+    unsigned long long fresh_next;
+    uint32_t n_in, items, flags;
   };
   __shared__ WaveShared ws;
   if (threadIdx.x == 0) {
@@ -318,38 +318,22 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     ws.n_in = ctrl->n_in;
     ws.items = ws.n_in + ctrl->fresh_count;
     ws.fresh_next = ctrl->fresh_next;
-    ws.qin = (wave & 1u) ? A->qb : A->qa;
-    ws.qout = (wave & 1u) ? A->qa : A->qb;
-    ws.T = A->threshold;
-    ws.cadence = A->cadence;
-    ws.qcap = A->qcap;
-    ws.first_id = A->first_id;
-    ws.iter_cap = A->iter_cap;
-    ws.chunk = A->chunk < 32u ? 32u : A->chunk;
-    ws.tally_of = A->tally_of;
-    ws.ev_shift = A->ev_shift;
-    ws.tail_steps = A->tail_steps < 1u ? 1u : A->tail_steps;
-    ws.slot_cache = A->slot_cache;
-    ws.flags = (ctrl->gs_error & kFarGenstep) != 0u ? A->flags & ~kOrdinary : A->flags;
-    ws.tc = A->tc;
+    ws.qin = (wave & 1u) ? A.qb : A.qa;
+    ws.qout = (wave & 1u) ? A.qa : A.qb;
+    ws.flags = (ctrl->gs_error & kFarGenstep) != 0u ? A.flags & ~kOrdinary : A.flags;
   }
   __syncthreads();
   const uint32_t& n_in = ws.n_in;
   const uint32_t& items = ws.items;
   const unsigned long long& fresh_next = ws.fresh_next;
-  const uint32_t& T = ws.T;
-  const uint32_t& cadence = ws.cadence;
-  const uint32_t& qcap = ws.qcap;
-  const unsigned long long& first_id = ws.first_id;
-  const unsigned long long& iter_cap = ws.iter_cap;
-  const uint32_t& wchunk = ws.chunk;
-  const uint32_t& tail_steps = ws.tail_steps;
+  const uint32_t T = A.threshold, cadence = A.cadence, qcap = A.qcap, wchunk = A.chunk, tail_steps = A.tail_steps;
+  const unsigned long long first_id = A.first_id;
   // Event of a record (a genstep's event; a plain batch's records are its events).
   auto event_of = [&](uint32_t rec) -> uint32_t {
-    const uint32_t* m = ws.tally_of;
+    const uint32_t* m = A.tally_of;
     return m == nullptr ? rec : __ldg(m + rec);
   };
-  const TallyDev& tc = ws.tc;
+  const TallyDev& tc = A.tc;
   const uint32_t n_bins = tc.len - 7u;
   const bool slot_bins = n_bins <= kSlotBins;
   uint32_t* s_sb = reinterpret_cast<uint32_t*>(extra + nwarps * kSlotCounterBytesPerWarp) +
@@ -365,9 +349,9 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     }
   }
   if (kAdj) {
-    const double* wb = A->w_bin;
+    const double* wb = A.w_bin;
     for (uint32_t b = threadIdx.x; b <= tc.time_bins; b += blockDim.x) s_w[b] = wb ? wb[b] : 0.0;
-    if (MODE == kModeMoments && A->moments_smem) {
+    if (MODE == kModeMoments && A.moments_smem) {
       for (uint32_t i = threadIdx.x; i < 5u * (tc.time_bins + 1u); i += blockDim.x) s_mom[i] = 0.0;
     }
   }
@@ -409,7 +393,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
   auto flush_slot = [&](uint32_t v, uint32_t tag) {
     __syncwarp();
     if (tag != kNoEvent) {
-      unsigned long long* G = A->tally + static_cast<size_t>(tag) * tc.len;
+      unsigned long long* G = A.tally + static_cast<size_t>(tag) * tc.len;
       if (lane < 7u) {  // 5 fates, then the nb and ns sums (the last two entries)
         const uint32_t c = s_evc[v * 8u + lane];
         if (c != 0u) {
@@ -434,7 +418,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
   // Bookkeeping of a finished photon.
   auto finish = [&](uint32_t fate, const DevParams& P) {
     if (MODE == kModeRecords) {
-      store_record(A->rec, pidx, s, fate);
+      store_record(A.rec, pidx, s, fate);
     } else if (MODE == kModeTally && BATCH) {
       // 32-bit shared-memory atomics into the event's slot when the warp caches
       // it (a 64-bit shared-memory add is not one atomic instruction: u64 slots
@@ -443,7 +427,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
       // kSlotMaxAdd (so is each photon's nb and ns), and the warp flushes its
       // slots every kSlotFlushPhotons photons (at a refill): no u32 counter wraps.
       const int slot = ev == tag0 ? 0 : (ev == tag1 ? 1 : -1);
-      unsigned long long* G = A->tally + static_cast<size_t>(ev) * tc.len;
+      unsigned long long* G = A.tally + static_cast<size_t>(ev) * tc.len;
       if (slot >= 0) {
         uint32_t* C = s_evc + slot * 8;
         atomicAdd(&C[fate], 1u);
@@ -475,8 +459,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
       // Per-lane step sums stay far below 2^31 between flushes (a lane sees at
       // most wave_quota / lanes photons of max_steps steps); flush early if not.
       if (snb > 0x7fffffffu || sns > 0x7fffffffu) {
-        atomicAdd(&A->tally[tc.len - 2u], static_cast<unsigned long long>(snb));
-        atomicAdd(&A->tally[tc.len - 1u], static_cast<unsigned long long>(sns));
+        atomicAdd(&A.tally[tc.len - 2u], static_cast<unsigned long long>(snb));
+        atomicAdd(&A.tally[tc.len - 1u], static_cast<unsigned long long>(sns));
         snb = sns = 0u;
       }
       snb += s.nb;
@@ -488,21 +472,21 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     } else {  // adjoint: score terms of detected photons (see WaveArgs)
       if (fate == kDetected) {
         const uint32_t tb = time_bin(s.t, tc.tscale, tc.time_bins);
-        const double w = s_w[tb] + A->w_det;
-        double* M = MODE == kModeMoments ? A->moments : nullptr;
+        const double w = s_w[tb] + A.w_det;
+        double* M = MODE == kModeMoments ? A.moments : nullptr;
         if (w != 0.0 || M != nullptr) {
           const double path = s.path;
-          const uint32_t m = A->score_mask;
-          const double s0 = (m & 1u) ? path * A->inv_la2 : 0.0;
-          const double s1 = (m & 2u) ? path * A->inv_ls2 - static_cast<double>(s.ns) * A->inv_ls : 0.0;
-          const double s2 = (m & 4u) ? static_cast<double>(aux.n_refl) * A->inv_r : 0.0;
-          const double s3 = (m & 8u) ? static_cast<double>(aux.t_emit) * A->inv_tau2 - A->inv_tau : 0.0;
+          const uint32_t m = A.score_mask;
+          const double s0 = (m & 1u) ? path * A.inv_la2 : 0.0;
+          const double s1 = (m & 2u) ? path * A.inv_ls2 - static_cast<double>(s.ns) * A.inv_ls : 0.0;
+          const double s2 = (m & 4u) ? static_cast<double>(aux.n_refl) * A.inv_r : 0.0;
+          const double s3 = (m & 8u) ? static_cast<double>(aux.t_emit) * A.inv_tau2 - A.inv_tau : 0.0;
           g0 += w * s0;
           g1 += w * s1;
           g2 += w * s2;
           g3 += w * s3;
           if (M != nullptr) {  // per-bin (count, score sums): histogram and Jacobian in one pass
-            double* mb = (MODE == kModeMoments && A->moments_smem ? s_mom : M) + 5u * tb;
+            double* mb = (MODE == kModeMoments && A.moments_smem ? s_mom : M) + 5u * tb;
             atomicAdd(mb, 1.0);
             if (s0 != 0.0) atomicAdd(mb + 1, s0);
             if (s1 != 0.0) atomicAdd(mb + 2, s1);
@@ -542,7 +526,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
   };
 
   for (;;) {
-    if (static_cast<unsigned long long>(iters) > iter_cap) {
+    if (iters > A.iter_cap) {
       if (lane == 0u) atomicOr(&ctrl->error, kErrWatchdog);
       break;
     }
@@ -600,10 +584,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
           } else {
             const unsigned long long g = fresh_next + (item - n_in);
             npidx = static_cast<uint32_t>(g);
-            if (BATCH) nev = find_event(A, g, ws.ev_shift);
-            const DevParams& R = BATCH ? A->params[nev] : P0;  // the photon's record
+            if (BATCH) nev = find_event(A, g);
+            const DevParams& R = BATCH ? A.params[nev] : P0;  // the photon's record
             nr.init(first_id + g, R.key_lo, R.key_hi, 0u);
-            const float4* sg = A->seg == nullptr ? nullptr : A->seg + 2u * nev;
+            const float4* sg = A.seg == nullptr ? nullptr : A.seg + 2u * nev;
             start_photon<kAdj>(R, ns, nr, first_id + g, na_aux, sg);
             if (BATCH) nev = event_of(nev);  // from here on the photon needs only its event
           }
@@ -636,7 +620,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
             fm = 3u;
             since = 0u;
           }
-          if (got > 0u && ws.slot_cache) {
+          if (got > 0u && A.slot_cache) {
             const uint32_t e_first = __shfl_sync(kFull, nev, 0);
             e_last = __shfl_sync(kFull, nev, got - 1u);
             if (e_last != tag0 && e_last != tag1) {
@@ -699,7 +683,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
         // after `tail_steps` (>= 1) steps in this one: every item of a wave makes
         // progress, so the run ends, and long histories advance many steps per
         // wave instead of one step per wave once the waves are small.
-        if (na < T && !queue_full) {
+        if (na < T && !queue_full && tail_steps != kNoSpill) {
           if (spill_lanes(alive && wsteps >= tail_steps)) alive = false;
           if (__ballot_sync(kFull, alive) == 0u) break;
         }
@@ -745,7 +729,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
                      r2 = __reduce_add_sync(kFull, f2), r3 = __reduce_add_sync(kFull, f3),
                      r4 = __reduce_add_sync(kFull, f4);
       const unsigned long long wnb = warp_sum_u64(snb), wns = warp_sum_u64(sns);
-      unsigned long long* gt = A->tally;
+      unsigned long long* gt = A.tally;
       if (lane == 0u) {
         if (r0) atomicAdd(&gt[0], static_cast<unsigned long long>(r0));
         if (r1) atomicAdd(&gt[1], static_cast<unsigned long long>(r1));
@@ -776,10 +760,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
     if (threadIdx.x < 4u) {
       double acc = 0.0;
       for (uint32_t w = 0; w < nwarps; ++w) acc += s_red[threadIdx.x][w];
-      if (acc != 0.0) atomicAdd(&A->grad[threadIdx.x], acc);
+      if (acc != 0.0) atomicAdd(&A.grad[threadIdx.x], acc);
     }
-    if (MODE == kModeMoments && A->moments_smem) {  // every lane's moments are in s_mom (barrier above)
-      double* M = A->moments;
+    if (MODE == kModeMoments && A.moments_smem) {  // every lane's moments are in s_mom (barrier above)
+      double* M = A.moments;
       for (uint32_t i = threadIdx.x; i < 5u * (tc.time_bins + 1u); i += blockDim.x) {
         if (s_mom[i] != 0.0) atomicAdd(M + i, s_mom[i]);
       }
@@ -796,9 +780,9 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
       volatile WaveCtrl* vc = ctrl;
       const unsigned n_out = vc->n_out < qcap ? vc->n_out : qcap;  // reservations past qcap were not written
       const unsigned long long next = vc->fresh_next + vc->fresh_count;
-      const unsigned long long remaining = A->total - next;
-      unsigned long long fresh = remaining < A->wave_quota ? remaining : A->wave_quota;
-      if (A->cadence != 0u) {
+      const unsigned long long remaining = vc->total - next;
+      unsigned long long fresh = remaining < A.wave_quota ? remaining : A.wave_quota;
+      if (A.cadence != 0u) {
         const unsigned long long room = qcap > n_out ? qcap - n_out : 0ull;
         if (fresh > room) fresh = room;
       }
@@ -810,11 +794,11 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB) wave_kernel(co
       vc->blocks_done = 0u;
       vc->spills = vc->spills + n_out;
       vc->wave = vc->wave + 1u;
-      if (vc->wave >= A->wave_cap && (n_out + fresh) > 0ull) vc->error = vc->error | kErrWatchdog;
+      if (vc->wave >= A.wave_cap && (n_out + fresh) > 0ull) vc->error = vc->error | kErrWatchdog;
       const bool more = (n_out + fresh) > 0ull && vc->error == 0u;
       vc->active = more ? 1u : 0u;
       __threadfence();
-      if (!more && A->use_graph != 0u) cudaGraphSetConditional(A->graph_handle, 0u);
+      if (!more && A.use_graph != 0u) cudaGraphSetConditional(A.graph_handle, 0u);
     }
   }
 }
@@ -1117,9 +1101,9 @@ cudaError_t launch_history_tally(const DevParams& P, const TallyDev& tc, uint64_
 
 const void* wave_prep_fn() { return reinterpret_cast<const void*>(&wave_prep_kernel); }
 
-cudaError_t launch_wave_prep(const WaveArgs* A_dev, WaveCtrl* ctrl, int grid, int block,
+cudaError_t launch_wave_prep(const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,
                              cudaStream_t st) {
-  wave_prep_kernel<<<grid, block, 0, st>>>(A_dev, ctrl);
+  wave_prep_kernel<<<grid, block, 0, st>>>(A, ctrl);
   return cudaGetLastError();
 }
 
@@ -1165,9 +1149,9 @@ cudaError_t wave_set_smem(int mode, int batch, int minb, size_t smem) {
                               cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
 }
 
-cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const WaveArgs* A_dev,
+cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const WaveArgs& A,
                         WaveCtrl* ctrl, int grid, int block, size_t smem, cudaStream_t st) {
-  void* args[] = {const_cast<DevParams*>(&P), &A_dev, &ctrl};
+  void* args[] = {const_cast<DevParams*>(&P), const_cast<WaveArgs*>(&A), &ctrl};
   return cudaLaunchKernel(wave_kernel_fn(mode, batch, minb), dim3(grid), dim3(block), args, smem, st);
 }
 

@@ -19,8 +19,9 @@ struct TallyDev {
   uint32_t len;  // 5 + time_bins + 1 + xy_bins^2 + 2
 };
 
-// Wavefront run description, resident in device memory (the host writes it
-// before each run; kernels read it, so a captured graph stays valid).
+// Wavefront run description, a kernel parameter: the kernels read it through the
+// constant bank (from device memory each use was a dependent load, and each run an
+// upload), and a graph holds the arguments that it was made for.
 struct WaveArgs {
   const DevParams* params;              // records: events, or gensteps (1 entry when not batched)
   const DevParams* phys;                // physics per event (= params unless gensteps)
@@ -32,6 +33,7 @@ struct WaveArgs {
   uint32_t cadence;                     // steps per photon per wave before a forced spill (0 = none)
   uint32_t qcap;                        // capacity of each state queue, photons
   unsigned long long total;             // the run covers relative photons [item_lo, total)
+  const unsigned long long* total_ptr;  // where the total is read from instead (device gensteps), or null
   unsigned long long item_lo;           // first relative photon of the run (0: the whole batch)
   unsigned long long first_id;          // Philox id of relative photon 0
   unsigned long long wave_quota;        // fresh photons admitted per wave
@@ -49,13 +51,14 @@ struct WaveArgs {
   double* moments;                      // adjoint mode, optional: (time_bins + 1) x 5 FP64
                                         // per-bin (count, sum S_La, S_Ls, S_R, S_tau)
   unsigned long long graph_handle;      // cudaGraphConditionalHandle of the wave loop
-  unsigned long long iter_cap;          // watchdog: max loop iterations per warp per wave
+  uint32_t iter_cap;                    // watchdog: max loop iterations per warp per wave
   uint32_t use_graph;                   // 1: the wave loop is a graph while node (set its condition)
   uint32_t wave_cap;                    // watchdog: max waves per run
   uint32_t chunk;                       // consecutive work items a warp claims per grab (>= 32)
   uint32_t n_tallies;                   // events = tally slices (= n_events unless gensteps)
   uint32_t ev_shift;                    // ev_table resolution: one entry per 2^ev_shift photons
-  uint32_t tail_steps;                  // steps a photon makes in a wave before it may be spilled at its end
+  uint32_t tail_steps;                  // steps a photon makes in a wave before it may be spilled at its
+                                        // end (kNoSpill: photons stay in their warp until they end)
   uint32_t slot_cache;                  // batched tallies: 1 = warps may cache events in shared-memory
                                         // slots (every record's max_steps < kSlotMaxAdd)
   uint32_t flags;                       // DevParams::flags that every record has
@@ -66,6 +69,7 @@ struct WaveArgs {
 
 // Dynamic state of a wavefront run (device memory).
 struct WaveCtrl {
+  unsigned long long total;        // the run's photon total (written by the prep kernel)
   unsigned long long fresh_next;   // first fresh photon (relative index) of the current wave
   unsigned long long useful;       // lane-steps that advanced a photon
   unsigned long long issued;       // 32 x warp step iterations
@@ -98,6 +102,7 @@ constexpr uint32_t kPantryBytesPerWarp = 32u * 112u;
 // default limit is 48 KB minus the kernel's static shared memory (at most 1 KB
 // for the kernels here).
 constexpr size_t kDynSmemOptIn = 47u * 1024u;
+constexpr uint32_t kNoSpill = 0xffffffffu;
 constexpr unsigned kErrQueue = 1u, kErrWatchdog = 2u;
 // Sources beyond this (mm) are not kOrdinary.
 constexpr float kFarCoordinate = 0x1p40f;
@@ -188,7 +193,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
                                    cudaStream_t st);                                             \
   int history_tally_blocks_per_sm(int block, size_t smem);                                       \
   /* Wavefront: prep (reset ctrl, zero tallies) and one wave. */                                 \
-  cudaError_t launch_wave_prep(const WaveArgs* A_dev, WaveCtrl* ctrl, int grid, int block,       \
+  cudaError_t launch_wave_prep(const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,           \
                                cudaStream_t st);                                                 \
   const void* wave_prep_fn();                                                                    \
   /* batch: kSingle, kBatch or kBatchUniform (see WaveVariant) */                               \
@@ -196,7 +201,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
   int wave_blocks_per_sm(int mode, int batch, int minb, int block, size_t smem);                 \
   cudaError_t wave_set_smem(int mode, int batch, int minb, size_t smem);                         \
   cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P,                     \
-                          const WaveArgs* A_dev, WaveCtrl* ctrl, int grid, int block,            \
+                          const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,                \
                           size_t smem, cudaStream_t st);                                         \
   cudaError_t launch_event_table(const unsigned long long* offsets, uint32_t n_events,           \
                                  uint32_t* table, unsigned long long total, uint32_t shift,      \

@@ -85,8 +85,7 @@ struct Fresnel {
 };
 struct Box {
   __device__ bool operator()(uint64_t i) const {
-    DevParams P{};
-    P.flags = kOrdinary;
+    StepParams P{};
     P.hx = (i & 1u) ? 25.0f : 0.01f + 200.0f * unit(i, 1);
     P.hy = (i & 1u) ? 25.0f : 0.01f + 200.0f * unit(i, 2);
     P.hz = (i & 2u) ? P.hx : 0.01f + 200.0f * unit(i, 3);
