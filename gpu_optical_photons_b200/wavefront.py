@@ -28,7 +28,7 @@ class WaveConfig:
     wave_quota: int = 0         # fresh photons per wave (0 = all)
     use_graph: bool = True
     math: str = "fast"
-    chunk: int = 0              # consecutive photons a warp claims per grab (0 = 256)
+    chunk: int = 0              # consecutive photons a warp claims per grab (0 = 32 to 256 by the run's photons)
     max_gensteps: int = 0       # capacity for set_gensteps (0 = no gensteps)
     tail_steps: int = 0         # steps in a wave before a photon may move to the next (0 = 4096)
 

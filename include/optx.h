@@ -105,8 +105,8 @@ typedef struct optx_wave_config {
   uint64_t wave_quota;   /* fresh photons admitted per wave, 0 = all (default) */
   int32_t use_graph;     /* 1: waves run as a CUDA-graph while loop (default); -1: host loop */
   int32_t math;          /* OPTX_MATH_FAST / OPTX_MATH_EXACT / OPTX_MATH_APPROX */
-  uint32_t chunk;        /* consecutive photons a warp claims per grab, 32..2^20 (default 256);
-                            results do not depend on it */
+  uint32_t chunk;        /* consecutive photons a warp claims per grab, 32..2^20 (default 32 to 256
+                            by the run's photons); results do not depend on it */
   uint32_t max_gensteps; /* capacity for optx_engine_set_gensteps, 0 = none (default) */
   uint32_t tail_steps;   /* at the end of a wave a photon moves on to the next wave only after
                             this many steps in the wave (default 4096: in practice a warp keeps its

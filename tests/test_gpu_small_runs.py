@@ -1,0 +1,52 @@
+"""Runs at the edges of the engine's work distribution (claims of 32 to 256 photons
+by the run's size, the last photons of a run finished in place): tallies and records
+equal the oracle's exactly, whatever the number of photons per warp."""
+import numpy as np
+import pytest
+
+from gpu_optical_photons_b200 import params as P
+from gpu_optical_photons_b200.wavefront import WaveConfig, WavefrontEngine
+
+pytestmark = pytest.mark.gpu
+
+TC = P.TallyConfig(100, 50.0, 10)
+SETUPS = {"cube": P.config1, "lambert": P.config2, "bar": P.config3}
+
+
+# 8 x 148 x 28 warps x 64 photons = 2,121,728: where claims grow from 32 to 64 photons.
+@pytest.mark.parametrize("setup,n", [("cube", 1), ("cube", 31), ("lambert", 33), ("bar", 1000), ("lambert", 40_001),
+                                     ("lambert", 2_121_727), ("lambert", 2_121_729)])
+def test_tally_equals_oracle(engine, oracle, setup, n):
+    p = SETUPS[setup]()[0]
+    _, flat, _ = engine.run_gpu_tally(p, TC, n, first_id=9, math="exact")
+    assert np.array_equal(flat, oracle.tally(p, TC, n, 9, mode=oracle.PORTABLE))
+
+
+@pytest.mark.parametrize("max_steps", [0, 1, 2, 7, 10_000])
+@pytest.mark.parametrize("setup", sorted(SETUPS))
+def test_records_equal_oracle(engine, oracle, setup, max_steps):
+    p = SETUPS[setup]()[0].replace(max_steps=max_steps)
+    rec, _ = engine.run_gpu_records(p, 777, first_id=3, math="exact")
+    ref = oracle.records(p, 777, 3, mode=oracle.PORTABLE)
+    for k in oracle.Records.FIELDS:
+        assert np.array_equal(np.asarray(rec[k]).view(np.uint8), np.asarray(ref[k]).view(np.uint8)), k
+
+
+@pytest.mark.parametrize("cfg", [dict(), dict(blocks_per_sm=7, threshold=32), dict(tail_steps=3), dict(cadence=4),
+                                 dict(chunk=4096), dict(use_graph=False)], ids=str)
+def test_small_ragged_batch_equals_oracle(engine, oracle, cfg):
+    """Events of 0 to 700 photons, one without steps, seeds that differ per event."""
+    rng = np.random.default_rng(4)
+    counts = rng.integers(0, 700, 23).astype(np.uint64)
+    counts[[3, 7]] = 0, 1
+    events = [P.SimParams(n_det=1.5, surface=P.LAMBERTIAN, abs_length=float(np.float32(rng.uniform(200, 3000))),
+                          scat_length=float(np.float32(rng.uniform(300, 1000))), source=int(i % 2),
+                          max_steps=0 if i == 5 else 10_000, seed=100 + i // 2) for i in range(23)]
+    arr = (P.CSimParams * 23)(*[e.to_c() for e in events])
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.uint64)
+    eng = WavefrontEngine(TC, 23, int(counts.sum()), WaveConfig(math="exact", **cfg))
+    eng.set_events(events, counts)
+    eng.run_tally()
+    got = eng.tallies()
+    eng.close()
+    assert np.array_equal(got, oracle.batch_tally(arr, offs, TC, mode=oracle.PORTABLE))
