@@ -487,17 +487,24 @@ struct optx_engine {
 
 namespace {
 
-size_t wave_smem(const optx_engine* e, int mode, int variant) {
-  const bool batch = variant != kSingle;
-  const size_t pantry = static_cast<size_t>(e->cfg.block_size / 32) * kPantryBytesPerWarp;
-  if (mode == kModeTally && !batch) return pantry + static_cast<size_t>(e->tdev.len - 7u) * 4u;
-  if (mode == kModeAdjoint || mode == kModeMoments)  // bin weights, then the block's moment table
-    return pantry + static_cast<size_t>(e->tdev.time_bins + 1u) * 8u +
-           (mode == kModeMoments ? moment_smem_bytes(e->tdev.time_bins) : 0u);
-  if (mode == kModeTally && batch)  // per-warp event slots
-    return pantry + static_cast<size_t>(e->cfg.block_size / 32) *
-                        (kSlotCounterBytesPerWarp + slot_bin_bytes_per_warp(e->tdev.len - 7u));
-  return pantry;
+// Dynamic shared memory of a block of `block` threads: its warps', then the block's
+// histograms (tally) or bin weights and moment table (adjoint).
+size_t wave_extra(const TallyDev& t, int mode, bool batch) {
+  if (mode == kModeTally) return batch ? 0u : static_cast<size_t>(t.len - 7u) * 4u;
+  if (mode == kModeAdjoint || mode == kModeMoments)
+    return static_cast<size_t>(t.time_bins + 1u) * 8u + (mode == kModeMoments ? moment_smem_bytes(t.time_bins) : 0u);
+  return 0u;
+}
+size_t wave_smem(const TallyDev& t, int mode, bool batch, int block) {
+  return static_cast<size_t>(block / 32) * wave_warp_bytes(mode, batch, t.len - 7u) +
+         wave_extra(t, mode, batch);
+}
+// What counts against the device's shared memory per block when a tally is accepted
+// or refused (kLimitBytesPerWarp).
+size_t wave_smem_limit(const TallyDev& t, int mode, bool batch, int block) {
+  const size_t fixed = (mode == kModeTally ? 96u : (mode == kModeRecords ? 80u : 608u)) + (batch ? (mode == kModeTally ? 272u : 256u) : 0u);
+  const size_t slots = mode == kModeTally && batch ? kSlotCounterBytesPerWarp + slot_bin_bytes_per_warp(t.len - 7u) : 0u;
+  return static_cast<size_t>(block / 32) * (kLimitBytesPerWarp + slots) + wave_extra(t, mode, batch) + fixed;
 }
 
 // Register-budget variant of the wave kernel: 2, 3 or 4 blocks of 256 threads
@@ -508,22 +515,29 @@ int engine_minb(const optx_engine* e) {
   return std::max(2, std::min(4, b));
 }
 
-int engine_grid(optx_engine* e, int mode, int batch, int& grid) {
-  const size_t smem = wave_smem(e, mode, batch);
+// Threads per block and blocks of a run: the engine's block size, halved while the
+// histograms leave its warps no room.
+int engine_grid(optx_engine* e, int mode, int variant, int& grid, int& block) {
   const int math = e->cfg.math;
   const int minb = engine_minb(e);
+  const bool batch = variant != kSingle;
   int dev = 0, max_smem = 0;
   OPTX_CUDA(cudaGetDevice(&dev));
   OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   // The opt-in maximum covers the kernel's static shared memory too.
   cudaFuncAttributes fa{};
-  OPTX_CUDA(cudaFuncGetAttributes(&fa, DISPATCH(math, wave_kernel_fn, mode, batch, minb)));
-  if (smem + fa.sharedSizeBytes > static_cast<size_t>(max_smem))
-    return fail(OPTX_ERR_RUNTIME, "wavefront kernel needs " + std::to_string(smem + fa.sharedSizeBytes) +
+  OPTX_CUDA(cudaFuncGetAttributes(&fa, DISPATCH(math, wave_kernel_fn, mode, variant, minb)));
+  const size_t want = wave_smem_limit(e->tdev, mode, batch, e->cfg.block_size);
+  if (want > static_cast<size_t>(max_smem))
+    return fail(OPTX_ERR_RUNTIME, "wavefront kernel needs " + std::to_string(want) +
                                       " bytes of shared memory per block (" + std::to_string(max_smem) +
                                       " available); reduce xy_bins / time_bins");
-  if (smem > kDynSmemOptIn) OPTX_CUDA(DISPATCH(math, wave_set_smem, mode, batch, minb, smem));
-  int bps = DISPATCH(math, wave_blocks_per_sm, mode, batch, minb, e->cfg.block_size, smem);
+  block = e->cfg.block_size;
+  while (block > 32 && wave_smem(e->tdev, mode, batch, block) + fa.sharedSizeBytes > static_cast<size_t>(max_smem))
+    block = block / 64 * 32;
+  const size_t smem = wave_smem(e->tdev, mode, batch, block);
+  if (smem > kDynSmemOptIn) OPTX_CUDA(DISPATCH(math, wave_set_smem, mode, variant, minb, smem));
+  int bps = DISPATCH(math, wave_blocks_per_sm, mode, variant, minb, block, smem);
   if (bps <= 0) return fail(OPTX_ERR_RUNTIME, "wavefront kernel cannot be resident with this block size / tally");
   if (e->cfg.blocks_per_sm == 7) bps = std::min(bps, 7);
   else if (e->cfg.blocks_per_sm > 0) bps = std::min(bps, e->cfg.blocks_per_sm * (256 / e->cfg.block_size));
@@ -544,7 +558,7 @@ uint32_t claim_size(uint64_t photons, uint64_t warps) {
 }
 
 // The arguments of a run.
-WaveArgs engine_args(const optx_engine* e, int mode, int grid, const DevRecords* rec, const double* w_bin, double w_det,
+WaveArgs engine_args(const optx_engine* e, int mode, int warps, const DevRecords* rec, const double* w_bin, double w_det,
                      const double* theta_inv, uint32_t score_mask, double* moments) {
   WaveArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -590,9 +604,13 @@ WaveArgs engine_args(const optx_engine* e, int mode, int grid, const DevRecords*
   // Watchdog: no warp can iterate more than (photons + queue) x (max_steps + 2) times.
   uint32_t max_steps = 0;
   a.flags = ~0u;
+  a.shared_key = 1u;
+  a.keys = philox_keys(e->P0.key_lo, e->P0.key_hi);
   for (const DevParams& p : e->h_params) {
     max_steps = std::max(max_steps, p.max_steps);
     a.flags &= p.flags;
+    if (p.max_steps == 0u) a.zero_steps = 1u;
+    if (p.key_lo != e->P0.key_lo || p.key_hi != e->P0.key_hi) a.shared_key = 0u;
   }
   a.iter_cap = static_cast<uint32_t>(std::min<unsigned long long>(
       (static_cast<unsigned long long>(e->total) + e->qcap + 64ull) *
@@ -610,18 +628,18 @@ WaveArgs engine_args(const optx_engine* e, int mode, int grid, const DevRecords*
     a.iter_cap = 1ull;
   }
   a.chunk = !e->default_chunk ? e->cfg.chunk
-                              : claim_size(a.total - a.item_lo, static_cast<uint64_t>(grid) * (e->cfg.block_size / 32));
+                              : claim_size(a.total - a.item_lo, static_cast<uint64_t>(warps));
   a.tail_steps = std::max(1u, e->cfg.tail_steps);
   a.slot_cache = max_steps < kSlotMaxAdd ? 1u : 0u;  // bounds the u32 slot sums
   return a;
 }
 
-int engine_graph(optx_engine* e, int mode, int batch, int grid, const WaveArgs& args,
+int engine_graph(optx_engine* e, int mode, int batch, int grid, int block, const WaveArgs& args,
                  optx_engine::Graph** out) {
-  const size_t smem = wave_smem(e, mode, batch);
+  const size_t smem = wave_smem(e->tdev, mode, batch != kSingle, block);
   const DevParams P0 = batch == kBatch ? DevParams{} : e->P0;
   for (auto& g : e->graphs) {
-    if (g.mode == mode && g.batch == batch && g.grid == grid && g.block == e->cfg.block_size &&
+    if (g.mode == mode && g.batch == batch && g.grid == grid && g.block == block &&
         g.smem == smem && std::memcmp(&g.P0, &P0, sizeof(P0)) == 0 &&
         std::memcmp(&g.args, &args, sizeof(args)) == 0) {
       *out = &g;
@@ -632,7 +650,7 @@ int engine_graph(optx_engine* e, int mode, int batch, int grid, const WaveArgs& 
   g.mode = mode;
   g.batch = batch;
   g.grid = grid;
-  g.block = e->cfg.block_size;
+  g.block = block;
   g.smem = smem;
   g.P0 = P0;
   g.args = args;
@@ -670,7 +688,7 @@ int engine_graph(optx_engine* e, int mode, int batch, int grid, const WaveArgs& 
   cudaKernelNodeParams wp{};
   wp.func = const_cast<void*>(DISPATCH(math, wave_kernel_fn, mode, batch, engine_minb(e)));
   wp.gridDim = dim3(grid);
-  wp.blockDim = dim3(e->cfg.block_size);
+  wp.blockDim = dim3(block);
   wp.sharedMemBytes = static_cast<unsigned>(smem);
   wp.kernelParams = wave_args;
   cudaGraphNode_t n_wave;
@@ -706,17 +724,17 @@ int engine_run(optx_engine* e, int mode, const DevRecords* rec, const double* w_
   if (e->n_events == 0) return fail(OPTX_ERR_INVALID_ARGUMENT, "no events uploaded");
   // Gensteps always run batched: each lane reads its genstep's record at emission.
   const int batch = (e->n_events > 1 || e->gensteps) ? (e->uniform ? kBatchUniform : kBatch) : kSingle;
-  int grid = 0;
-  OPTX_TRY(engine_grid(e, mode, batch, grid));
-  const size_t smem = wave_smem(e, mode, batch);
+  int grid = 0, block = 0;
+  OPTX_TRY(engine_grid(e, mode, batch, grid, block));
+  const size_t smem = wave_smem(e->tdev, mode, batch != kSingle, block);
   const int math = e->cfg.math;
-  WaveArgs a = engine_args(e, mode, grid, rec, w_bin, w_det, theta_inv, score_mask, moments);
+  WaveArgs a = engine_args(e, mode, grid * (block / 32), rec, w_bin, w_det, theta_inv, score_mask, moments);
   const DevParams P0 = batch == kBatch ? DevParams{} : e->P0;
   const int prep_grid = std::max(1, std::min(grid, 4 * e->n_sm));
   const bool host_loop = e->cfg.use_graph < 0;
   if (!host_loop && !one_wave(e, a)) {
     optx_engine::Graph* g = nullptr;
-    OPTX_TRY(engine_graph(e, mode, batch, grid, a, &g));
+    OPTX_TRY(engine_graph(e, mode, batch, grid, block, a, &g));
     OPTX_CUDA(cudaEventRecord(e->ev0, st));
     OPTX_CUDA(cudaGraphLaunch(g->exec, st));
   } else {
@@ -725,7 +743,7 @@ int engine_run(optx_engine* e, int mode, const DevRecords* rec, const double* w_
     OPTX_CUDA(DISPATCH(math, launch_wave_prep, a, e->d_ctrl, prep_grid, 256, st));
     for (;;) {
       OPTX_CUDA(DISPATCH(math, launch_wave, mode, batch, engine_minb(e), P0, a, e->d_ctrl, grid,
-                         e->cfg.block_size, smem, st));
+                         block, smem, st));
       if (!host_loop) break;
       unsigned active = 0;
       OPTX_CUDA(cudaMemcpyAsync(&active, &e->d_ctrl->active, sizeof(active),
@@ -1370,8 +1388,8 @@ int optx_engine_create(const optx_tally_config* c, uint32_t max_events, uint64_t
   int grid_max = 0;
   for (int mode = 0; mode < 3; ++mode) {
     for (int b = kSingle; b <= kBatchUniform; ++b) {
-      int g = 0;
-      const int rc = engine_grid(e, mode, b, g);
+      int g = 0, block = 0;
+      const int rc = engine_grid(e, mode, b, g, block);
       if (rc != OPTX_OK && mode == kModeTally) return cleanup(rc);
       grid_max = std::max(grid_max, g);
     }
@@ -2119,6 +2137,7 @@ int optx_sorted_run(optx_sorted* s, const optx_params* p, const optx_faces* face
   a.tally = reinterpret_cast<unsigned long long*>(dev_tally);
   a.tc = td;
   if (dev_records != nullptr) a.rec = to_dev(dev_records);
+  a.keys = philox_keys(P.key_lo, P.key_hi);
   // Each photon needs at most max_steps + 1 iterations in flight, and the
   // queues admit `cap` photons at a time.
   const unsigned long long bound =
@@ -2225,15 +2244,18 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   OPTX_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kNoAllocMaxDevices) return fail(OPTX_ERR_RUNTIME, "device ordinal out of range");
   constexpr int kBlock = 256, kMinB = 4;
-  // The histograms sit in shared memory beside the 8 warps' pantries, so the
-  // longest tally is what the opt-in shared memory per block leaves (B200:
-  // 232,448 B), capped by the static tally accumulator.
+  // The histograms sit in shared memory beside the warps' windows and pantries. The
+  // longest tally is what the opt-in shared memory per block (B200: 232,448 B) leaves
+  // beside 8 warps' share of it (wave_smem_limit), capped by the static tally
+  // accumulator; the longest ones run with fewer warps per block.
   int max_optin = 0;
   OPTX_CUDA(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   cudaFuncAttributes fa{};
   OPTX_CUDA(cudaFuncGetAttributes(&fa, DISPATCH(math, wave_kernel_fn, kModeTally, kSingle, kMinB)));
-  const long long pantries = static_cast<long long>(kBlock / 32) * kPantryBytesPerWarp;
-  const long long room = static_cast<long long>(max_optin) - static_cast<long long>(fa.sharedSizeBytes) - pantries;
+  TallyDev none = td;
+  none.len = 7u;
+  const long long room = static_cast<long long>(max_optin) -
+                         static_cast<long long>(wave_smem_limit(none, kModeTally, false, kBlock));
   const uint64_t max_len = std::min<uint64_t>(kNoAllocMaxTally, room > 0 ? static_cast<uint64_t>(room / 4) + 7u : 0u);
   if (td.len > max_len)
     return fail(OPTX_ERR_INVALID_ARGUMENT,
@@ -2254,19 +2276,25 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
   const DevParams P = make_dev_params(*p, faces);
-  const size_t smem = static_cast<size_t>(kBlock / 32) * kPantryBytesPerWarp +
-                      static_cast<size_t>(td.len - 7u) * 4u;
+  int block = kBlock;
+  while (block > 32 &&
+         wave_smem(td, kModeTally, false, block) + fa.sharedSizeBytes > static_cast<size_t>(max_optin))
+    block /= 2;
+  const size_t smem = wave_smem(td, kModeTally, false, block);
   if (smem > kDynSmemOptIn) OPTX_CUDA(DISPATCH(math, wave_set_smem, kModeTally, kSingle, kMinB, smem));
-  const int bps = DISPATCH(math, wave_blocks_per_sm, kModeTally, kSingle, kMinB, kBlock, smem);
+  const int bps = DISPATCH(math, wave_blocks_per_sm, kModeTally, kSingle, kMinB, block, smem);
   if (bps <= 0)
     return fail(OPTX_ERR_RUNTIME, "tally histograms need too much shared memory; reduce xy_bins / time_bins");
-  const int grid = std::min(bps, kMinB) * num_sms();
+  const int grid = std::min(bps, kMinB * (kBlock / block)) * num_sms();
 
   WaveArgs a;
   std::memset(&a, 0, sizeof(a));
   a.n_events = 1;
   a.n_tallies = 1;
   a.flags = P.flags;
+  a.zero_steps = P.max_steps == 0u ? 1u : 0u;
+  a.shared_key = 1u;
+  a.keys = philox_keys(P.key_lo, P.key_hi);
   a.ev_shift = kEvShift;
   a.threshold = 28;
   a.cadence = 0;
@@ -2279,7 +2307,7 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   a.tally = d_tally;
   a.tc = td;
   a.use_graph = 0u;
-  a.chunk = claim_size(n, static_cast<uint64_t>(grid) * (kBlock / 32));
+  a.chunk = claim_size(n, static_cast<uint64_t>(grid) * (block / 32));
   a.tail_steps = 4096u;
   a.iter_cap = static_cast<uint32_t>(std::min<unsigned long long>(
       (static_cast<unsigned long long>(n) + a.qcap + 64ull) * (P.max_steps + 2ull) + 4096ull, 0xfffffff0ull));
@@ -2289,7 +2317,7 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   // tally accumulator (the array keeps the previous call's contents).
   OPTX_CUDA(DISPATCH(math, launch_wave_prep, a, d_ctrl, std::min(grid, 4 * num_sms()), 256, st));
   for (;;) {
-    OPTX_CUDA(DISPATCH(math, launch_wave, kModeTally, kSingle, kMinB, P, a, d_ctrl, grid, kBlock,
+    OPTX_CUDA(DISPATCH(math, launch_wave, kModeTally, kSingle, kMinB, P, a, d_ctrl, grid, block,
                        smem, st));
     unsigned active = 0;
     OPTX_CUDA(cudaMemcpyAsync(&active, &d_ctrl->active, sizeof(active), cudaMemcpyDeviceToHost, st));

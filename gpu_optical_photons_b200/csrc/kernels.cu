@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "optx_device.cuh"
 #include "optx_engine.hpp"
@@ -72,7 +73,7 @@ __device__ __forceinline__ void store_record(const DevRecords& out, uint64_t i, 
 // records and tallies do not depend on the grid. done(i, s, fate) is called
 // once per photon.
 template <class Done>
-__device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_id, uint64_t n,
+__device__ __forceinline__ void history_loop(const DevParams& P, const PhiloxKeys& K, uint64_t first_id, uint64_t n,
                                              uint64_t i, uint64_t stride, Done&& done) {
   Photon s;
   Rng r;
@@ -84,11 +85,10 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
   if (i + stride >= n) {
     if (i < n) {
       const uint64_t id = first_id + i;
-      r.init(id, P.key_lo, P.key_hi, 0u);
-      start_photon<false>(P, s, r, id, aux);
+      start_photon(P, K, s, r, id, aux);
       uint32_t fate = kMaxSteps;
       if (P.max_steps != 0u) {
-        while (step_photon<false>(P, P.flags, s, r, id, fate, aux)) {}
+        while (step_photon<false>(P, P.flags, K, s, r, id, fate, aux)) {}
       }
       done(i, s, fate);
     }
@@ -104,12 +104,11 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
       cur = i;
       i += stride;
       const uint64_t id = first_id + cur;
-      r.init(id, P.key_lo, P.key_hi, 0u);
-      start_photon<false>(P, s, r, id, aux);
+      start_photon(P, K, s, r, id, aux);
       alive = true;
       ended = P.max_steps == 0u;
     } else {
-      ended = !step_photon<false>(P, P.flags, s, r, first_id + cur, fate, aux);
+      ended = !step_photon<false>(P, P.flags, K, s, r, first_id + cur, fate, aux);
     }
     if (ended) {
       alive = false;
@@ -119,9 +118,9 @@ __device__ __forceinline__ void history_loop(const DevParams& P, uint64_t first_
 }
 
 // Blocks of up to 1024 threads (the accepted block sizes): at most 64 registers.
-__global__ void __launch_bounds__(1024, 1) history_records_kernel(const DevParams P, uint64_t first_id, uint64_t n,
+__global__ void __launch_bounds__(1024, 1) history_records_kernel(const DevParams P, const __grid_constant__ PhiloxKeys K, uint64_t first_id, uint64_t n,
                                        DevRecords out) {
-  history_loop(P, first_id, n, static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x,
+  history_loop(P, K, first_id, n, static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x,
                static_cast<uint64_t>(gridDim.x) * blockDim.x,
                [&](uint64_t i, const Photon& s, uint32_t fate) { store_record(out, i, s, fate); });
 }
@@ -142,7 +141,7 @@ __device__ __forceinline__ double warp_sum_f64(double v) {
 // Launch bounds: blocks of up to 1024 threads (the accepted block sizes), which
 // caps the kernel at 64 registers: 4 resident blocks of 256, measured 6-8 %
 // faster than the unbounded 75 registers (3 blocks) despite 12 B of spills.
-__global__ void __launch_bounds__(1024, 1) history_tally_kernel(const DevParams P, const TallyDev tc, uint64_t first_id,
+__global__ void __launch_bounds__(1024, 1) history_tally_kernel(const DevParams P, const __grid_constant__ PhiloxKeys K, const TallyDev tc, uint64_t first_id,
                                      uint64_t n, unsigned long long* __restrict__ gt) {
   extern __shared__ uint32_t s_hist[];  // [time_bins + 1 | xy_bins^2]
   const uint32_t n_bins = tc.len - 7u;
@@ -151,7 +150,7 @@ __global__ void __launch_bounds__(1024, 1) history_tally_kernel(const DevParams 
 
   uint32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0, f4 = 0;
   unsigned long long snb = 0, sns = 0;
-  history_loop(P, first_id, n, static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x,
+  history_loop(P, K, first_id, n, static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x,
                static_cast<uint64_t>(gridDim.x) * blockDim.x,
                [&](uint64_t, const Photon& s, uint32_t fate) {
                  f0 += fate == 0u;
@@ -221,6 +220,9 @@ __global__ void event_table_kernel(const unsigned long long* __restrict__ offset
   }
 }
 
+__device__ __forceinline__ uint4 __float4_as_uint4(float4 v) {
+  return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+}
 __device__ __forceinline__ float4 make_uint4_as_float4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   return make_float4(__uint_as_float(a), __uint_as_float(b), __uint_as_float(c), __uint_as_float(d));
 }
@@ -290,18 +292,31 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t nwarps = blockDim.x >> 5;
-  // [pantries: nwarps x 32 x 112 B][block histograms (tally), bin weights (adjoint)
-  //  or, batched tally, per-warp event slots: nwarps x 2 x 8 u32 counters, then
-  //  nwarps x 2 x n_bins u32 bins when n_bins <= kSlotBins]
+  // [per warp (wave_warp_bytes): ring windows | pantry | batched: bookkeeping | batched
+  //  tally: 2 x 8 u32 slot counters, then 2 x n_bins u32 bins when n_bins <=
+  //  kSlotBins][block histograms (tally), bin weights (adjoint)]
   constexpr bool kSlots = BATCH && MODE == kModeTally;
   constexpr bool kAdj = MODE == kModeAdjoint || MODE == kModeMoments;  // replay modes
   constexpr bool kPath = MODE != kModeTally;  // tallies do not use the path length
-  float4* pantry = reinterpret_cast<float4*>(smem_raw + warp * kPantryBytesPerWarp);
-  unsigned char* extra = smem_raw + nwarps * kPantryBytesPerWarp;
+  constexpr bool kRing = wave_ring(MODE, BATCH);
+  constexpr uint32_t kEntry = pantry_vec4(MODE, BATCH);
+  const uint32_t warp_bytes = wave_warp_bytes(MODE, BATCH, A.tc.len - 7u);
+  // The key that the run's photons share (batched: if A.shared_key): its round keys, or
+  // its two words where the schedule comes out on the uniform datapath anyway (with
+  // the table the single-configuration kernels spill: Lambertian cube 14.01 -> 14.35 ms).
+  constexpr bool kSharedKey = !BATCH || UNI;
+  auto run_key = [&]() -> decltype(auto) {
+    if constexpr (BATCH) return (A.keys);
+    else return make_uint2(P0.key_lo, P0.key_hi);
+  };
+  unsigned char* mine = smem_raw + warp * warp_bytes;
+  float4* pantry = reinterpret_cast<float4*>(mine + (kRing ? kWindowBytesPerWarp : 0u));
+  uint32_t* s_book = reinterpret_cast<uint32_t*>(pantry + 32u * kEntry);
+  unsigned char* extra = smem_raw + nwarps * warp_bytes;
   uint32_t* s_hist = reinterpret_cast<uint32_t*>(extra);
   double* s_w = reinterpret_cast<double*>(extra);
   double* s_mom = s_w + (A.tc.time_bins + 1u);  // adjoint, moments_smem: [time_bins + 1][5]
-  uint32_t* s_evc = reinterpret_cast<uint32_t*>(extra) + warp * 16u;
+  uint32_t* s_evc = s_book + kBookWords;
   __shared__ double s_red[4][16];
 
   // What changes from wave to wave lives in shared memory, not in each thread's
@@ -336,8 +351,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   const TallyDev& tc = A.tc;
   const uint32_t n_bins = tc.len - 7u;
   const bool slot_bins = n_bins <= kSlotBins;
-  uint32_t* s_sb = reinterpret_cast<uint32_t*>(extra + nwarps * kSlotCounterBytesPerWarp) +
-                   warp * 2u * n_bins;  // this warp's [2][n_bins] (when slot_bins)
+  uint32_t* s_sb = s_evc + 16;  // [2][n_bins] (when slot_bins)
 
   if (MODE == kModeTally && !BATCH) {
     for (uint32_t b = threadIdx.x; b < n_bins; b += blockDim.x) s_hist[b] = 0u;
@@ -358,7 +372,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   __syncthreads();
 
   Photon s{};
-  Rng r{};
+  std::conditional_t<kRing, Window, Rng> r{};
+  if constexpr (kRing) r.ring = reinterpret_cast<float*>(mine) + lane * kWindowWords;
   ScoreAux aux{0u, 0.0f};
   uint32_t pidx = 0u, ev = 0u;
   bool alive = false;
@@ -371,11 +386,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   // memory (measured: fewer local-memory spills, -2.5 % per photon-step on the
   // batch), the single-configuration ones in registers.
   constexpr uint32_t kNoEvent = 0xffffffffu;
-  // [warp][chunk_lo, chunk_hi, tag0, tag1, victim, photons since the last slot flush]
-  __shared__ uint32_t s_book[8][8];
+  // [chunk_lo, chunk_hi, tag0, tag1, victim, photons since the last slot flush]
   uint32_t r_book[6] = {0u, 0u, kNoEvent, kNoEvent, 0u, 0u};
-  uint32_t* book = BATCH ? s_book[warp] : r_book;
-  if (BATCH && lane < 6u) s_book[warp][lane] = (lane == 2u || lane == 3u) ? kNoEvent : 0u;
+  uint32_t* book = BATCH ? s_book : r_book;
+  if (BATCH && lane < 6u) s_book[lane] = (lane == 2u || lane == 3u) ? kNoEvent : 0u;
   __syncwarp();
   uint32_t& chunk_lo = book[0];
   uint32_t& chunk_hi = book[1];
@@ -561,11 +575,15 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         uint32_t nev = 0u;
         if (lane < got) {
           const uint32_t item = lane < got1 ? base1 + lane : base2 + (lane - got1);
+          const bool fresh = item >= n_in;
           Photon ns{};
-          Rng nr{};
           ScoreAux na_aux{0u, 0.0f};
-          uint32_t npidx;
-          if (item < n_in) {
+          uint32_t npidx, draws = 0u;
+          if (fresh) {
+            const unsigned long long g = fresh_next + (item - n_in);
+            npidx = static_cast<uint32_t>(g);
+            if (BATCH) nev = find_event(A, g);
+          } else {
             // A survivor of the previous wave: 4 x 128-bit loads from its tile.
             const float4* q = ws.qin + qidx(item);
             const float4 a = q[0], b = q[32], c = q[64], d = q[96];
@@ -573,37 +591,58 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
             ns.dx = b.x; ns.dy = b.y; ns.dz = b.z; ns.path = b.w;
             ns.nb = __float_as_uint(c.x);
             ns.ns = __float_as_uint(c.y);
+            draws = __float_as_uint(c.z);
             npidx = __float_as_uint(c.w);
             if (kAdj) {
               na_aux.n_refl = __float_as_uint(d.x);
               na_aux.t_emit = d.y;
             }
             nev = __float_as_uint(d.z);
-            const DevParams& P = params_of<BATCH, UNI>(P0, A, nev);
-            nr.init(first_id + npidx, P.key_lo, P.key_hi, __float_as_uint(c.z));
+          }
+          // Its record (a fresh photon's, or the event's: the key is the same).
+          const DevParams& R = !BATCH ? P0 : (fresh ? A.params[nev] : A.phys[nev]);
+          const uint64_t id = first_id + npidx;
+          const uint32_t b0 = draws >> 2;
+          // The window's blocks (two in registers, three in the ring) as independent
+          // chains: instruction-level parallelism.
+          const bool shared_key = kSharedKey || A.shared_key != 0u;
+          uint4 w0, w1, w2{};
+          if (shared_key) {
+            w0 = philox10(philox_counter(b0, id), run_key());
+            w1 = philox10(philox_counter(b0 + 1u, id), run_key());
+            if (kRing) w2 = philox10(philox_counter(b0 + 2u, id), run_key());
           } else {
-            const unsigned long long g = fresh_next + (item - n_in);
-            npidx = static_cast<uint32_t>(g);
-            if (BATCH) nev = find_event(A, g);
-            const DevParams& R = BATCH ? A.params[nev] : P0;  // the photon's record
-            nr.init(first_id + g, R.key_lo, R.key_hi, 0u);
-            const float4* sg = A.seg == nullptr ? nullptr : A.seg + 2u * nev;
-            start_photon<kAdj>(R, ns, nr, first_id + g, na_aux, sg);
+            const uint32_t k0 = R.key_lo, k1 = R.key_hi;
+            w0 = philox10(philox_counter(b0, id), k0, k1);
+            w1 = philox10(philox_counter(b0 + 1u, id), k0, k1);
+            w2 = philox10(philox_counter(b0 + 2u, id), k0, k1);
+          }
+          if (fresh) {
+            const float u[6] = {to_uniform(w0.x), to_uniform(w0.y), to_uniform(w0.z),
+                                to_uniform(w0.w), to_uniform(w1.x), to_uniform(w1.y)};
+            draws = start_photon<kAdj>(R, ns, u, na_aux, A.seg == nullptr ? nullptr : A.seg + 2u * nev);
+            if (draws >= 4u) {  // block 0 is used up
+              const uint4 c = philox_counter(kRing ? 3u : 2u, id);
+              const uint4 next = shared_key ? philox10(c, run_key()) : philox10(c, R.key_lo, R.key_hi);
+              w0 = w1;
+              w1 = kRing ? w2 : next;
+              w2 = next;
+            }
             if (BATCH) nev = event_of(nev);  // from here on the photon needs only its event
           }
-          float4* e = pantry + (pc + lane) * 7u;
+          float4* e = pantry + (pc + lane) * kEntry;
           e[0] = make_float4(ns.px, ns.py, ns.pz, ns.t);
-          e[1] = make_float4(ns.dx, ns.dy, ns.dz, ns.path);
+          e[1] = make_float4(ns.dx, ns.dy, ns.dz, __uint_as_float(draws));
           e[2] = make_uint4_as_float4(ns.nb, ns.ns, npidx, nev);
-          e[3] = make_uint4_as_float4(nr.w[0], nr.w[1], nr.w[2], nr.w[3]);
-          e[4] = make_uint4_as_float4(nr.w[4], nr.w[5], nr.w[6], nr.w[7]);
-          if (kAdj) {
-            e[5] = make_float4(__uint_as_float(nr.o), __uint_as_float(nr.blk),
-                               __uint_as_float(na_aux.n_refl), na_aux.t_emit);
+          if constexpr (kRing) {
+            e[3] = make_float4(to_uniform(w0.x), to_uniform(w0.y), to_uniform(w0.z), to_uniform(w0.w));
+            e[4] = make_float4(to_uniform(w1.x), to_uniform(w1.y), to_uniform(w1.z), to_uniform(w1.w));
+            e[5] = make_float4(to_uniform(w2.x), to_uniform(w2.y), to_uniform(w2.z), to_uniform(w2.w));
           } else {
-            reinterpret_cast<float2*>(e + 5)[0] =
-                make_float2(__uint_as_float(nr.o), __uint_as_float(nr.blk));
+            e[3] = make_uint4_as_float4(w0.x, w0.y, w0.z, w0.w);
+            e[4] = make_uint4_as_float4(w1.x, w1.y, w1.z, w1.w);
           }
+          if (kPath) e[kEntry - 1u] = make_float4(ns.path, __uint_as_float(na_aux.n_refl), na_aux.t_emit, 0.0f);
         }
         pc += got;
         if (kSlots) {
@@ -643,34 +682,39 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         const uint32_t take = min(need, pc);
         const uint32_t rank = static_cast<uint32_t>(__popc(~amask & lt));
         if (!alive && rank < take) {
-          const float4* e = pantry + (pc - 1u - rank) * 7u;
-          const float4 a = e[0], b = e[1], c = e[2], d = e[3], f = e[4];
+          const float4* e = pantry + (pc - 1u - rank) * kEntry;
+          const float4 a = e[0], b = e[1], c = e[2];
           s.px = a.x; s.py = a.y; s.pz = a.z; s.t = a.w;
           s.dx = b.x; s.dy = b.y; s.dz = b.z;
-          if (kPath) s.path = b.w;
           s.nb = __float_as_uint(c.x);
           s.ns = __float_as_uint(c.y);
           pidx = __float_as_uint(c.z);
           ev = __float_as_uint(c.w);
-          r.w[0] = __float_as_uint(d.x); r.w[1] = __float_as_uint(d.y);
-          r.w[2] = __float_as_uint(d.z); r.w[3] = __float_as_uint(d.w);
-          r.w[4] = __float_as_uint(f.x); r.w[5] = __float_as_uint(f.y);
-          r.w[6] = __float_as_uint(f.z); r.w[7] = __float_as_uint(f.w);
-          if (kAdj) {
-            const float4 h = e[5];
-            r.o = __float_as_uint(h.x);
-            r.blk = __float_as_uint(h.y);
-            aux.n_refl = __float_as_uint(h.z);
-            aux.t_emit = h.w;
+          const uint32_t draws = __float_as_uint(b.w);
+          if constexpr (kRing) {
+            float4* w = reinterpret_cast<float4*>(r.ring);
+            w[0] = e[3];
+            w[1] = e[4];
+            w[2] = e[5];
+            r.rp = draws & 3u;
+            r.av = kWindowWords - r.rp;
+            r.made = (draws >> 2) + kWindowWords / 4u;
           } else {
-            const float2 h = reinterpret_cast<const float2*>(e + 5)[0];
-            r.o = __float_as_uint(h.x);
-            r.blk = __float_as_uint(h.y);
+            r.set(__float4_as_uint4(e[3]), __float4_as_uint4(e[4]), draws);
           }
-          const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
+          if (kPath) {
+            const float4 h = e[kEntry - 1u];
+            s.path = h.x;
+            aux.n_refl = __float_as_uint(h.y);
+            aux.t_emit = h.z;
+          }
           wsteps = 0u;
-          alive = s.nb + s.ns < P.max_steps;
-          if (!alive) finish(kMaxSteps, P);
+          alive = true;
+          if (A.zero_steps != 0u) {  // a photon that may not step at all
+            const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
+            alive = s.nb + s.ns < P.max_steps;
+            if (!alive) finish(kMaxSteps, P);
+          }
         }
         pc -= take;
         __syncwarp();
@@ -692,21 +736,34 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
 
     // One step for every live lane; the lanes whose photon ended reconverge
     // here to record it together (one pass of the tally code per warp step).
-    // Batched variants also reconverge inside the step before the Philox
-    // advance (measured: -6 % per photon-step on the batch; the
-    // single-configuration kernels gain nothing from it and spill more).
-    const uint32_t smask = BATCH ? __ballot_sync(kFull, alive) : 0u;
     uint32_t fate = kMaxSteps;
     bool ended = false;
     if (alive) {
       const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
-      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, s, r, first_id + pidx, fate, aux, smask);
+      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, run_key(), s, r, first_id + pidx, fate, aux);
       ++wsteps;
     }
     __syncwarp();
     if (ended) {
       alive = false;
       finish(fate, params_of<BATCH, UNI>(P0, A, ev));
+    }
+    if constexpr (kRing) {
+      // Windows: while a live lane lacks the words of a step, every lane with room for
+      // a block makes one.
+      __syncwarp();
+#pragma unroll 1
+      while (__any_sync(kFull, alive && r.av < kStepWords)) {
+        if (alive && r.av <= kWindowRoom) {
+          const uint4 c = philox_counter(r.made, first_id + pidx);
+          if (kSharedKey || A.shared_key != 0u) {
+            r.put(philox10(c, run_key()));
+          } else {  // batched: from the event's record
+            r.put(philox10(c, __ldg(reinterpret_cast<const uint2*>(&A.phys[ev].key_lo))));
+          }
+        }
+        __syncwarp();
+      }
     }
     ++iters;
     useful += na;
@@ -848,7 +905,7 @@ __global__ void sorted_prep_kernel(const SortArgs A, SortCtrl* __restrict__ ctrl
 
 template <int MINB>
 __global__ void __launch_bounds__(kSortThreads, MINB)
-    sorted_kernel(const DevParams P, const SortArgs A, SortCtrl* __restrict__ ctrl) {
+    sorted_kernel(const DevParams P, const __grid_constant__ SortArgs A, SortCtrl* __restrict__ ctrl) {
   // Host-loop launches past the end of the run do nothing (the flag only changes
   // in the last block of a launch, after every block has read it).
   if (ctrl->active == 0u) return;
@@ -907,14 +964,13 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         r.blk = v4.w;
       } else {
         rel = static_cast<uint32_t>(emit_base + idx);
-        r.init(A.first_id + rel, P.key_lo, P.key_hi, 0u);
-        start_photon<false>(P, s, r, A.first_id + rel, aux);
+        start_photon(P, A.keys, s, r, A.first_id + rel, aux);
       }
     }
     const uint64_t id = A.first_id + rel;
     if (seg < 3u) {
       const uint32_t m = __ballot_sync(kFull, valid);
-      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, s, r, id, fate, aux, hit, m);
+      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, A.keys, s, r, id, fate, aux, hit, m);
     }
 
     int next = -1;
@@ -924,7 +980,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         fate = kMaxSteps;
         live = false;
       }
-      while (live) live = step_photon<false>(P, P.flags, s, r, id, fate, aux);
+      while (live) live = step_photon<false>(P, P.flags, A.keys, s, r, id, fate, aux);
     } else if (live) {
       // Photons that have made max_steps steps end here (each live step counted
       // one boundary or one scatter).
@@ -1074,7 +1130,8 @@ cudaError_t launch_history_records(const DevParams& P, uint64_t first_id, uint64
       bps < 1)
     bps = 1;
   const uint64_t grid = std::min<uint64_t>((n + block - 1) / block, static_cast<uint64_t>(bps) * sms);
-  history_records_kernel<<<static_cast<unsigned>(grid), block, 0, st>>>(P, first_id, n, out);
+  history_records_kernel<<<static_cast<unsigned>(grid), block, 0, st>>>(P, philox_keys(P.key_lo, P.key_hi), first_id, n,
+                                                                        out);
   return cudaGetLastError();
 }
 
@@ -1095,7 +1152,7 @@ cudaError_t launch_history_tally(const DevParams& P, const TallyDev& tc, uint64_
         history_tally_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  history_tally_kernel<<<grid, block, smem, st>>>(P, tc, first_id, n, tally);
+  history_tally_kernel<<<grid, block, smem, st>>>(P, philox_keys(P.key_lo, P.key_hi), tc, first_id, n, tally);
   return cudaGetLastError();
 }
 

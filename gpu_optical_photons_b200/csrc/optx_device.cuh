@@ -107,6 +107,28 @@ __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1) {
   return c;
 }
 
+// The same with the round keys of one key made beforehand (philox_keys), in the
+// constant bank: no key additions for the batched kernels, whose photons usually
+// share a key, and for the history kernels (device tally of 1e8 bar photons 43.2 ->
+// 42.0 ms, 10 registers fewer).
+struct PhiloxKeys {
+  uint32_t k0[10], k1[10];
+};
+__device__ __forceinline__ uint4 philox10(uint4 c, const PhiloxKeys& K) {
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const unsigned long long p0 = static_cast<unsigned long long>(0xD2511F53u) * c.x;
+    const unsigned long long p1 = static_cast<unsigned long long>(0xCD9E8D57u) * c.z;
+    c = make_uint4(static_cast<uint32_t>(p1 >> 32) ^ c.y ^ K.k0[r], static_cast<uint32_t>(p1),
+                   static_cast<uint32_t>(p0 >> 32) ^ c.w ^ K.k1[r], static_cast<uint32_t>(p0));
+  }
+  return c;
+}
+__device__ __forceinline__ uint4 philox10(uint4 c, uint2 key) { return philox10(c, key.x, key.y); }
+__device__ __forceinline__ uint4 philox_counter(uint32_t block, uint64_t id) {
+  return make_uint4(block, 0u, static_cast<uint32_t>(id), static_cast<uint32_t>(id >> 32));
+}
+
 // (bits >> 8) + 1 times 2^-24, in (0, 1], exact (philox.hpp:82-84).
 __device__ __forceinline__ float to_uniform(uint32_t bits) {
   // One FMA for the addition and the scaling: the sum is at most 2^24, so exact.
@@ -121,6 +143,7 @@ __device__ __forceinline__ float to_uniform(uint32_t bits) {
 // parameters, the id is first id + photon index), which keeps the per-lane state
 // at 10 registers.
 struct Rng {
+  static constexpr bool kRefilledByCaller = false;
   uint32_t w[8];
   uint32_t o, blk;
 
@@ -128,15 +151,16 @@ struct Rng {
   // (philox.hpp:117-134): blocks draws/4 and draws/4 + 1 fill the window, as two
   // independent Philox chains (instruction-level parallelism: -1 % on the batch,
   // -3 % on the history kernels).
-  __device__ __forceinline__ void init(uint64_t id, uint32_t key_lo, uint32_t key_hi,
-                                       uint32_t draws) {
+  template <class K>
+  __device__ __forceinline__ void init(uint64_t id, const K& key, uint32_t draws) {
     const uint32_t block = draws >> 2;
-    const uint32_t lo = static_cast<uint32_t>(id), hi = static_cast<uint32_t>(id >> 32);
-    const uint4 b0 = philox10(make_uint4(block, 0u, lo, hi), key_lo, key_hi);
-    const uint4 b1 = philox10(make_uint4(block + 1u, 0u, lo, hi), key_lo, key_hi);
+    set(philox10(philox_counter(block, id), key), philox10(philox_counter(block + 1u, id), key), draws);
+  }
+  // The window from its two blocks, `draws` words into the stream.
+  __device__ __forceinline__ void set(const uint4& b0, const uint4& b1, uint32_t draws) {
     w[0] = b0.x; w[1] = b0.y; w[2] = b0.z; w[3] = b0.w;
     w[4] = b1.x; w[5] = b1.y; w[6] = b1.z; w[7] = b1.w;
-    blk = block;
+    blk = draws >> 2;
     o = draws & 3u;
   }
   __device__ __forceinline__ uint32_t draws() const { return 4u * blk + o; }
@@ -152,20 +176,59 @@ struct Rng {
   __device__ __forceinline__ float uniform() const { return to_uniform(word<I>()); }
 
   // Consumes k words; slides the window (one Philox call per block used up).
-  __device__ __forceinline__ void advance(uint32_t k, uint64_t id, uint32_t key_lo,
-                                          uint32_t key_hi) {
+  template <class K>
+  __device__ __forceinline__ void advance(uint32_t k, uint64_t id, const K& key) {
     o += k;
 #pragma unroll 1
     while (o >= 4u) {
       w[0] = w[4]; w[1] = w[5]; w[2] = w[6]; w[3] = w[7];
       ++blk;
-      const uint4 b = philox10(make_uint4(blk + 1u, 0u, static_cast<uint32_t>(id),
-                                          static_cast<uint32_t>(id >> 32)), key_lo, key_hi);
+      const uint4 b = philox10(philox_counter(blk + 1u, id), key);
       w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
       o -= 4u;
     }
   }
 };
+
+// The photon's random stream as up to 12 unread uniforms (three Philox blocks) in a
+// ring in shared memory, for kernels that refill all lanes of a warp together: a
+// photon holds three registers of it instead of ten, a step reads its words with
+// indexed loads instead of selects, words are turned into uniforms once, and with
+// more than a step's words in hand most warp steps need one Philox pass, not two (a
+// photon starts with 9 words or 10, a bounce reads 5). For the batched variants,
+// whose registers are the scarcest: against the register window the 4096-event batch
+// ran 8.61 -> 8.13 ms, 512 events of gensteps 0.854 -> 0.807. One configuration keeps
+// the register window: a polished or specular step reads three words, and the ring's
+// shared-memory round trip cost more (polished cube 1e8 photons 8.48 -> 9.26 ms, bar
+// 26.8 -> 28.1, Lambertian cube 14.13 -> 14.10), except in the adjoint replays.
+// Invariant between steps: av >= 5; rp + av is a multiple of 4, so a block is one
+// aligned 128-bit store.
+constexpr uint32_t kWindowWords = 12u;
+struct Window {
+  static constexpr bool kRefilledByCaller = true;
+  float* ring;    // this photon's kWindowWords places
+  uint32_t rp;    // place of the next unread word
+  uint32_t av;    // unread words
+  uint32_t made;  // Philox blocks made so far
+  __device__ __forceinline__ uint32_t draws() const { return 4u * made - av; }
+  // j mod kWindowWords for j < 2 kWindowWords: the difference wraps around below 0.
+  static __device__ __forceinline__ uint32_t wrap(uint32_t j) { return min(j, j - kWindowWords); }
+  template <int I>
+  __device__ __forceinline__ float uniform() const { return ring[wrap(rp + I)]; }
+  __device__ __forceinline__ void consume(uint32_t k) {
+    rp = wrap(rp + k);
+    av -= k;
+  }
+  // Appends block `made`; av <= kWindowWords - 4.
+  __device__ __forceinline__ void put(const uint4& v) {
+    *reinterpret_cast<float4*>(ring + wrap(rp + av)) =
+        make_float4(to_uniform(v.x), to_uniform(v.y), to_uniform(v.z), to_uniform(v.w));
+    av += 4u;
+    ++made;
+  }
+};
+// Words a step reads at most, and room for another block.
+constexpr uint32_t kStepWords = 5u, kWindowRoom = kWindowWords - 4u;
 
 // ---------------------------------------------------------------------------
 // Correctly rounded quotient, reciprocal and square root without a branch: the
@@ -323,13 +386,6 @@ __device__ __forceinline__ StepParams load_step(const DevParams& P) {
   return {P.hx, P.hy, P.hz, P.inv_speed, P.abs_length, P.scat_length, P.max_steps, P.surf_bits};
 }
 
-// The two words of the Philox key.
-template <bool GP>
-__device__ __forceinline__ uint2 load_key(const DevParams& P) {
-  if (GP) return __ldg(reinterpret_cast<const uint2*>(&P.key_lo));
-  return make_uint2(P.key_lo, P.key_hi);
-}
-
 // Branch-free orthonormal basis (Duff et al., JCGT 6(1) 2017) and rotation
 // about `axis` by polar cosine ct and azimuth 2 pi * phi_u (vec3.hpp:35-53).
 __device__ __forceinline__ void rotate_about(float ax, float ay, float az, float ct, float phi_u,
@@ -427,34 +483,31 @@ __device__ __forceinline__ bool fresnel_reflects(float n1, float n2, float eta2,
 // (end x, y, z, t0) and (dt, -, -, -) of the photon's genstep (null otherwise).
 constexpr uint32_t kSourceSegment = 2u;
 
+// `u`: the first six uniforms of the stream. Returns the words used (3 or 6).
 template <bool AUX>
-__device__ __forceinline__ void start_photon(const DevParams& P, Photon& s, Rng& r, uint64_t id,
-                                             ScoreAux& aux, const float4* seg = nullptr) {
-  uint32_t k;
-  float t_start = 0.0f;
+__device__ __forceinline__ uint32_t start_photon(const DevParams& P, Photon& s, const float (&u)[6], ScoreAux& aux,
+                                                 const float4* seg = nullptr) {
+  float t_start = 0.0f, ua = u[0], ub = u[1], ue = u[2];
   if (P.source == 0u) {
     s.px = P.src_x;
     s.py = P.src_y;
     s.pz = P.src_z;
-    k = 3u;
-  } else if (P.source == 1u) {
-    const float u1 = r.uniform<0>(), u2 = r.uniform<1>(), u3 = r.uniform<2>();
-    s.px = P.hx * (2.0f * u1 - 1.0f);
-    s.py = P.hy * (2.0f * u2 - 1.0f);
-    s.pz = P.hz * (2.0f * u3 - 1.0f);
-    r.o += 3u;  // o stays <= 3: the window still holds the next 5 words
-    k = 3u;
   } else {
-    const float4 e = seg[0], w = seg[1];
-    const float u1 = r.uniform<0>(), u2 = r.uniform<1>();
-    s.px = P.src_x + u1 * (e.x - P.src_x);
-    s.py = P.src_y + u1 * (e.y - P.src_y);
-    s.pz = P.src_z + u1 * (e.z - P.src_z);
-    t_start = e.w + u2 * w.x;
-    r.o += 3u;
-    k = 3u;
+    if (P.source == 1u) {
+      s.px = P.hx * (2.0f * u[0] - 1.0f);
+      s.py = P.hy * (2.0f * u[1] - 1.0f);
+      s.pz = P.hz * (2.0f * u[2] - 1.0f);
+    } else {
+      const float4 e = seg[0], w = seg[1];
+      s.px = P.src_x + u[0] * (e.x - P.src_x);
+      s.py = P.src_y + u[0] * (e.y - P.src_y);
+      s.pz = P.src_z + u[0] * (e.z - P.src_z);
+      t_start = e.w + u[1] * w.x;
+    }
+    ua = u[3];
+    ub = u[4];
+    ue = u[5];
   }
-  const float ua = r.uniform<0>(), ub = r.uniform<1>(), ue = r.uniform<2>();
   const float ct = 2.0f * ua - 1.0f;
   const float st = m_sqrt(fmaxf(0.0f, 1.0f - ct * ct));
   float sp, cp;
@@ -468,7 +521,16 @@ __device__ __forceinline__ void start_photon(const DevParams& P, Photon& s, Rng&
   s.path = 0.0f;
   s.nb = 0u;
   s.ns = 0u;
-  r.advance(k, id, P.key_lo, P.key_hi);
+  return P.source == 0u ? 3u : 6u;
+}
+// The same with the register window, from the start of the stream.
+template <class K>
+__device__ __forceinline__ void start_photon(const DevParams& P, const K& key, Photon& s, Rng& r, uint64_t id,
+                                             ScoreAux& aux) {
+  r.init(id, key, 0u);
+  const float u[6] = {to_uniform(r.w[0]), to_uniform(r.w[1]), to_uniform(r.w[2]),
+                      to_uniform(r.w[3]), to_uniform(r.w[4]), to_uniform(r.w[5])};
+  r.advance(start_photon<false>(P, s, u, aux), id, key);
 }
 
 // A step's interaction, decided by step_move: a face index 0..5 (a boundary
@@ -525,9 +587,9 @@ __device__ __forceinline__ void box_exit(const StepParams& P, uint32_t flags, co
 // scattering distances (window words 0 and 1), the box exit, and the move to the
 // nearest of the three. Returns the interaction; the window is not advanced. Without
 // PATH the path length is left alone (tallies do not use it).
-template <bool PATH = true>
-__device__ __forceinline__ int step_move(const StepParams& P, uint32_t flags, Photon& s, const Rng& r) {
-  const float u_abs = r.uniform<0>(), u_sca = r.uniform<1>();
+template <bool PATH = true, class R>
+__device__ __forceinline__ int step_move(const StepParams& P, uint32_t flags, Photon& s, const R& r) {
+  const float u_abs = r.template uniform<0>(), u_sca = r.template uniform<1>();
   float dist;
   int face;
   box_exit(P, flags, s, dist, face);
@@ -572,15 +634,15 @@ __device__ __forceinline__ uint32_t face_model(uint32_t surf_bits, int face) {
 // this step together) the warp reconverges before the advance, so the Philox block
 // runs once per warp step for all lanes that need one rather than once per
 // divergent group.
-template <bool AUX, bool GP = false>
-__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags, Photon& s, Rng& r,
-                                         uint64_t id, uint32_t& fate, ScoreAux& aux, int hit,
+template <bool AUX, bool GP = false, class R, class K>
+__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags,
+                                         const K& key, Photon& s, R& r, uint64_t id, uint32_t& fate, ScoreAux& aux, int hit,
                                          uint32_t sync_mask = 0u) {
   const int face = hit;
   const int axis = face >> 1;
   // The window's words 2..4 as uniforms, once for every outcome (measured -2 % on
   // the batch against drawing them where an outcome uses them).
-  const float u2 = r.uniform<2>(), u3 = r.uniform<3>(), u4 = r.uniform<4>();
+  const float u2 = r.template uniform<2>(), u3 = r.template uniform<3>(), u4 = r.template uniform<4>();
   const bool scattered = hit == kHitScatter, surface = hit < kHitScatter;
   const uint32_t model = face_model(surf_bits, face);
   bool kept = false;
@@ -629,8 +691,9 @@ __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits,
   if (sync_mask != 0u) __syncwarp(sync_mask);
   if (live) {
     fate = kMaxSteps;
-    const uint2 key = load_key<GP>(P);
-    r.advance(scattered ? 4u : (diffuse ? 5u : 3u), id, key.x, key.y);
+    const uint32_t k = scattered ? 4u : (diffuse ? 5u : 3u);
+    if constexpr (R::kRefilledByCaller) r.consume(k);
+    else r.advance(k, id, key);
   }
   return live;
 }
@@ -638,13 +701,13 @@ __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits,
 // One step (transport.hpp:71-145): move, then interact. `flags`: those that hold for
 // every record of the run. False when the photon has ended, with its fate, or has
 // made max_steps steps (the fate is then kMaxSteps).
-template <bool AUX, bool GP = false, bool PATH = true>
-__device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, Photon& s, Rng& r, uint64_t id,
-                                            uint32_t& fate, ScoreAux& aux,
+template <bool AUX, bool GP = false, bool PATH = true, class R, class K>
+__device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, const K& key, Photon& s,
+                                            R& r, uint64_t id, uint32_t& fate, ScoreAux& aux,
                                             uint32_t sync_mask = 0u) {
   const StepParams q = load_step<GP>(P);
   const int hit = step_move<PATH>(q, flags, s, r);
-  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, s, r, id, fate, aux, hit, sync_mask);
+  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, key, s, r, id, fate, aux, hit, sync_mask);
   return live && s.nb + s.ns < q.max_steps;
 }
 

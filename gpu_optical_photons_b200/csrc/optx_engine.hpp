@@ -62,6 +62,9 @@ struct WaveArgs {
   uint32_t slot_cache;                  // batched tallies: 1 = warps may cache events in shared-memory
                                         // slots (every record's max_steps < kSlotMaxAdd)
   uint32_t flags;                       // DevParams::flags that every record has
+  uint32_t zero_steps;                  // 1: some record has max_steps 0
+  uint32_t shared_key;                  // 1: every record has the same Philox key, whose round keys are:
+  PhiloxKeys keys;
   uint32_t keep_tally;                  // 1: the run adds to the tallies (no zeroing by the prep kernel)
   const uint32_t* tally_of;             // record -> event (null: the record's own index)
   const float4* seg;                    // genstep records: 2 float4 each (end x,y,z,t0), (dt,-,-,-)
@@ -95,9 +98,26 @@ enum WaveMode : int { kModeTally = 0, kModeRecords = 1, kModeAdjoint = 2, kModeM
 // step physics (kernel argument), with per-record emission and per-event tallies.
 enum WaveVariant : int { kSingle = 0, kBatch = 1, kBatchUniform = 2 };
 constexpr uint32_t kEvShift = 7;  // coarsest event-table resolution: one entry per 128 photons
-// Shared memory of one warp's pantry: 32 ready photons x 112 bytes (7 x 16 B;
-// the 112-byte stride makes 8 lanes' 128-bit accesses hit 8 distinct bank groups).
-constexpr uint32_t kPantryBytesPerWarp = 32u * 112u;
+// Variants whose photons hold their unread words in the shared-memory ring (Window)
+// rather than in registers (Rng): the batched ones and the adjoint replays, which
+// are short of registers.
+inline __host__ __device__ constexpr bool wave_ring(int mode, bool batch) {
+  return batch || mode == kModeAdjoint || mode == kModeMoments;
+}
+// Shared memory of one warp, before the block's histograms: its lanes' rings
+// (kWindowWords uniforms each) if it has them; its pantry of 32 ready photons (state
+// and unread words: 6 float4 with a ring, else 5; one more for the path length and
+// score terms when the mode keeps them); batched, the warp's bookkeeping and, for
+// tallies, two event slots.
+constexpr uint32_t kWindowBytesPerWarp = 32u * kWindowWords * 4u;
+constexpr uint32_t kBookWords = 8u;
+inline __host__ __device__ constexpr uint32_t pantry_vec4(int mode, bool batch) {
+  return (wave_ring(mode, batch) ? 6u : 5u) + (mode == kModeTally ? 0u : 1u);
+}
+// The limit on histograms that a block of `warps` warps accepts dates from pantries of
+// 112 bytes per photon and no windows; blocks that no longer fit beside them are
+// launched with fewer warps.
+constexpr uint32_t kLimitBytesPerWarp = 32u * 112u;
 // Dynamic shared memory above this needs the kernel's opt-in attribute: the
 // default limit is 48 KB minus the kernel's static shared memory (at most 1 KB
 // for the kernels here).
@@ -124,6 +144,21 @@ static_assert((static_cast<unsigned long long>(kSlotFlushPhotons) + 64u) * kSlot
               "slot counters must not wrap between flushes");
 inline __host__ __device__ uint32_t slot_bin_bytes_per_warp(uint32_t n_bins) {
   return n_bins <= kSlotBins ? 2u * n_bins * 4u : 0u;
+}
+inline __host__ __device__ uint32_t wave_warp_bytes(int mode, bool batch, uint32_t n_bins) {
+  uint32_t b = 32u * 16u * pantry_vec4(mode, batch);
+  if (wave_ring(mode, batch)) b += kWindowBytesPerWarp;
+  if (batch) b += kBookWords * 4u;
+  if (batch && mode == kModeTally) b += kSlotCounterBytesPerWarp + slot_bin_bytes_per_warp(n_bins);
+  return (b + 15u) & ~15u;
+}
+inline PhiloxKeys philox_keys(uint32_t lo, uint32_t hi) {
+  PhiloxKeys K;
+  for (uint32_t r = 0; r < 10u; ++r) {
+    K.k0[r] = lo + r * 0x9E3779B9u;
+    K.k1[r] = hi + r * 0xBB67AE85u;
+  }
+  return K;
 }
 // Score moments: a block-private (time_bins + 1) x 5 FP64 table in shared memory,
 // added to global memory once per block, when it takes at most this many bytes
@@ -157,6 +192,7 @@ struct SortArgs {
   unsigned long long* tally;            // null: no tally (else ADDED to, flat layout)
   TallyDev tc;
   DevRecords rec;                       // rec.fate null: no records
+  PhiloxKeys keys;                      // round keys of the configuration's key
   unsigned long long graph_handle;      // cudaGraphConditionalHandle of the iteration loop
   uint32_t iter_cap;                    // watchdog: max iterations per run
   uint32_t use_graph;                   // 1: iterations run as a graph while node (set its condition)
