@@ -87,8 +87,9 @@ __device__ __forceinline__ void history_loop(const DevParams& P, const PhiloxKey
       const uint64_t id = first_id + i;
       start_photon(P, K, s, r, id, aux);
       uint32_t fate = kMaxSteps;
+      uint32_t used = 0u;
       if (P.max_steps != 0u) {
-        while (step_photon<false>(P, P.flags, K, s, r, id, fate, aux)) {}
+        while (step_photon<false>(P, P.flags, s, r, fate, aux, used)) r.advance(used, id, K);
       }
       done(i, s, fate);
     }
@@ -108,7 +109,9 @@ __device__ __forceinline__ void history_loop(const DevParams& P, const PhiloxKey
       alive = true;
       ended = P.max_steps == 0u;
     } else {
-      ended = !step_photon<false>(P, P.flags, K, s, r, first_id + cur, fate, aux);
+      uint32_t used = 0u;
+      ended = !step_photon<false>(P, P.flags, s, r, fate, aux, used);
+      if (!ended) r.advance(used, first_id + cur, K);
     }
     if (ended) {
       alive = false;
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   //  kSlotBins][block histograms (tally), bin weights (adjoint)]
   constexpr bool kSlots = BATCH && MODE == kModeTally;
   constexpr bool kAdj = MODE == kModeAdjoint || MODE == kModeMoments;  // replay modes
+  constexpr bool kLaneCounts = MODE == kModeTally && !BATCH;
   constexpr bool kPath = MODE != kModeTally;  // tallies do not use the path length
   constexpr bool kRing = wave_ring(MODE, BATCH);
   constexpr uint32_t kEntry = pantry_vec4(MODE, BATCH);
@@ -397,8 +401,14 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   uint32_t& tag1 = book[3];
   uint32_t& victim = book[4];
   uint32_t& since = book[5];
-  // Single configuration: per-lane tallies, flushed at the end of the wave.
-  uint32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0, f4 = 0, snb = 0, sns = 0;
+  // Single-configuration tallies: this lane's 5 fate counts and step sums, in shared
+  // memory (in registers they cost the loop 60 bytes of spills: bar 1e8 photons 27.4
+  // against 26.2 ms), added up at the end of the wave.
+  uint32_t* s_lane = s_book + lane;  // [7][32 lanes]
+  if (kLaneCounts) {
+#pragma unroll
+    for (uint32_t k = 0; k < kLaneCounters; ++k) s_lane[32u * k] = 0u;
+  }
   double g0 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;
   uint32_t useful = 0u, iters = 0u;
 
@@ -465,11 +475,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         }
       }
     } else if (MODE == kModeTally) {
-      f0 += fate == 0u;
-      f1 += fate == 1u;
-      f2 += fate == 2u;
-      f3 += fate == 3u;
-      f4 += fate == 4u;
+      s_lane[32u * fate] += 1u;
+      uint32_t snb = s_lane[32u * 5u], sns = s_lane[32u * 6u];
       // Per-lane step sums stay far below 2^31 between flushes (a lane sees at
       // most wave_quota / lanes photons of max_steps steps); flush early if not.
       if (snb > 0x7fffffffu || sns > 0x7fffffffu) {
@@ -477,8 +484,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         atomicAdd(&A.tally[tc.len - 1u], static_cast<unsigned long long>(sns));
         snb = sns = 0u;
       }
-      snb += s.nb;
-      sns += s.ns;
+      s_lane[32u * 5u] = snb + s.nb;
+      s_lane[32u * 6u] = sns + s.ns;
       if (fate == kDetected) {
         atomicAdd(&s_hist[time_bin(s.t, tc.tscale, tc.time_bins)], 1u);
         atomicAdd(&s_hist[tc.time_bins + 1u + xy_bin(s.px, s.py, P, tc.xy_bins)], 1u);
@@ -539,8 +546,11 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     return done;
   };
 
+  const bool drain = tail_steps == kNoSpill && cadence == 0u;
+  bool over_cap = false;
   for (;;) {
     if (iters > A.iter_cap) {
+      over_cap = true;
       if (lane == 0u) atomicOr(&ctrl->error, kErrWatchdog);
       break;
     }
@@ -722,12 +732,12 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         na = static_cast<uint32_t>(__popc(amask));
       }
       if (exhausted && pc == 0u) {
-        if (na == 0u) break;
+        if (na == 0u || drain) break;
         // A photon moves on to the next wave (compaction into fuller warps) only
         // after `tail_steps` (>= 1) steps in this one: every item of a wave makes
         // progress, so the run ends, and long histories advance many steps per
         // wave instead of one step per wave once the waves are small.
-        if (na < T && !queue_full && tail_steps != kNoSpill) {
+        if (na < T && !queue_full) {
           if (spill_lanes(alive && wsteps >= tail_steps)) alive = false;
           if (__ballot_sync(kFull, alive) == 0u) break;
         }
@@ -740,7 +750,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     bool ended = false;
     if (alive) {
       const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
-      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, run_key(), s, r, first_id + pidx, fate, aux);
+      uint32_t used = 0u;
+      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, s, r, fate, aux, used);
+      if constexpr (kRing) r.consume(used);
+      else if (!ended) r.advance(used, first_id + pidx, run_key());
       ++wsteps;
     }
     __syncwarp();
@@ -772,6 +785,53 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     }
   }
 
+  // ---- drain: the warp's last photons ------------------------------------------
+  // Nothing is left to claim: each lane runs its photon to its end in a loop of its
+  // own, without the warp's bookkeeping, and makes the next Philox block beside the
+  // step's first half rather than after it. A run is as long as its longest history,
+  // and a lone photon's step is one dependent chain: what counts is its length
+  // (kernel times with the main loop to the end: 1000 photons of the polished cube 187
+  // -> 131 us, 3e4 of the bar 307 -> 210, 1e6 of a gradient forward 225 -> 205; with
+  // the block made after the step 135 | 225 | 203).
+  if (!over_cap) {
+    const bool had = alive;
+    const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
+    const uint64_t id = first_id + pidx;
+    const uint32_t flags = ws.flags, cap = A.iter_cap - iters;
+    const bool shared_key = kSharedKey || A.shared_key != 0u;
+    uint32_t fate = kMaxSteps, steps = 0u;
+    while (alive) {
+      if (steps > cap) {
+        atomicOr(&ctrl->error, kErrWatchdog);
+        break;
+      }
+      ++steps;
+      auto block = [&](uint32_t b) {
+        const uint4 c = philox_counter(b, id);
+        if (shared_key) return philox10(c, run_key());
+        return philox10(c, make_uint2(P.key_lo, P.key_hi));
+      };
+      uint32_t used = 0u;
+      if constexpr (kRing) {
+        const uint4 next = block(r.made);
+        alive = step_photon<kAdj, BATCH && !UNI, kPath>(P, flags, s, r, fate, aux, used);
+        if (!alive) break;
+        r.consume(used);
+        if (r.av <= kWindowRoom) r.put(next);
+        if (r.av < kStepWords) r.put(block(r.made));
+      } else {
+        const uint4 next = block(r.blk + 2u);
+        alive = step_photon<kAdj, BATCH && !UNI, kPath>(P, flags, s, r, fate, aux, used);
+        if (!alive) break;
+        r.advance(used, id, run_key(), next);
+      }
+    }
+    __syncwarp();
+    if (had && !alive) finish(fate, P);
+    useful += __reduce_add_sync(kFull, steps);
+    iters += __reduce_max_sync(kFull, steps);
+  }
+
   // ---- end of this block's share of the wave: flush --------------------------
   if (lane == 0u) {
     atomicAdd(&ctrl->useful, static_cast<unsigned long long>(useful));
@@ -782,19 +842,11 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
       flush_slot(0u, tag0);
       flush_slot(1u, tag1);
     } else {
-      const uint32_t r0 = __reduce_add_sync(kFull, f0), r1 = __reduce_add_sync(kFull, f1),
-                     r2 = __reduce_add_sync(kFull, f2), r3 = __reduce_add_sync(kFull, f3),
-                     r4 = __reduce_add_sync(kFull, f4);
-      const unsigned long long wnb = warp_sum_u64(snb), wns = warp_sum_u64(sns);
       unsigned long long* gt = A.tally;
-      if (lane == 0u) {
-        if (r0) atomicAdd(&gt[0], static_cast<unsigned long long>(r0));
-        if (r1) atomicAdd(&gt[1], static_cast<unsigned long long>(r1));
-        if (r2) atomicAdd(&gt[2], static_cast<unsigned long long>(r2));
-        if (r3) atomicAdd(&gt[3], static_cast<unsigned long long>(r3));
-        if (r4) atomicAdd(&gt[4], static_cast<unsigned long long>(r4));
-        if (wnb) atomicAdd(&gt[tc.len - 2u], wnb);
-        if (wns) atomicAdd(&gt[tc.len - 1u], wns);
+#pragma unroll 1
+      for (uint32_t k = 0; k < kLaneCounters; ++k) {
+        const unsigned long long sum = warp_sum_u64(s_lane[32u * k]);
+        if (lane == 0u && sum != 0ull) atomicAdd(&gt[k < 5u ? k : tc.len - 7u + k], sum);
       }
       __syncthreads();
       for (uint32_t b = threadIdx.x; b < tc.len - 7u; b += blockDim.x) {
@@ -969,8 +1021,12 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
     }
     const uint64_t id = A.first_id + rel;
     if (seg < 3u) {
-      const uint32_t m = __ballot_sync(kFull, valid);
-      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, A.keys, s, r, id, fate, aux, hit, m);
+      // The warp reconverges before the advance: the Philox block runs once per warp
+      // step for all lanes that need one.
+      uint32_t used = 0u;
+      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, s, r, fate, aux, hit, used);
+      __syncwarp();
+      if (live) r.advance(used, id, A.keys);
     }
 
     int next = -1;
@@ -980,7 +1036,11 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         fate = kMaxSteps;
         live = false;
       }
-      while (live) live = step_photon<false>(P, P.flags, A.keys, s, r, id, fate, aux);
+      while (live) {
+        uint32_t used = 0u;
+        live = step_photon<false>(P, P.flags, s, r, fate, aux, used);
+        if (live) r.advance(used, id, A.keys);
+      }
     } else if (live) {
       // Photons that have made max_steps steps end here (each live step counted
       // one boundary or one scatter).

@@ -143,7 +143,6 @@ __device__ __forceinline__ float to_uniform(uint32_t bits) {
 // parameters, the id is first id + photon index), which keeps the per-lane state
 // at 10 registers.
 struct Rng {
-  static constexpr bool kRefilledByCaller = false;
   uint32_t w[8];
   uint32_t o, blk;
 
@@ -180,13 +179,21 @@ struct Rng {
   __device__ __forceinline__ void advance(uint32_t k, uint64_t id, const K& key) {
     o += k;
 #pragma unroll 1
-    while (o >= 4u) {
-      w[0] = w[4]; w[1] = w[5]; w[2] = w[6]; w[3] = w[7];
-      ++blk;
-      const uint4 b = philox10(philox_counter(blk + 1u, id), key);
-      w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-      o -= 4u;
-    }
+    while (o >= 4u) slide(philox10(philox_counter(blk + 2u, id), key));
+  }
+  // The same when block blk + 2 has been made already.
+  template <class K>
+  __device__ __forceinline__ void advance(uint32_t k, uint64_t id, const K& key, const uint4& next) {
+    o += k;
+    if (o >= 4u) slide(next);
+    if (o >= 4u) slide(philox10(philox_counter(blk + 2u, id), key));
+  }
+  // Moves the window on by one block; b: block blk + 2.
+  __device__ __forceinline__ void slide(const uint4& b) {
+    w[0] = w[4]; w[1] = w[5]; w[2] = w[6]; w[3] = w[7];
+    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    ++blk;
+    o -= 4u;
   }
 };
 
@@ -205,7 +212,6 @@ struct Rng {
 // aligned 128-bit store.
 constexpr uint32_t kWindowWords = 12u;
 struct Window {
-  static constexpr bool kRefilledByCaller = true;
   float* ring;    // this photon's kWindowWords places
   uint32_t rp;    // place of the next unread word
   uint32_t av;    // unread words
@@ -622,22 +628,16 @@ __device__ __forceinline__ uint32_t face_model(uint32_t surf_bits, int face) {
 }
 
 // Second half of a step (transport.hpp:98-145): the interaction `hit` at the
-// photon's position, then the window advance past the words the step used.
-// Returns true while the photon is alive; otherwise `fate` is set and the photon
-// sits at its final interaction. The window is advanced only for photons that
-// stay alive.
+// photon's position. Returns true while the photon is alive, with the words of the
+// window that the step used in `used` (the caller advances the window); otherwise
+// `fate` is set and the photon sits at its final interaction.
 // The outcome of every interaction comes first, as a few predicates (kept,
-// scattered, mirrored, diffuse), then one pass each of the rotation, the mirror
-// flip and the advance for all lanes that need it: fewer branches than a body per
-// outcome (per warp step of the batch 47 of them, not 66; Lambertian cube 1e7
-// photons 1.63 -> 1.55 ms). With sync_mask != 0 (the lanes of the warp that call
-// this step together) the warp reconverges before the advance, so the Philox block
-// runs once per warp step for all lanes that need one rather than once per
-// divergent group.
-template <bool AUX, bool GP = false, class R, class K>
-__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags,
-                                         const K& key, Photon& s, R& r, uint64_t id, uint32_t& fate, ScoreAux& aux, int hit,
-                                         uint32_t sync_mask = 0u) {
+// scattered, mirrored, diffuse), then one pass each of the rotation and the mirror
+// flip for all lanes that need it: fewer branches than a body per outcome (per warp
+// step of the batch 47 of them, not 66; Lambertian cube 1e7 photons 1.63 -> 1.55 ms).
+template <bool AUX, bool GP = false, class R>
+__device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags, Photon& s, const R& r,
+                                         uint32_t& fate, ScoreAux& aux, int hit, uint32_t& used) {
   const int face = hit;
   const int axis = face >> 1;
   // The window's words 2..4 as uniforms, once for every outcome (measured -2 % on
@@ -688,26 +688,20 @@ __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits,
   if (mirrored && axis == 0) s.dx = -s.dx;
   if (mirrored && axis == 1) s.dy = -s.dy;
   if (mirrored && axis == 2) s.dz = -s.dz;
-  if (sync_mask != 0u) __syncwarp(sync_mask);
-  if (live) {
-    fate = kMaxSteps;
-    const uint32_t k = scattered ? 4u : (diffuse ? 5u : 3u);
-    if constexpr (R::kRefilledByCaller) r.consume(k);
-    else r.advance(k, id, key);
-  }
+  if (live) fate = kMaxSteps;
+  used = scattered ? 4u : (diffuse ? 5u : 3u);
   return live;
 }
 
 // One step (transport.hpp:71-145): move, then interact. `flags`: those that hold for
 // every record of the run. False when the photon has ended, with its fate, or has
-// made max_steps steps (the fate is then kMaxSteps).
-template <bool AUX, bool GP = false, bool PATH = true, class R, class K>
-__device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, const K& key, Photon& s,
-                                            R& r, uint64_t id, uint32_t& fate, ScoreAux& aux,
-                                            uint32_t sync_mask = 0u) {
+// made max_steps steps (the fate is then kMaxSteps); true with the words used.
+template <bool AUX, bool GP = false, bool PATH = true, class R>
+__device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, Photon& s, const R& r, uint32_t& fate,
+                                            ScoreAux& aux, uint32_t& used) {
   const StepParams q = load_step<GP>(P);
   const int hit = step_move<PATH>(q, flags, s, r);
-  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, key, s, r, id, fate, aux, hit, sync_mask);
+  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, s, r, fate, aux, hit, used);
   return live && s.nb + s.ns < q.max_steps;
 }
 

@@ -108,9 +108,10 @@ inline __host__ __device__ constexpr bool wave_ring(int mode, bool batch) {
 // (kWindowWords uniforms each) if it has them; its pantry of 32 ready photons (state
 // and unread words: 6 float4 with a ring, else 5; one more for the path length and
 // score terms when the mode keeps them); batched, the warp's bookkeeping and, for
-// tallies, two event slots.
+// tallies, two event slots; single-configuration tallies, its lanes' counters.
 constexpr uint32_t kWindowBytesPerWarp = 32u * kWindowWords * 4u;
 constexpr uint32_t kBookWords = 8u;
+constexpr uint32_t kLaneCounters = 7u;  // single-configuration tallies: counters per lane
 inline __host__ __device__ constexpr uint32_t pantry_vec4(int mode, bool batch) {
   return (wave_ring(mode, batch) ? 6u : 5u) + (mode == kModeTally ? 0u : 1u);
 }
@@ -149,6 +150,7 @@ inline __host__ __device__ uint32_t wave_warp_bytes(int mode, bool batch, uint32
   uint32_t b = 32u * 16u * pantry_vec4(mode, batch);
   if (wave_ring(mode, batch)) b += kWindowBytesPerWarp;
   if (batch) b += kBookWords * 4u;
+  if (!batch && mode == kModeTally) b += 32u * 4u * kLaneCounters;
   if (batch && mode == kModeTally) b += kSlotCounterBytesPerWarp + slot_bin_bytes_per_warp(n_bins);
   return (b + 15u) & ~15u;
 }
