@@ -204,7 +204,7 @@ def records_device(p: SimParams, n: int, first_id: int = 0, out=None, block_size
 
 def tally_device(p: SimParams, c: TallyConfig, n: int, first_id: int = 0, out=None,
                  block_size: int = 256, math="fast", stream=None, check: bool = True):
-    """History tally kernel accumulating into a torch int64 device tensor of
+    """Tally of n photons accumulated into a torch int64 device tensor of
     c.length. `check=False` skips the output check for callers that checked the
     buffer once for many launches."""
     import torch

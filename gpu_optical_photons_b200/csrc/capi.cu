@@ -1275,6 +1275,49 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
   return OPTX_OK;
 }
 
+}  // extern "C"
+
+// The device calls' photons as fixed shares of the wave kernel's blocks, when that is
+// the faster kernel: with more photons than the history kernel has resident threads
+// (`threads`: its threads would run several photons each, one after another and
+// emitting on few lanes) and histograms that fit beside 28 warps' pantries. Measured,
+// history kernel against shares: device tally of the bar 1e6 951 | 547 us, 1.6e7 7.97
+// | 4.44 ms, records of the Lambertian cube 2.5e5 166 | 109 us, 4e6 1.09 | 0.60 ms,
+// tally with 130 KB of histograms 4e6 1.67 | 0.64 ms; with one photon per thread the
+// two are level and the history kernel needs no pantry (cube 6e4 181 | 188 us).
+static int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_id, uint64_t n,
+                      uint64_t threads, unsigned long long* tally, const DevRecords* rec, int math, cudaStream_t st,
+                      bool& done) {
+  done = false;
+  if (n <= threads || n > 0xffff0000ull) return OPTX_OK;  // 32-bit cursors, with room to run past the end
+  const size_t smem = wave_smem(td, mode, false, kSharesBlock);
+  int dev = 0, max_smem = 0;
+  OPTX_CUDA(cudaGetDevice(&dev));
+  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (smem + 1024u > static_cast<size_t>(max_smem)) return OPTX_OK;
+  WaveArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.n_events = 1;
+  a.n_tallies = 1;
+  a.flags = P.flags;
+  a.zero_steps = P.max_steps == 0u ? 1u : 0u;
+  a.shared_key = 1u;
+  a.keys = philox_keys(P.key_lo, P.key_hi);
+  a.threshold = 28;
+  a.total = n;
+  a.first_id = first_id;
+  a.tally = tally;
+  a.tc = td;
+  if (rec != nullptr) a.rec = *rec;
+  a.chunk = 32u;
+  a.tail_steps = kNoSpill;
+  a.iter_cap = 0xfffffff0u;
+  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, smem, num_sms(), done, st));
+  return OPTX_OK;
+}
+
+extern "C" {
+
 int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t n,
                         uint64_t first_id, const optx_records* dev_out, int block_size, int math,
                         void* stream) {
@@ -1297,8 +1340,16 @@ int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t 
     dd.y += done;
     dd.z += done;
     dd.path += done;
-    OPTX_CUDA(DISPATCH(math, launch_history_records, P, first_id + done, m, dd, block_size,
-                       static_cast<cudaStream_t>(stream)));
+    TallyDev none{};
+    none.len = 7u;
+    bool launched = false;
+    const uint64_t threads = static_cast<uint64_t>(DISPATCH(math, history_records_blocks_per_sm, block_size)) *
+                             block_size * num_sms();
+    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, threads, nullptr, &dd, math,
+                        static_cast<cudaStream_t>(stream), launched));
+    if (!launched)
+      OPTX_CUDA(DISPATCH(math, launch_history_records, P, first_id + done, m, dd, block_size,
+                         static_cast<cudaStream_t>(stream)));
     done += m;
   }
   return OPTX_OK;
@@ -1330,6 +1381,11 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
                                         num_sms())));
   if (n / grid >= 0xffffffffull)
     return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
+  bool launched = false;
+  OPTX_TRY(run_shares(kModeTally, P, td, first_id, n, static_cast<uint64_t>(std::max(bps, 1)) * block_size * num_sms(),
+                      reinterpret_cast<unsigned long long*>(dev_tally), nullptr, math,
+                      static_cast<cudaStream_t>(stream), launched));
+  if (launched) return OPTX_OK;
   OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n,
                      reinterpret_cast<unsigned long long*>(dev_tally), block_size, grid,
                      static_cast<cudaStream_t>(stream)));

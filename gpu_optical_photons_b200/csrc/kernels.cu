@@ -284,9 +284,15 @@ __device__ __forceinline__ const DevParams& params_of(const DevParams& P0,
 // allow: 2, 3 or 4 blocks of 256 threads (<= 128 / 80 / 64 registers), or 7
 // blocks of 128 threads (<= 72 registers, 28 warps per SM); a tuning knob.
 template <int MINB>
-constexpr int wave_max_threads() { return MINB >= 5 ? 128 : 256; }
+constexpr int wave_max_threads() { return MINB == 1 ? kSharesBlock : (MINB >= 5 ? 128 : 256); }
 
-template <int MODE, bool BATCH, int MINB, bool UNI>
+// SHARES: the stateless device calls (launch_shares). One configuration, one wave, no
+// control block (ctrl is null): each block, one per SM, runs its equal share of the
+// photons, a range of ids that its warps claim from a cursor in shared memory, so
+// launches need no memory of their own and may overlap on any streams. (The warps of
+// an SM do not advance alike: with a share per warp the bar at 1e8 photons took 31.6
+// ms, against 26.1.)
+template <int MODE, bool BATCH, int MINB, bool UNI, bool SHARES = false>
 __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     wave_kernel(const __grid_constant__ DevParams P0, const __grid_constant__ WaveArgs A,
                 WaveCtrl* __restrict__ ctrl) {
@@ -332,7 +338,16 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     uint32_t n_in, items, flags;
   };
   __shared__ WaveShared ws;
-  if (threadIdx.x == 0) {
+  __shared__ uint32_t s_cursor;  // SHARES: next photon of the block's share
+  if (SHARES) {
+    if (threadIdx.x == 0) {
+      ws.n_in = 0u;
+      ws.items = static_cast<uint32_t>(A.total * (blockIdx.x + 1u) / gridDim.x);
+      ws.fresh_next = 0ull;
+      ws.flags = A.flags;
+      s_cursor = static_cast<uint32_t>(A.total * blockIdx.x / gridDim.x);
+    }
+  } else if (threadIdx.x == 0) {
     const uint32_t wave = ctrl->wave;
     ws.n_in = ctrl->n_in;
     ws.items = ws.n_in + ctrl->fresh_count;
@@ -345,7 +360,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   const uint32_t& n_in = ws.n_in;
   const uint32_t& items = ws.items;
   const unsigned long long& fresh_next = ws.fresh_next;
-  const uint32_t T = A.threshold, cadence = A.cadence, qcap = A.qcap, wchunk = A.chunk, tail_steps = A.tail_steps;
+  const uint32_t T = A.threshold, cadence = SHARES ? 0u : A.cadence, qcap = A.qcap, wchunk = A.chunk, tail_steps = A.tail_steps;
   const unsigned long long first_id = A.first_id;
   // Event of a record (a genstep's event; a plain batch's records are its events).
   auto event_of = [&](uint32_t rec) -> uint32_t {
@@ -546,12 +561,12 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     return done;
   };
 
-  const bool drain = tail_steps == kNoSpill && cadence == 0u;
+  const bool drain = SHARES || (tail_steps == kNoSpill && cadence == 0u);
   bool over_cap = false;
   for (;;) {
     if (iters > A.iter_cap) {
       over_cap = true;
-      if (lane == 0u) atomicOr(&ctrl->error, kErrWatchdog);
+      if (!SHARES && lane == 0u) atomicOr(&ctrl->error, kErrWatchdog);
       break;
     }
     uint32_t amask = __ballot_sync(kFull, alive);
@@ -570,7 +585,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
         uint32_t base2 = 0u, got = got1;
         if (got1 < room) {
           unsigned long long b = 0ull;
-          if (lane == 0u) b = atomicAdd(&ctrl->cursor, static_cast<unsigned long long>(wchunk));
+          if (lane == 0u) {
+            // (A share's cursor runs past its end by one claim per warp at most.)
+            b = SHARES ? atomicAdd(&s_cursor, wchunk) : atomicAdd(&ctrl->cursor, static_cast<unsigned long long>(wchunk));
+          }
           b = __shfl_sync(kFull, b, 0);
           const unsigned long long hi = b + wchunk;
           chunk_lo = b < items ? static_cast<uint32_t>(b) : items;
@@ -780,8 +798,10 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     }
     ++iters;
     useful += na;
-    if (cadence != 0u && !queue_full) {  // forced compaction after `cadence` steps in this wave
-      if (spill_lanes(alive && wsteps >= cadence)) alive = false;
+    if constexpr (!SHARES) {
+      if (cadence != 0u && !queue_full) {  // forced compaction after `cadence` steps in this wave
+        if (spill_lanes(alive && wsteps >= cadence)) alive = false;
+      }
     }
   }
 
@@ -802,7 +822,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     uint32_t fate = kMaxSteps, steps = 0u;
     while (alive) {
       if (steps > cap) {
-        atomicOr(&ctrl->error, kErrWatchdog);
+        if (!SHARES) atomicOr(&ctrl->error, kErrWatchdog);
         break;
       }
       ++steps;
@@ -833,7 +853,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   }
 
   // ---- end of this block's share of the wave: flush --------------------------
-  if (lane == 0u) {
+  if (!SHARES && lane == 0u) {
     atomicAdd(&ctrl->useful, static_cast<unsigned long long>(useful));
     atomicAdd(&ctrl->issued, 32ull * iters);
   }
@@ -880,8 +900,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   }
 
   // ---- the last block to finish sets up the next wave --------------------------
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  if (!SHARES) __syncthreads();
+  if (!SHARES && threadIdx.x == 0) {
     __threadfence();
     const unsigned done = atomicAdd(&ctrl->blocks_done, 1u);
     if (done == gridDim.x - 1u) {
@@ -1179,16 +1199,21 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
 // ---------------------------------------------------------------------------
 // Host launchers.
 
+int history_records_blocks_per_sm(int block) {
+  int bps = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, history_records_kernel, block, 0) != cudaSuccess || bps < 1)
+    bps = 1;
+  return bps;
+}
+
 cudaError_t launch_history_records(const DevParams& P, uint64_t first_id, uint64_t n,
                                    const DevRecords& out, int block, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   // At most one wave of resident blocks: each thread runs several histories.
-  int dev = 0, sms = 1, bps = 1;
+  int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, history_records_kernel, block, 0) != cudaSuccess ||
-      bps < 1)
-    bps = 1;
+  const int bps = history_records_blocks_per_sm(block);
   const uint64_t grid = std::min<uint64_t>((n + block - 1) / block, static_cast<uint64_t>(bps) * sms);
   history_records_kernel<<<static_cast<unsigned>(grid), block, 0, st>>>(P, philox_keys(P.key_lo, P.key_hi), first_id, n,
                                                                         out);
@@ -1270,6 +1295,29 @@ cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const
                         WaveCtrl* ctrl, int grid, int block, size_t smem, cudaStream_t st) {
   void* args[] = {const_cast<DevParams*>(&P), const_cast<WaveArgs*>(&A), &ctrl};
   return cudaLaunchKernel(wave_kernel_fn(mode, batch, minb), dim3(grid), dim3(block), args, smem, st);
+}
+
+template <int MODE>
+static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, size_t smem, int sms, bool& done,
+                                      cudaStream_t st) {
+  const auto fn = wave_kernel<MODE, false, 1, false, true>;
+  done = false;
+  if (smem > kDynSmemOptIn) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  int bps = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kSharesBlock, smem);
+  if (e != cudaSuccess) return e;
+  if (bps < 1) return cudaSuccess;
+  done = true;
+  fn<<<sms, kSharesBlock, smem, st>>>(P, A, nullptr);
+  return cudaGetLastError();
+}
+cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, size_t smem, int sms, bool& done,
+                          cudaStream_t st) {
+  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, smem, sms, done, st)
+                            : launch_shares_mode<kModeRecords>(P, A, smem, sms, done, st);
 }
 
 const void* sorted_prep_fn() { return reinterpret_cast<const void*>(&sorted_prep_kernel); }

@@ -171,6 +171,9 @@ inline __host__ __device__ uint32_t moment_smem_bytes(uint32_t time_bins) {
   return b <= kMomentSmemMaxBytes ? b : 0u;
 }
 
+// Fixed-share launches: one block of 28 warps (72 registers) per SM.
+constexpr int kSharesBlock = 896;
+
 // Per-interaction sorted run (sorted_kernel): between steps each photon waits in
 // the state queue of its pending interaction; every iteration is one launch in
 // which each warp takes 32 photons of one queue (or 32 fresh emissions), so the
@@ -230,6 +233,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
                                    uint64_t n, unsigned long long* tally, int block, int grid,   \
                                    cudaStream_t st);                                             \
   int history_tally_blocks_per_sm(int block, size_t smem);                                       \
+  int history_records_blocks_per_sm(int block);                                                  \
   /* Wavefront: prep (reset ctrl, zero tallies) and one wave. */                                 \
   cudaError_t launch_wave_prep(const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,           \
                                cudaStream_t st);                                                 \
@@ -241,6 +245,10 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
   cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P,                     \
                           const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,                \
                           size_t smem, cudaStream_t st);                                         \
+  /* The wave kernel with fixed shares of A.total photons (tally or records mode); done =    \
+     false without a launch when its block does not fit. */                                      \
+  cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, size_t smem, int sms, \
+                            bool& done, cudaStream_t st);                                        \
   cudaError_t launch_event_table(const unsigned long long* offsets, uint32_t n_events,           \
                                  uint32_t* table, unsigned long long total, uint32_t shift,      \
                                  cudaStream_t st);                                               \

@@ -50,3 +50,38 @@ def test_small_ragged_batch_equals_oracle(engine, oracle, cfg):
     got = eng.tallies()
     eng.close()
     assert np.array_equal(got, oracle.batch_tally(arr, offs, TC, mode=oracle.PORTABLE))
+
+
+# Device calls around the sizes where they go from one photon per thread to fixed
+# shares of a warp (the resident threads of the history kernel), and tallies whose
+# histograms leave the shares no room (150 x 150 bins).
+@pytest.mark.parametrize("n,block,xy", [(1, 256, 10), (130_000, 256, 50), (152_000, 1024, 10), (152_000, 32, 100),
+                                        (400_003, 256, 50), (400_003, 256, 150)])
+def test_device_calls_equal_oracle(engine, oracle, n, block, xy):
+    import torch
+    p = P.config2()[0]
+    c = P.TallyConfig(100, 50.0, xy)
+    out = torch.ones(c.length, dtype=torch.int64, device="cuda")  # the call adds to it
+    engine.tally_device(p, c, n, first_id=2**33 + 5, out=out, block_size=block, math="exact")
+    want = oracle.tally(p, c, n, 2**33 + 5, mode=oracle.PORTABLE)
+    assert np.array_equal(out.cpu().numpy() - 1, want.astype(np.int64))
+    rec = engine.records_to_numpy(engine.records_device(p, n, first_id=2**33 + 5, block_size=block, math="exact"))
+    ref = oracle.records(p, n, 2**33 + 5, mode=oracle.PORTABLE)
+    for k in oracle.Records.FIELDS:
+        assert np.array_equal(np.asarray(rec[k]).view(np.uint8), np.asarray(ref[k]).view(np.uint8)), k
+
+
+def test_device_calls_overlap_on_streams(engine):
+    """Launches in flight together on several streams share nothing."""
+    import torch
+    p, c = P.config1()[0], TC
+    want = engine.run_gpu_tally(p, c, 600_000, first_id=1, math="fast")[1].astype(np.int64)
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    outs = [torch.zeros(c.length, dtype=torch.int64, device="cuda") for _ in streams]
+    torch.cuda.synchronize()
+    for i in range(3):
+        for st, o in zip(streams, outs):
+            engine.tally_device(p, c, 200_000, first_id=1 + 200_000 * i, out=o, stream=st)
+    torch.cuda.synchronize()
+    for o in outs:
+        assert np.array_equal(o.cpu().numpy(), want)
