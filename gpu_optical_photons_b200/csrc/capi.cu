@@ -217,7 +217,7 @@ int num_sms() {
 // ---- cached device buffers (per process; the library serialises calls) ---------
 // g_cache.rec belongs to optx_run_records_event, which holds g_event_mu for its
 // whole call (its engine writes the buffer between its own g_mu sections).
-// Lock order: g_event_mu, g_pipe_mu, an API engine's mu, g_mu.
+// Lock order: g_event_mu, g_pipe_mu, a tally workspace's mu, g_mu.
 std::mutex g_event_mu;
 struct Cache {
   void* rec = nullptr;
@@ -557,6 +557,12 @@ uint32_t claim_size(uint64_t photons, uint64_t warps) {
   return static_cast<uint32_t>(std::min<uint64_t>(256u, std::max<uint64_t>(32u, photons / (8u * warps) / 32u * 32u)));
 }
 
+// Watchdog: no warp can iterate more than (photons + queue) x (max_steps + 2) times.
+uint32_t run_iter_cap(uint64_t photons, uint64_t qcap, uint32_t max_steps) {
+  const unsigned long long cap = (photons + qcap + 64ull) * (max_steps + 2ull) + 4096ull;
+  return static_cast<uint32_t>(std::min(cap, 0xfffffff0ull));
+}
+
 // The arguments of a run.
 WaveArgs engine_args(const optx_engine* e, int mode, int warps, const DevRecords* rec, const double* w_bin, double w_det,
                      const double* theta_inv, uint32_t score_mask, double* moments) {
@@ -601,7 +607,6 @@ WaveArgs engine_args(const optx_engine* e, int mode, int warps, const DevRecords
   a.grad = (mode == kModeAdjoint || mode == kModeMoments) ? e->d_grad : nullptr;
   a.moments = (mode == kModeMoments) ? moments : nullptr;
   a.moments_smem = (a.moments != nullptr && moment_smem_bytes(e->tdev.time_bins) != 0u) ? 1u : 0u;
-  // Watchdog: no warp can iterate more than (photons + queue) x (max_steps + 2) times.
   uint32_t max_steps = 0;
   a.flags = ~0u;
   a.shared_key = 1u;
@@ -612,10 +617,7 @@ WaveArgs engine_args(const optx_engine* e, int mode, int warps, const DevRecords
     if (p.max_steps == 0u) a.zero_steps = 1u;
     if (p.key_lo != e->P0.key_lo || p.key_hi != e->P0.key_hi) a.shared_key = 0u;
   }
-  a.iter_cap = static_cast<uint32_t>(std::min<unsigned long long>(
-      (static_cast<unsigned long long>(e->total) + e->qcap + 64ull) *
-              (static_cast<unsigned long long>(max_steps) + 2ull) + 4096ull,
-      0xfffffff0ull));
+  a.iter_cap = run_iter_cap(e->total, e->qcap, max_steps);
   // Every photon of a wave steps at least once, so a run needs at most about
   // (admission waves) + max_steps waves; the cap only stops a broken run.
   const unsigned long long per_wave = std::max<unsigned long long>(
@@ -796,7 +798,8 @@ struct RecPipe {
   unsigned char* pin[2] = {nullptr, nullptr};
   cudaStream_t comp = nullptr, copy = nullptr;
   cudaEvent_t k0[2], k1[2], c1[2];
-  unsigned* err = nullptr;  // pinned: the engine run's error word per buffer set
+  unsigned* err = nullptr;  // pinned: the run's error word per buffer set
+  WaveCtrl* ctrl = nullptr;  // device: the control blocks they are read from
   bool events = false;
 };
 RecPipe g_pipe;
@@ -828,6 +831,7 @@ int pipe_ensure(uint64_t cap) {
                             cudaHostAllocDefault));
     g_pipe.events = true;
   }
+  if (g_pipe.ctrl == nullptr) OPTX_CUDA(cudaMalloc(&g_pipe.ctrl, 2 * sizeof(WaveCtrl)));
   if (g_pipe.cap >= cap) return OPTX_OK;
   for (int b = 0; b < 2; ++b) {
     if (g_pipe.dev[b]) cudaFree(g_pipe.dev[b]);
@@ -930,79 +934,100 @@ class PageToucher {
   std::vector<std::thread> th_;
 };
 
-// ---- engines behind the reference-API host calls ------------------------------
-// optx_run_tally and optx_run_records run the wavefront engine: the same
-// per-photon arithmetic as the history kernels (bit-identical records, equal
-// integer tallies) at 2-4x their speed on one configuration. One engine per
-// (device, math mode, tally configuration, photon capacity) is created on first
-// use; the most recent kApiMaxEngines are kept (until optx_release_cache). A call
-// holds a reference to its engine, so an engine dropped from the cache lives until
-// its last call ends; its mutex serialises a call's upload / run / read-back
-// sequence. Lock order: g_event_mu, g_pipe_mu, then an engine's mu, then g_mu (taken inside
-// the optx_engine_* calls).
-struct ApiEngine {
-  int device = -1;
-  int math = 0;
-  optx_tally_config tc{};
-  uint64_t cap = 0;
-  optx_engine* e = nullptr;
-  std::mutex mu;
-  ~ApiEngine() { optx_engine_destroy(e); }
-};
-// Guarded by g_mu, oldest first. Never destroyed: at process exit the CUDA
-// runtime may already be gone, so cached engines are not freed then.
-std::vector<std::shared_ptr<ApiEngine>>& g_api = *new std::vector<std::shared_ptr<ApiEngine>>();
-constexpr size_t kApiMaxEngines = 8;
-std::mutex g_pipe_mu;                           // the records pipeline (g_pipe)
-constexpr uint64_t kApiMaxCap = 1ull << 27;     // photons per engine run
+// ---- one configuration as fixed shares ---------------------------------------
+// The wave kernel with one block per SM, each running an equal share of the photons
+// (wave_kernel, SHARES): the same per-photon arithmetic as the history kernels
+// (bit-identical records, equal integer tallies), nothing to set up before it and no
+// state to keep after it.
 
-// Photon capacity of an engine serving runs of n photons: a power of two in
-// [2^20, 2^27], so that a few engines serve all sizes.
-uint64_t api_capacity(uint64_t n) {
-  uint64_t c = 1ull << 20;
-  while (c < n && c < kApiMaxCap) c <<= 1;
-  return c;
+// Whether a tally's histograms fit beside the warps' pantries.
+int shares_fit(const TallyDev& td, int mode, bool& fit) {
+  int dev = 0, max_smem = 0;
+  OPTX_CUDA(cudaGetDevice(&dev));
+  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  fit = wave_smem(td, mode, false, kSharesBlock) + kSharesStaticSmem <= static_cast<size_t>(max_smem);
+  return OPTX_OK;
 }
 
-// Finds or creates the engine. OPTX_ERR_RUNTIME means the wave kernel cannot be
-// resident beside these histograms (the caller then runs the history kernel).
-int api_engine(int math, const optx_tally_config& tc, uint64_t cap, std::shared_ptr<ApiEngine>& out) {
+// n <= kSharesMaxPhotons photons, added to `tally` or written to `rec`, async on st.
+int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_id, uint64_t n,
+               unsigned long long* tally, const DevRecords* rec, WaveCtrl* ctrl, int math, cudaStream_t st) {
+  WaveArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.n_events = 1;
+  a.n_tallies = 1;
+  a.flags = P.flags;
+  a.zero_steps = P.max_steps == 0u ? 1u : 0u;
+  a.shared_key = 1u;
+  a.keys = philox_keys(P.key_lo, P.key_hi);
+  a.threshold = 28;
+  a.total = n;
+  a.first_id = first_id;
+  a.tally = tally;
+  a.tc = td;
+  if (rec != nullptr) a.rec = *rec;
+  // A claim is a refill; fewer photons than that per warp are spread over the warps.
+  const int sms = num_sms();
+  const uint64_t warps = static_cast<uint64_t>(sms) * (kSharesBlock / 32);
+  a.chunk = static_cast<uint32_t>(std::min<uint64_t>(32u, (n + warps - 1u) / warps));
+  a.tail_steps = kNoSpill;
+  a.iter_cap = test_fault("watchdog") ? 1u : run_iter_cap(n, 0u, P.max_steps);
+  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, wave_smem(td, mode, false, kSharesBlock), sms, st));
+  return OPTX_OK;
+}
+
+std::mutex g_pipe_mu;  // the records pipeline (g_pipe)
+
+// Workspace of the host tally calls, one per device: [WaveCtrl][tally] on the device
+// and the pinned copy that comes back in one transfer. A call holds it for its length;
+// it lives until optx_release_cache and the last call that uses it.
+struct TallySpace {
+  int device = -1;
+  size_t bytes = 0;
+  unsigned char *dev = nullptr, *host = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  std::mutex mu;
+  ~TallySpace() {
+    cudaFree(dev);
+    cudaFreeHost(host);
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+  }
+};
+constexpr size_t kTallySpaceHead = 256;
+static_assert(sizeof(WaveCtrl) <= kTallySpaceHead, "the error word sits before the tally");
+// Guarded by g_mu. Never destroyed: at process exit the CUDA runtime may already be
+// gone, so kept workspaces are not freed then.
+std::vector<std::shared_ptr<TallySpace>>& g_spaces = *new std::vector<std::shared_ptr<TallySpace>>();
+
+int tally_space(std::shared_ptr<TallySpace>& out) {
   int dev = 0;
   OPTX_CUDA(cudaGetDevice(&dev));
-  auto match = [&](const ApiEngine& a) {
-    return a.device == dev && a.math == math && a.cap >= cap && a.tc.time_bins == tc.time_bins &&
-           a.tc.time_max == tc.time_max && a.tc.xy_bins == tc.xy_bins;
-  };
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    for (auto& a : g_api)
-      if (match(*a)) {
-        out = a;
-        return OPTX_OK;
-      }
-  }
-  optx_wave_config cfg{};
-  cfg.block_size = 128;   // the 72-register budget: 28 warps per SM, the fastest
-  cfg.blocks_per_sm = 7;  // single-configuration variant on the reference setups
-  cfg.threshold = 28;
-  cfg.use_graph = 1;
-  cfg.math = math;
-  optx_engine* e = nullptr;
-  OPTX_TRY(optx_engine_create(&tc, 1, cap, &cfg, &e));
-  auto a = std::make_shared<ApiEngine>();
-  a->device = dev;
-  a->math = math;
-  a->tc = tc;
-  a->cap = cap;
-  a->e = e;
-  out = a;
-  std::shared_ptr<ApiEngine> dropped;  // released after g_mu
   std::lock_guard<std::mutex> lk(g_mu);
-  if (g_api.size() >= kApiMaxEngines) {
-    dropped = g_api.front();
-    g_api.erase(g_api.begin());
-  }
-  g_api.push_back(std::move(a));
+  for (auto& t : g_spaces)
+    if (t->device == dev) {
+      out = t;
+      return OPTX_OK;
+    }
+  out = std::make_shared<TallySpace>();
+  out->device = dev;
+  g_spaces.push_back(out);
+  return OPTX_OK;
+}
+
+// With t.mu held: room for a tally of `len` entries.
+int tally_space_ensure(TallySpace& t, size_t len) {
+  if (t.e0 == nullptr) OPTX_CUDA(cudaEventCreate(&t.e0));
+  if (t.e1 == nullptr) OPTX_CUDA(cudaEventCreate(&t.e1));
+  const size_t bytes = kTallySpaceHead + 8u * len;
+  if (t.bytes >= bytes) return OPTX_OK;
+  cudaFree(t.dev);
+  cudaFreeHost(t.host);
+  t.dev = t.host = nullptr;
+  t.bytes = 0;
+  OPTX_CUDA(cudaMalloc(&t.dev, bytes));
+  OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&t.host), bytes, cudaHostAllocDefault));
+  t.bytes = bytes;
   return OPTX_OK;
 }
 
@@ -1041,7 +1066,7 @@ int optx_release_cache(void) {
   // No records call is in flight while g_event_mu (held to the end, so that
   // g_cache.rec is not in use when it is freed) and g_pipe_mu are held.
   std::lock_guard<std::mutex> elk(g_event_mu);
-  std::vector<std::shared_ptr<ApiEngine>> engines;  // destroyed after g_mu, once unused
+  std::vector<std::shared_ptr<TallySpace>> spaces;  // destroyed after g_mu, once unused
   {
     // Copies left queued by a records call that returned an error are drained first.
     std::lock_guard<std::mutex> plk(g_pipe_mu);
@@ -1056,6 +1081,8 @@ int optx_release_cache(void) {
       g_pipe.pin[b] = nullptr;
     }
     g_pipe.cap = 0;
+    cudaFree(g_pipe.ctrl);
+    g_pipe.ctrl = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
   }
   {
@@ -1065,12 +1092,12 @@ int optx_release_cache(void) {
     if (g_cache.e0) cudaEventDestroy(g_cache.e0);
     if (g_cache.e1) cudaEventDestroy(g_cache.e1);
     g_cache = Cache{};
-    engines.swap(g_api);
+    spaces.swap(g_spaces);
     // After a device reset the module is loaded again, possibly elsewhere: the
     // next allocation-free call looks the scratch address up afresh.
     noalloc_forget_addresses();
   }
-  engines.clear();  // an engine still used by a call is destroyed when that call ends
+  spaces.clear();  // one still used by a call is destroyed when that call ends
   return OPTX_OK;
 }
 
@@ -1096,14 +1123,8 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
       1, std::min<uint64_t>({n, chunk ? chunk : (uint64_t{1} << 24), uint64_t{1} << 22}));
   const auto ta = std::chrono::steady_clock::now();
   OPTX_TRY(pipe_ensure(cap));
-  // The wavefront engine writes each chunk's records (the history kernel when the
-  // engine cannot be created, which a records run never needs in practice).
-  std::shared_ptr<ApiEngine> ae;
-  const optx_tally_config no_tally{1u, 1.0f, 1u};
-  const int erc = api_engine(math, no_tally, api_capacity(cap), ae);
-  if (erc != OPTX_OK && erc != OPTX_ERR_RUNTIME) return erc;
-  std::unique_lock<std::mutex> elk;
-  if (erc == OPTX_OK) elk = std::unique_lock<std::mutex>(ae->mu);
+  TallyDev none{};
+  none.len = 7u;  // no histograms
   tm.alloc_ms = ms_since(ta);
   void* outs[8] = {out->fate, out->n_boundary, out->n_scatter, out->t, out->x, out->y, out->z, out->path};
   bool direct = true;
@@ -1140,16 +1161,10 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
                        reinterpret_cast<float*>(dv[3]), reinterpret_cast<float*>(dv[4]),
                        reinterpret_cast<float*>(dv[5]), reinterpret_cast<float*>(dv[6]),
                        reinterpret_cast<float*>(dv[7])};
-    if (ae != nullptr) {
-      const uint64_t cnt = m;
-      const optx_records dr{d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
-      OPTX_TRY(optx_engine_set_events(ae->e, p, faces, &cnt, 1, first_id + done, g_pipe.comp));
-      OPTX_TRY(optx_engine_run_records(ae->e, &dr, g_pipe.comp));
-      OPTX_CUDA(cudaMemcpyAsync(&g_pipe.err[b], &ae->e->d_ctrl->error, sizeof(unsigned),
-                                cudaMemcpyDeviceToHost, g_pipe.comp));
-    } else {
-      OPTX_CUDA(DISPATCH(math, launch_history_records, P, first_id + done, m, d, block_size, g_pipe.comp));
-    }
+    OPTX_CUDA(cudaMemsetAsync(&g_pipe.ctrl[b], 0, sizeof(WaveCtrl), g_pipe.comp));
+    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &d, &g_pipe.ctrl[b], math, g_pipe.comp));
+    OPTX_CUDA(cudaMemcpyAsync(&g_pipe.err[b], &g_pipe.ctrl[b].error, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                              g_pipe.comp));
     OPTX_CUDA(cudaEventRecord(g_pipe.k1[b], g_pipe.comp));
     OPTX_CUDA(cudaStreamWaitEvent(g_pipe.copy, g_pipe.k1[b], 0));
     auto hv = views(b, true);
@@ -1172,7 +1187,7 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
       kms += ms;
       OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[pb], g_pipe.c1[pb]));
       cms += ms;
-      if (ae != nullptr) OPTX_TRY(run_error(g_pipe.err[pb]));
+      OPTX_TRY(run_error(g_pipe.err[pb]));
       if (!direct) host_fill(i - 1);
     }
   }
@@ -1183,7 +1198,7 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
   kms += ms;
   OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[lb], g_pipe.c1[lb]));
   cms += ms;
-  if (ae != nullptr) OPTX_TRY(run_error(g_pipe.err[lb]));
+  OPTX_TRY(run_error(g_pipe.err[lb]));
   if (!direct) host_fill(chunks - 1);
   tm.kernel_ms = kms;
   tm.d2h_ms = cms;  // kernel end to copy end per chunk (copies overlap later kernels)
@@ -1209,36 +1224,41 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
   OPTX_TRY(ensure_device());
   optx_timing tm{};
   const auto t0 = std::chrono::steady_clock::now();
-  if (n > 0) {
-    // The wavefront engine, in runs of at most its capacity, tallies summed on the host.
-    std::shared_ptr<ApiEngine> ae;
-    const int erc = api_engine(math, *c, api_capacity(n), ae);
-    if (erc != OPTX_OK && erc != OPTX_ERR_RUNTIME) return erc;
-    if (erc == OPTX_OK) {
-      tm.alloc_ms = ms_since(t0);
-      std::lock_guard<std::mutex> elk(ae->mu);
-      std::vector<uint64_t> part(td.len);
-      std::memset(tally_out, 0, td.len * 8ull);
-      for (uint64_t done = 0; done < n;) {
-        const uint64_t m = std::min(ae->cap, n - done);
-        OPTX_TRY(optx_engine_set_events(ae->e, p, faces, &m, 1, first_id + done, nullptr));
-        OPTX_TRY(optx_engine_run_tally(ae->e, nullptr));
-        const auto tc = std::chrono::steady_clock::now();
-        OPTX_TRY(optx_engine_get_tallies(ae->e, part.data(), nullptr));
-        tm.d2h_ms += ms_since(tc);
-        for (uint32_t k = 0; k < td.len; ++k) tally_out[k] += part[k];
-        optx_event_stats s{};
-        OPTX_TRY(optx_engine_stats(ae->e, &s, nullptr));
-        tm.kernel_ms += s.kernels_ms;
-        done += m;
-      }
-      tm.total_ms = ms_since(t0);
-      if (timing) *timing = tm;
-      return OPTX_OK;
+  bool fit = false;
+  OPTX_TRY(shares_fit(td, kModeTally, fit));
+  if (fit) {
+    std::shared_ptr<TallySpace> space;
+    OPTX_TRY(tally_space(space));
+    std::lock_guard<std::mutex> slk(space->mu);
+    OPTX_TRY(tally_space_ensure(*space, td.len));
+    tm.alloc_ms = ms_since(t0);
+    const DevParams P = make_dev_params(*p, faces);
+    const size_t bytes = kTallySpaceHead + 8ull * td.len;
+    auto* ctrl = reinterpret_cast<WaveCtrl*>(space->dev);
+    auto* tally = reinterpret_cast<unsigned long long*>(space->dev + kTallySpaceHead);
+    OPTX_CUDA(cudaMemsetAsync(space->dev, 0, bytes, nullptr));
+    OPTX_CUDA(cudaEventRecord(space->e0, nullptr));
+    for (uint64_t done = 0; done < n;) {  // one launch, but for more photons than its cursors count
+      const uint64_t m = std::min(n - done, kSharesMaxPhotons);
+      OPTX_TRY(run_shares(kModeTally, P, td, first_id + done, m, tally, nullptr, ctrl, math, nullptr));
+      done += m;
     }
+    OPTX_CUDA(cudaEventRecord(space->e1, nullptr));
+    const auto tc = std::chrono::steady_clock::now();
+    OPTX_CUDA(cudaMemcpyAsync(space->host, space->dev, bytes, cudaMemcpyDeviceToHost, nullptr));
+    OPTX_CUDA(cudaStreamSynchronize(nullptr));
+    float kms = 0.f;
+    OPTX_CUDA(cudaEventElapsedTime(&kms, space->e0, space->e1));
+    OPTX_TRY(run_error(reinterpret_cast<const WaveCtrl*>(space->host)->error));
+    std::memcpy(tally_out, space->host + kTallySpaceHead, 8ull * td.len);
+    tm.kernel_ms = kms;
+    tm.d2h_ms = ms_since(tc);
+    tm.total_ms = ms_since(t0);
+    if (timing) *timing = tm;
+    return OPTX_OK;
   }
-  // The history kernel: n = 0, or the wave kernel's pantries do not fit beside
-  // these histograms in shared memory.
+  // The history kernel: the wave kernel's pantries do not fit beside these histograms
+  // in shared memory.
   std::lock_guard<std::mutex> lk(g_mu);
   OPTX_TRY(cache_events());
   const DevParams P = make_dev_params(*p, faces);
@@ -1277,43 +1297,19 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
 
 }  // extern "C"
 
-// The device calls' photons as fixed shares of the wave kernel's blocks, when that is
-// the faster kernel: with more photons than the history kernel has resident threads
-// (`threads`: its threads would run several photons each, one after another and
-// emitting on few lanes) and histograms that fit beside 28 warps' pantries. Measured,
-// history kernel against shares: device tally of the bar 1e6 951 | 547 us, 1.6e7 7.97
-// | 4.44 ms, records of the Lambertian cube 2.5e5 166 | 109 us, 4e6 1.09 | 0.60 ms,
-// tally with 130 KB of histograms 4e6 1.67 | 0.64 ms; with one photon per thread the
-// two are level and the history kernel needs no pantry (cube 6e4 181 | 188 us).
-static int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_id, uint64_t n,
-                      uint64_t threads, unsigned long long* tally, const DevRecords* rec, int math, cudaStream_t st,
-                      bool& done) {
-  done = false;
-  if (n <= threads || n > 0xffff0000ull) return OPTX_OK;  // 32-bit cursors, with room to run past the end
-  const size_t smem = wave_smem(td, mode, false, kSharesBlock);
-  int dev = 0, max_smem = 0;
-  OPTX_CUDA(cudaGetDevice(&dev));
-  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (smem + 1024u > static_cast<size_t>(max_smem)) return OPTX_OK;
-  WaveArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.n_events = 1;
-  a.n_tallies = 1;
-  a.flags = P.flags;
-  a.zero_steps = P.max_steps == 0u ? 1u : 0u;
-  a.shared_key = 1u;
-  a.keys = philox_keys(P.key_lo, P.key_hi);
-  a.threshold = 28;
-  a.total = n;
-  a.first_id = first_id;
-  a.tally = tally;
-  a.tc = td;
-  if (rec != nullptr) a.rec = *rec;
-  a.chunk = 32u;
-  a.tail_steps = kNoSpill;
-  a.iter_cap = 0xfffffff0u;
-  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, smem, num_sms(), done, st));
-  return OPTX_OK;
+// Whether a device call's photons run as fixed shares (run_shares), when that is the
+// faster kernel: with more photons than the history kernel has resident threads
+// (its threads would run several photons each, one after another and emitting on few
+// lanes) and histograms that fit beside 28 warps' pantries. Measured, history kernel
+// against shares: device tally of the bar 1e6 951 | 547 us, 1.6e7 7.97 | 4.44 ms,
+// records of the Lambertian cube 2.5e5 166 | 109 us, 4e6 1.09 | 0.60 ms, tally with
+// 130 KB of histograms 4e6 1.67 | 0.64 ms; with one photon per thread the two are
+// level and the history kernel needs no pantry (cube 6e4 181 | 188 us).
+static int use_shares(int mode, const TallyDev& td, uint64_t n, int blocks_per_sm, int block, bool& use) {
+  use = false;
+  if (n <= static_cast<uint64_t>(std::max(blocks_per_sm, 1)) * block * num_sms() || n > kSharesMaxPhotons)
+    return OPTX_OK;
+  return shares_fit(td, mode, use);
 }
 
 extern "C" {
@@ -1341,13 +1337,14 @@ int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t 
     dd.z += done;
     dd.path += done;
     TallyDev none{};
-    none.len = 7u;
-    bool launched = false;
-    const uint64_t threads = static_cast<uint64_t>(DISPATCH(math, history_records_blocks_per_sm, block_size)) *
-                             block_size * num_sms();
-    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, threads, nullptr, &dd, math,
-                        static_cast<cudaStream_t>(stream), launched));
-    if (!launched)
+    none.len = 7u;  // no histograms
+    bool shares = false;
+    OPTX_TRY(use_shares(kModeRecords, none, m, DISPATCH(math, history_records_blocks_per_sm, block_size), block_size,
+                        shares));
+    if (shares)
+      OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &dd, nullptr, math,
+                          static_cast<cudaStream_t>(stream)));
+    else
       OPTX_CUDA(DISPATCH(math, launch_history_records, P, first_id + done, m, dd, block_size,
                          static_cast<cudaStream_t>(stream)));
     done += m;
@@ -1381,11 +1378,11 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
                                         num_sms())));
   if (n / grid >= 0xffffffffull)
     return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
-  bool launched = false;
-  OPTX_TRY(run_shares(kModeTally, P, td, first_id, n, static_cast<uint64_t>(std::max(bps, 1)) * block_size * num_sms(),
-                      reinterpret_cast<unsigned long long*>(dev_tally), nullptr, math,
-                      static_cast<cudaStream_t>(stream), launched));
-  if (launched) return OPTX_OK;
+  bool shares = false;
+  OPTX_TRY(use_shares(kModeTally, td, n, bps, block_size, shares));
+  if (shares)
+    return run_shares(kModeTally, P, td, first_id, n, reinterpret_cast<unsigned long long*>(dev_tally), nullptr,
+                      nullptr, math, static_cast<cudaStream_t>(stream));
   OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n,
                      reinterpret_cast<unsigned long long*>(dev_tally), block_size, grid,
                      static_cast<cudaStream_t>(stream)));
@@ -2365,8 +2362,7 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
   a.use_graph = 0u;
   a.chunk = claim_size(n, static_cast<uint64_t>(grid) * (block / 32));
   a.tail_steps = 4096u;
-  a.iter_cap = static_cast<uint32_t>(std::min<unsigned long long>(
-      (static_cast<unsigned long long>(n) + a.qcap + 64ull) * (P.max_steps + 2ull) + 4096ull, 0xfffffff0ull));
+  a.iter_cap = run_iter_cap(n, a.qcap, P.max_steps);
   a.wave_cap = static_cast<uint32_t>(std::min<unsigned long long>(
       std::max<unsigned long long>(4ull * (P.max_steps + 2ull) + 64ull, 100000ull), 0xfffffff0ull));
   // The prep kernel clears what must start at zero: the control block and the

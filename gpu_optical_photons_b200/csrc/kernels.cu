@@ -286,8 +286,9 @@ __device__ __forceinline__ const DevParams& params_of(const DevParams& P0,
 template <int MINB>
 constexpr int wave_max_threads() { return MINB == 1 ? kSharesBlock : (MINB >= 5 ? 128 : 256); }
 
-// SHARES: the stateless device calls (launch_shares). One configuration, one wave, no
-// control block (ctrl is null): each block, one per SM, runs its equal share of the
+// SHARES: the device calls and the host tally and records calls (launch_shares). One
+// configuration, one wave, no state between launches (ctrl, where it is not null,
+// takes a watchdog's error word only): each block, one per SM, runs its equal share of the
 // photons, a range of ids that its warps claim from a cursor in shared memory, so
 // launches need no memory of their own and may overlap on any streams. (The warps of
 // an SM do not advance alike: with a share per warp the bar at 1e8 photons took 31.6
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   for (;;) {
     if (iters > A.iter_cap) {
       over_cap = true;
-      if (!SHARES && lane == 0u) atomicOr(&ctrl->error, kErrWatchdog);
+      if (lane == 0u && (!SHARES || ctrl != nullptr)) atomicOr(&ctrl->error, kErrWatchdog);
       break;
     }
     uint32_t amask = __ballot_sync(kFull, alive);
@@ -822,7 +823,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     uint32_t fate = kMaxSteps, steps = 0u;
     while (alive) {
       if (steps > cap) {
-        if (!SHARES) atomicOr(&ctrl->error, kErrWatchdog);
+        if (!SHARES || ctrl != nullptr) atomicOr(&ctrl->error, kErrWatchdog);
         break;
       }
       ++steps;
@@ -1298,26 +1299,20 @@ cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const
 }
 
 template <int MODE>
-static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, size_t smem, int sms, bool& done,
+static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, size_t smem, int sms,
                                       cudaStream_t st) {
   const auto fn = wave_kernel<MODE, false, 1, false, true>;
-  done = false;
   if (smem > kDynSmemOptIn) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  int bps = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kSharesBlock, smem);
-  if (e != cudaSuccess) return e;
-  if (bps < 1) return cudaSuccess;
-  done = true;
-  fn<<<sms, kSharesBlock, smem, st>>>(P, A, nullptr);
+  fn<<<sms, kSharesBlock, smem, st>>>(P, A, ctrl);
   return cudaGetLastError();
 }
-cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, size_t smem, int sms, bool& done,
+cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, size_t smem, int sms,
                           cudaStream_t st) {
-  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, smem, sms, done, st)
-                            : launch_shares_mode<kModeRecords>(P, A, smem, sms, done, st);
+  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, ctrl, smem, sms, st)
+                            : launch_shares_mode<kModeRecords>(P, A, ctrl, smem, sms, st);
 }
 
 const void* sorted_prep_fn() { return reinterpret_cast<const void*>(&sorted_prep_kernel); }

@@ -173,6 +173,8 @@ inline __host__ __device__ uint32_t moment_smem_bytes(uint32_t time_bins) {
 
 // Fixed-share launches: one block of 28 warps (72 registers) per SM.
 constexpr int kSharesBlock = 896;
+constexpr uint64_t kSharesMaxPhotons = 0xffff0000ull;  // 32-bit cursors, with room to run past the end
+constexpr size_t kSharesStaticSmem = 1024;             // at least the kernel's static shared memory
 
 // Per-interaction sorted run (sorted_kernel): between steps each photon waits in
 // the state queue of its pending interaction; every iteration is one launch in
@@ -245,10 +247,9 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
   cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P,                     \
                           const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,                \
                           size_t smem, cudaStream_t st);                                         \
-  /* The wave kernel with fixed shares of A.total photons (tally or records mode); done =    \
-     false without a launch when its block does not fit. */                                      \
-  cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, size_t smem, int sms, \
-                            bool& done, cudaStream_t st);                                        \
+  /* The wave kernel with fixed shares of A.total photons (tally or records mode). */            \
+  cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl,      \
+                            size_t smem, int sms, cudaStream_t st);                              \
   cudaError_t launch_event_table(const unsigned long long* offsets, uint32_t n_events,           \
                                  uint32_t* table, unsigned long long total, uint32_t shift,      \
                                  cudaStream_t st);                                               \
