@@ -1045,7 +1045,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
       // The warp reconverges before the advance: the Philox block runs once per warp
       // step for all lanes that need one.
       uint32_t used = 0u;
-      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, s, r, fate, aux, hit, used);
+      if (valid) live = step_act<false>(P, P.surf_bits, P.flags, s, r, fate, aux, Hit::of(hit, s), used);
       __syncwarp();
       if (live) r.advance(used, id, A.keys);
     }
@@ -1069,14 +1069,15 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
         fate = kMaxSteps;
         live = false;
       } else {
-        hit = step_move(load_step<false>(P), P.flags, s, r);
-        if (hit == kHitAbsorb) {  // bulk absorption (transport.hpp:98-101)
+        const Hit h = step_move(load_step<false>(P), P.flags, s, r);
+        hit = h.code();
+        if (h.absorb) {  // bulk absorption (transport.hpp:98-101)
           fate = kAbsorbedBulk;
           live = false;
-        } else if (hit == kHitScatter) {
+        } else if (h.scatter) {
           next = kQScatter;
         } else {
-          const uint32_t model = face_model(P.surf_bits, hit);
+          const uint32_t model = face_model(P.surf_bits, h);
           if (model == kBlack) {  // black face: absorbed, no draw (transport.hpp:129-132)
             ++s.nb;
             fate = kAbsorbedSurface;

@@ -106,11 +106,17 @@ struct Box {
     if ((m & 192u) == 0u) s.dx = (m & 256u) ? 0.0f : -0.0f;
     if ((m & 1536u) == 0u) { s.dy = s.dx; s.py = s.px; }  // ties
     if (s.dx == 0.0f && s.dy == 0.0f && s.dz == 0.0f) s.dy = 1.0f;
-    float d0, d1;
-    int f0, f1;
-    box_exit(P, kOrdinary, s, d0, f0);
-    box_exit_ieee(P, s, d1, f1);
-    return same(fmaxf(d0, 0.0f), fmaxf(d1, 0.0f)) && f0 == f1;
+    Hit h0{}, h1{};
+    const float d0 = box_exit(P, kOrdinary, s, h0), d1 = box_exit_ieee(P, s, h1);
+    return same(fmaxf(d0, 0.0f), fmaxf(d1, 0.0f)) && h0.code() == h1.code() && same(h0.along, h1.along) &&
+           h0.x == h1.x && h0.y == h1.y && h0.z == h1.z && Hit::of(h0.code(), s).along == h0.along;
+  }
+};
+
+struct Log {  // i: a word's upper 24 bits
+  __device__ bool operator()(uint64_t i) const {
+    const float u = to_uniform(static_cast<uint32_t>(i) << 8), l = -m_log(u), g = lg2_approx(u);
+    return log_lo(g) <= l && l <= log_hi(g);
   }
 };
 
@@ -153,6 +159,7 @@ int main(int argc, char** argv) {
     rc |= run("m_sqrt", Sqrt{}, bits(0x1p-60f), bits(0x1p60f) + 1, bad);
     rc |= run("m_sqrt(0)", Sqrt{}, 0, 1, bad);
     rc |= run("m_rcp", Rcp{}, bits(0x1p-100f), bits(0x1p100f) + 1, bad);
+    rc |= run("log bounds", Log{}, 0, 1ull << 24, bad);
     rc |= run("to_uniform", Uniform{}, 0, 1ull << 32, bad);
     rc |= run("m_div", Div{}, 0, 1ull << 32, bad);
     rc |= run("fresnel_reflects", Fresnel{}, 0, 1ull << 30, bad);

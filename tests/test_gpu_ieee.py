@@ -23,7 +23,7 @@ def test_step_arithmetic_equals_ieee(engine, tmp_path, flags):
                    + [os.path.join(HERE, "cuda", "ieee_check.cu"), "-o", exe], check=True)
     out = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stdout + out.stderr
-    assert out.stdout.count(" 0 mismatches") == 7, out.stdout
+    assert out.stdout.count(" 0 mismatches") == 8, out.stdout
 
 
 @pytest.mark.parametrize("kw", [
