@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     if (alive) {
       const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
       uint32_t used = 0u;
-      ended = !step_photon<kAdj, BATCH && !UNI, kPath>(P, ws.flags, s, r, fate, aux, used);
+      ended = !step_photon<kAdj, BATCH && !UNI, kPath, BATCH ? kFlat : kBranches>(P, ws.flags, s, r, fate, aux, used);
       if constexpr (kRing) r.consume(used);
       else if (!ended) r.advance(used, first_id + pidx, run_key());
       ++wsteps;
@@ -835,14 +835,14 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
       uint32_t used = 0u;
       if constexpr (kRing) {
         const uint4 next = block(r.made);
-        alive = step_photon<kAdj, BATCH && !UNI, kPath>(P, flags, s, r, fate, aux, used);
+        alive = step_photon<kAdj, BATCH && !UNI, kPath, kLone>(P, flags, s, r, fate, aux, used);
         if (!alive) break;
         r.consume(used);
         if (r.av <= kWindowRoom) r.put(next);
         if (r.av < kStepWords) r.put(block(r.made));
       } else {
         const uint4 next = block(r.blk + 2u);
-        alive = step_photon<kAdj, BATCH && !UNI, kPath>(P, flags, s, r, fate, aux, used);
+        alive = step_photon<kAdj, BATCH && !UNI, kPath, kLone>(P, flags, s, r, fate, aux, used);
         if (!alive) break;
         r.advance(used, id, run_key(), next);
       }

@@ -459,11 +459,12 @@ __device__ __forceinline__ float fresnel_R(float n1, float n2, float eta2, float
 // included), a quarter of the margin; within 2^-10 of total internal
 // reflection, where sqrt(1 - sin2_t) magnifies the rounding of sin2_t, and outside
 // the ordinary range, fresnel_R decides too. Measured against calling it always:
-// batch 9.27 -> 9.09 ms, gradient run of 1e6 photons 0.272 -> 0.259 ms.
+// batch 9.27 -> 9.09 ms, gradient run of 1e6 photons 0.272 -> 0.259 ms. Without
+// `asked` the outcome is not used and may be left open.
 __device__ __forceinline__ bool fresnel_reflects(float n1, float n2, float eta2, float cos_i, float u,
-                                                 uint32_t flags) {
+                                                 uint32_t flags, bool asked = true) {
 #if OPTX_APPROX
-  (void)flags;
+  (void)flags, (void)asked;
   return u <= fresnel_R(n1, n2, eta2, cos_i);
 #else
   const float c2 = 1.0f - eta2 * fmaxf(0.0f, 1.0f - cos_i * cos_i);
@@ -474,7 +475,7 @@ __device__ __forceinline__ bool fresnel_reflects(float n1, float n2, float eta2,
   const float diff = fmaf(v, v, w * w) - 2.0f * u * den;
   bool r = c2 < 0.0f || diff > 0.0f;
   const bool open = !(fabsf(diff) > 0x1p-15f * den) && !(c2 <= -0x1p-10f);
-  if (open || fabsf(c2) < 0x1p-10f || !(flags & kOrdinary)) r = u <= fresnel_R(n1, n2, eta2, cos_i);
+  if (asked && (open || fabsf(c2) < 0x1p-10f || !(flags & kOrdinary))) r = u <= fresnel_R(n1, n2, eta2, cos_i);
   return r;
 #endif
 }
@@ -539,6 +540,16 @@ __device__ __forceinline__ void start_photon(const DevParams& P, const K& key, P
   r.advance(start_photon<false>(P, s, u, aux), id, key);
 }
 
+// How a step is laid out. kBranches: the Fresnel decision and the painted faces behind
+// branches, the rare IEEE box exit behind one after the quotients, which then stand in
+// one block with what precedes them (Lambertian and polished cube, bar 1e8 photons
+// -0.5 to -1 %). kFlat: every lane computes both and selects, for batches, where some
+// lane of a warp nearly always needs each (4096 events 8.10 -> 7.87 ms, with the
+// reordered box exit; in one configuration's main loop the bar gains a percent without
+// it). kLone: as kBranches but with the box exit's branch first, for the last photons
+// of a warp (bar 3e4 photons 209 us, 222 with the branch after).
+enum StepShape { kBranches, kFlat, kLone };
+
 // A step's interaction, decided by step_move: absorption, a scatter, or a hit on the
 // face across the x, y or z axis on the side that `along`, the direction component
 // across it, points to. Predicates rather than a face number: the step asks for the
@@ -586,19 +597,21 @@ __device__ __forceinline__ float box_exit_ieee(const StepParams& P, const Photon
 // photon does not move along is NaN and fminf passes over it; an earlier axis wins
 // a tie, as in the order of the comparisons above. (A direction component is 0 or
 // far above 2^-100: it comes out of sums of products of uniforms and sines.)
+template <StepShape SHAPE = kBranches>
 __device__ __forceinline__ float box_exit(const StepParams& P, uint32_t flags, const Photon& s, Hit& hit) {
 #if OPTX_APPROX
   return box_exit_ieee(P, s, hit);
 #else
-  if (!(flags & kOrdinary)) return box_exit_ieee(P, s, hit);
+  if (SHAPE == kLone && !(flags & kOrdinary)) return box_exit_ieee(P, s, hit);
   const float tx = m_div(copysignf(P.hx, s.dx) - s.px, s.dx);
   const float ty = m_div(copysignf(P.hy, s.dy) - s.py, s.dy);
   const float tz = m_div(copysignf(P.hz, s.dz) - s.pz, s.dz);
-  const float dist = fminf(fminf(tx, ty), tz);
+  float dist = fminf(fminf(tx, ty), tz);
   hit.x = tx == dist;
   hit.y = !hit.x && ty == dist;
   hit.z = !hit.x && !hit.y;
   hit.along = hit.x ? s.dx : (hit.y ? s.dy : s.dz);
+  if (SHAPE != kLone && !(flags & kOrdinary)) dist = box_exit_ieee(P, s, hit);
   return dist;
 #endif
 }
@@ -621,11 +634,11 @@ __device__ __forceinline__ float log_hi(float lg2) { return fmaf(lg2, -0.6931471
 // the bounds leave it open (~1e-5 of the steps). Kernel times against taking both
 // always, with a face number in place of Hit's predicates: polished cube 1e8 photons
 // 8.11 -> 7.70 ms, bar 25.9 -> 25.1, Lambertian cube 13.6 -> 13.1, batch 8.08 -> 7.87.
-template <bool PATH = true, bool ENDS = true, class R>
+template <bool PATH = true, bool ENDS = true, StepShape SHAPE = kBranches, class R>
 __device__ __forceinline__ Hit step_move(const StepParams& P, uint32_t flags, Photon& s, const R& r) {
   const float u_abs = r.template uniform<0>(), u_sca = r.template uniform<1>();
   Hit hit;
-  const float dist = fmaxf(box_exit(P, flags, s, hit), 0.0f);
+  const float dist = fmaxf(box_exit<SHAPE>(P, flags, s, hit), 0.0f);
   float d = dist;
 #if OPTX_APPROX
   {
@@ -673,7 +686,7 @@ __device__ __forceinline__ uint32_t face_model(uint32_t surf_bits, const Hit& hi
 // scattered, mirrored, diffuse), then one pass each of the rotation and the mirror
 // flip for all lanes that need it: fewer branches than a body per outcome (per warp
 // step of the batch 47 of them, not 66; Lambertian cube 1e7 photons 1.63 -> 1.55 ms).
-template <bool AUX, bool GP = false, class R>
+template <bool AUX, bool GP = false, StepShape SHAPE = kBranches, class R>
 __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits, uint32_t flags, Photon& s, const R& r,
                                          uint32_t& fate, ScoreAux& aux, const Hit& hit, uint32_t& used) {
   // The window's words 2..4 as uniforms, once for every outcome (measured -2 % on
@@ -681,20 +694,30 @@ __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits,
   const float u2 = r.template uniform<2>(), u3 = r.template uniform<3>(), u4 = r.template uniform<4>();
   const bool scattered = hit.scatter, surface = hit.surface();
   const uint32_t model = face_model(surf_bits, hit);
+  // Readout face: interface to n_det, transmitted = detected; other polished faces:
+  // interface to n_out, transmitted = escaped (transport.hpp:108-128).
+  auto reflects = [&](bool asked) {
+    float2 n2;  // index beyond the face, eta2
+    if (GP) n2 = __ldg(reinterpret_cast<const float2*>(&P.n_det) + (hit.readout() ? 0 : 1));
+    else n2 = hit.readout() ? make_float2(P.n_det, P.eta2_det) : make_float2(P.n_out, P.eta2_out);
+    return fresnel_reflects(GP ? __ldg(&P.n_scint) : P.n_scint, n2.x, n2.y, fabsf(hit.along), u2, flags, asked);
+  };
+  // Painted reflector: absorbed with 1 - R; black: always (transport.hpp:129-144).
   bool kept = false;
-  if (surface) {
+  if constexpr (SHAPE == kFlat && !OPTX_APPROX) {
+    const bool polished = surface && model == kPolished;
+    const bool reflected = reflects(polished);
+    const float refl = face_refl<GP>(P, hit.face());
+    const bool kept_paint = surface & (model != kBlack) & (u2 <= refl);
+    kept = polished ? reflected : kept_paint;
+    fate = polished ? (hit.readout() ? kDetected : kEscaped) : (surface ? kAbsorbedSurface : kAbsorbedBulk);
+    if (AUX) aux.n_refl += (kept_paint && !polished) ? 1u : 0u;
+    if (surface) ++s.nb;
+  } else if (surface) {
     if (model == kPolished) {
-      // Readout face: interface to n_det, transmitted = detected; other faces:
-      // interface to n_out, transmitted = escaped (transport.hpp:108-128).
-      const bool readout = hit.readout();
-      const float cos_i = fabsf(hit.along);
-      float2 n2;  // index beyond the face, eta2
-      if (GP) n2 = __ldg(reinterpret_cast<const float2*>(&P.n_det) + (readout ? 0 : 1));
-      else n2 = readout ? make_float2(P.n_det, P.eta2_det) : make_float2(P.n_out, P.eta2_out);
-      kept = fresnel_reflects(GP ? __ldg(&P.n_scint) : P.n_scint, n2.x, n2.y, cos_i, u2, flags);
-      fate = readout ? kDetected : kEscaped;
+      kept = reflects(true);
+      fate = hit.readout() ? kDetected : kEscaped;
     } else {
-      // Painted reflector: absorbed with 1 - R; black: always (transport.hpp:129-144).
       kept = model != kBlack && u2 <= face_refl<GP>(P, hit.face());
       fate = kAbsorbedSurface;
       if (AUX && kept) ++aux.n_refl;
@@ -732,12 +755,12 @@ __device__ __forceinline__ bool step_act(const DevParams& P, uint32_t surf_bits,
 // One step (transport.hpp:71-145): move, then interact. `flags`: those that hold for
 // every record of the run. False when the photon has ended, with its fate, or has
 // made max_steps steps (the fate is then kMaxSteps); true with the words used.
-template <bool AUX, bool GP = false, bool PATH = true, class R>
+template <bool AUX, bool GP = false, bool PATH = true, StepShape SHAPE = kBranches, class R>
 __device__ __forceinline__ bool step_photon(const DevParams& P, uint32_t flags, Photon& s, const R& r, uint32_t& fate,
                                             ScoreAux& aux, uint32_t& used) {
   const StepParams q = load_step<GP>(P);
-  const Hit hit = step_move<PATH, PATH && !AUX>(q, flags, s, r);
-  const bool live = step_act<AUX, GP>(P, q.surf_bits, flags, s, r, fate, aux, hit, used);
+  const Hit hit = step_move<PATH, PATH && !AUX, SHAPE>(q, flags, s, r);
+  const bool live = step_act<AUX, GP, SHAPE>(P, q.surf_bits, flags, s, r, fate, aux, hit, used);
   return live && s.nb + s.ns < q.max_steps;
 }
 
