@@ -17,6 +17,7 @@
 #include <unistd.h>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -200,6 +201,8 @@ int ensure_device() {
 // Forgets the looked-up device addresses of the allocation-free call's static
 // scratch (defined with that call, at the end of this file).
 void noalloc_forget_addresses();
+// Frees the engines kept by the event-records calls (defined with them).
+void free_event_engines();
 
 int num_sms() {
   int dev = 0, n = 0;
@@ -271,18 +274,6 @@ int cache_tally(size_t len) {
     OPTX_CUDA(cudaMalloc(&g_cache.tally, len * 8));
     g_cache.tally_bytes = len * 8;
   }
-  return OPTX_OK;
-}
-
-int copy_records_d2h(const optx_records* out, uint64_t offset, const DevRecords& d, uint64_t m) {
-  OPTX_CUDA(cudaMemcpy(out->fate + offset, d.fate, m, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->n_boundary + offset, d.n_boundary, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->n_scatter + offset, d.n_scatter, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->t + offset, d.t, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->x + offset, d.x, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->y + offset, d.y, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->z + offset, d.z, m * 4, cudaMemcpyDeviceToHost));
-  OPTX_CUDA(cudaMemcpy(out->path + offset, d.path, m * 4, cudaMemcpyDeviceToHost));
   return OPTX_OK;
 }
 
@@ -792,12 +783,16 @@ int engine_check_ctrl(optx_engine* e, WaveCtrl& c, cudaStream_t st) {
 // pageable vectors, gpu_backend.cu:119-156, cuda_util.cuh:98-111).
 namespace {
 
+constexpr uint64_t kPiece = 1ull << 18;  // photons per staged copy (7.6 MB)
+constexpr int kSlots = 3;                // staging slots: copies in flight ahead of the host
+
 struct RecPipe {
-  uint64_t cap = 0;  // photons per buffer set
+  uint64_t cap[2] = {0, 0};   // photons per device buffer set
+  uint64_t pin_cap = 0;       // photons per staging slot
   void* dev[2] = {nullptr, nullptr};
-  unsigned char* pin[2] = {nullptr, nullptr};
+  unsigned char* pin[kSlots] = {};
   cudaStream_t comp = nullptr, copy = nullptr;
-  cudaEvent_t k0[2], k1[2], c1[2];
+  cudaEvent_t k0[2], k1[2], c1[2], done[kSlots];
   unsigned* err = nullptr;  // pinned: the run's error word per buffer set
   WaveCtrl* ctrl = nullptr;  // device: the control blocks they are read from
   bool events = false;
@@ -818,7 +813,8 @@ void carve(unsigned char* base, uint64_t cap, Ptr& fate, Ptr (&w)[7]) {
 }
 size_t set_bytes(uint64_t cap) { return cap + 7 * ((cap * 4 + 255) & ~size_t(255)) + 256; }
 
-int pipe_ensure(uint64_t cap) {
+// Streams and events, and `sets` device buffer sets of `cap` photons.
+int pipe_ensure(int sets, uint64_t cap) {
   if (!g_pipe.events) {
     OPTX_CUDA(cudaStreamCreateWithFlags(&g_pipe.comp, cudaStreamNonBlocking));
     OPTX_CUDA(cudaStreamCreateWithFlags(&g_pipe.copy, cudaStreamNonBlocking));
@@ -827,25 +823,35 @@ int pipe_ensure(uint64_t cap) {
       OPTX_CUDA(cudaEventCreate(&g_pipe.k1[b]));
       OPTX_CUDA(cudaEventCreate(&g_pipe.c1[b]));
     }
+    for (cudaEvent_t& e : g_pipe.done) OPTX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g_pipe.err), 2 * sizeof(unsigned),
                             cudaHostAllocDefault));
     g_pipe.events = true;
   }
   if (g_pipe.ctrl == nullptr) OPTX_CUDA(cudaMalloc(&g_pipe.ctrl, 2 * sizeof(WaveCtrl)));
-  if (g_pipe.cap >= cap) return OPTX_OK;
-  for (int b = 0; b < 2; ++b) {
-    if (g_pipe.dev[b]) cudaFree(g_pipe.dev[b]);
-    if (g_pipe.pin[b]) cudaFreeHost(g_pipe.pin[b]);
+  for (int b = 0; b < sets; ++b) {
+    if (g_pipe.cap[b] >= cap) continue;
+    cudaFree(g_pipe.dev[b]);
     g_pipe.dev[b] = nullptr;
-    g_pipe.pin[b] = nullptr;
-  }
-  g_pipe.cap = 0;
-  for (int b = 0; b < 2; ++b) {
+    g_pipe.cap[b] = 0;
     OPTX_CUDA(cudaMalloc(&g_pipe.dev[b], set_bytes(cap)));
-    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g_pipe.pin[b]), set_bytes(cap),
-                            cudaHostAllocDefault));
+    g_pipe.cap[b] = cap;
   }
-  g_pipe.cap = cap;
+  return OPTX_OK;
+}
+
+// Staging slots of `cap` photons, for pageable caller arrays.
+int pipe_ensure_staging(uint64_t cap) {
+  if (g_pipe.pin_cap >= cap) return OPTX_OK;
+  OPTX_CUDA(cudaStreamSynchronize(g_pipe.copy));  // no copy of an earlier, failed call still lands there
+  g_pipe.pin_cap = 0;
+  for (unsigned char*& p : g_pipe.pin) {
+    cudaFreeHost(p);
+    p = nullptr;
+  }
+  for (unsigned char*& p : g_pipe.pin)
+    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), set_bytes(cap), cudaHostAllocDefault));
+  g_pipe.pin_cap = cap;
   return OPTX_OK;
 }
 
@@ -862,27 +868,83 @@ bool is_pinned(const void* p) {
 // staging copies for host memory bandwidth).
 unsigned copy_threads() { return std::max(1u, std::min(8u, std::thread::hardware_concurrency())); }
 
-// memcpy of large blocks split over a few host threads.
-void parallel_copy(const std::vector<std::tuple<void*, const void*, size_t>>& jobs) {
-  size_t total = 0;
-  for (auto& j : jobs) total += std::get<2>(j);
-  const unsigned hw = copy_threads();
-  if (total < (8u << 20) || hw == 1) {
-    for (auto& j : jobs) std::memcpy(std::get<0>(j), std::get<1>(j), std::get<2>(j));
-    return;
+// memcpy of large blocks split over a few host threads, which live as long as the
+// call that owns the crew (started with its first large copy).
+class CopyCrew {
+ public:
+  struct Job {
+    void* to;
+    const void* from;
+    size_t bytes;
+  };
+  void copy(const std::vector<Job>& jobs) {
+    size_t total = 0;
+    for (const Job& j : jobs) total += j.bytes;
+    if (total >= (2u << 20) && helpers_.empty() && !tried_) start();
+    const size_t n = helpers_.empty() || total < (2u << 20) ? 1 : helpers_.size() + 1;
+    if (n > 1) {
+      std::lock_guard<std::mutex> lk(mu_);
+      jobs_ = &jobs;
+      left_ = helpers_.size();
+      ++round_;
+      go_.notify_all();
+    }
+    part(jobs, n - 1, n);
+    if (n > 1) {
+      std::unique_lock<std::mutex> lk(mu_);
+      end_.wait(lk, [&] { return left_ == 0; });
+    }
   }
-  std::vector<std::thread> th;
-  for (unsigned t = 0; t < hw; ++t) {
-    th.emplace_back([&, t] {
-      for (auto& j : jobs) {
-        const size_t b = std::get<2>(j), lo = b * t / hw, hi = b * (t + 1) / hw;
-        std::memcpy(static_cast<char*>(std::get<0>(j)) + lo, static_cast<const char*>(std::get<1>(j)) + lo,
-                    hi - lo);
-      }
-    });
+  ~CopyCrew() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      stop_ = true;
+      go_.notify_all();
+    }
+    for (auto& x : helpers_) x.join();
   }
-  for (auto& x : th) x.join();
-}
+
+ private:
+  static void part(const std::vector<Job>& jobs, size_t t, size_t n) {
+    for (const Job& j : jobs) {
+      const size_t lo = j.bytes * t / n, hi = j.bytes * (t + 1) / n;
+      std::memcpy(static_cast<char*>(j.to) + lo, static_cast<const char*>(j.from) + lo, hi - lo);
+    }
+  }
+  void start() {
+    tried_ = true;
+    const size_t want = copy_threads() - 1u;
+    try {
+      helpers_.reserve(want);
+      for (size_t t = 0; t < want; ++t)
+        helpers_.emplace_back([this, t] {
+          for (uint64_t seen = 0;;) {
+            const std::vector<Job>* jobs;
+            size_t n;
+            {
+              std::unique_lock<std::mutex> lk(mu_);
+              go_.wait(lk, [&] { return stop_ || round_ != seen; });
+              if (stop_) return;
+              seen = round_;
+              jobs = jobs_;
+              n = helpers_.size() + 1;
+            }
+            part(*jobs, t, n);
+            std::lock_guard<std::mutex> lk(mu_);
+            if (--left_ == 0) end_.notify_one();
+          }
+        });
+    } catch (const std::exception&) {  // no more threads: those that started do the copies
+    }
+  }
+  std::vector<std::thread> helpers_;
+  std::mutex mu_;
+  std::condition_variable go_, end_;
+  const std::vector<Job>* jobs_ = nullptr;
+  size_t left_ = 0;
+  uint64_t round_ = 0;
+  bool stop_ = false, tried_ = false;
+};
 
 // Fraction of the pages of [p, p + len) resident in memory (1 when unknown).
 double resident_fraction(void* p, size_t len, size_t page) {
@@ -933,6 +995,72 @@ class PageToucher {
  private:
   std::vector<std::thread> th_;
 };
+
+// Brings the records d[0, m) to the caller's arrays from entry `at` on, once `ready`
+// has happened; c1 follows the last copy. Pinned arrays receive the DMA directly;
+// pageable ones through the staging slots, piece by piece: the host copies one piece
+// out while the next are on their way. (As one piece, 1e6 records took their kernel,
+// 0.6 ms of DMA and 1.1 ms of host copies one after another.)
+struct RecordArrays {
+  void* outs[8];
+  bool direct;
+  explicit RecordArrays(const optx_records* r)
+      : outs{r->fate, r->n_boundary, r->n_scatter, r->t, r->x, r->y, r->z, r->path}, direct(true) {
+    for (void* q : outs) direct = direct && is_pinned(q);
+  }
+  static size_t elem(int k) { return k == 0 ? 1u : 4u; }
+  std::vector<std::pair<void*, size_t>> ranges(uint64_t n) const {
+    std::vector<std::pair<void*, size_t>> v;
+    for (int k = 0; k < 8; ++k) v.emplace_back(outs[k], n * elem(k));
+    return v;
+  }
+};
+int records_out(const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t at, cudaEvent_t ready, cudaEvent_t c1,
+                CopyCrew& crew, PageToucher* touch) {
+  const void* from[8] = {d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
+  OPTX_CUDA(cudaStreamWaitEvent(g_pipe.copy, ready, 0));
+  const uint64_t piece = a.direct ? m : std::min(m, kPiece);
+  if (!a.direct) OPTX_TRY(pipe_ensure_staging(piece));
+  const uint64_t pieces = (m + piece - 1) / piece;
+  auto slot = [&](int i) {
+    unsigned char* fate;
+    unsigned char* w[7];
+    carve(g_pipe.pin[i], g_pipe.pin_cap, fate, w);
+    return std::array<unsigned char*, 8>{fate, w[0], w[1], w[2], w[3], w[4], w[5], w[6]};
+  };
+  auto queue = [&](uint64_t j) -> int {
+    const uint64_t lo = j * piece, cnt = std::min(piece, m - lo);
+    std::array<unsigned char*, 8> pin{};
+    if (!a.direct) pin = slot(static_cast<int>(j % kSlots));
+    for (int k = 0; k < 8; ++k) {
+      const size_t e = RecordArrays::elem(k);
+      void* to = a.direct ? static_cast<char*>(a.outs[k]) + (at + lo) * e : static_cast<void*>(pin[k]);
+      OPTX_CUDA(cudaMemcpyAsync(to, static_cast<const char*>(from[k]) + lo * e, cnt * e, cudaMemcpyDeviceToHost,
+                                g_pipe.copy));
+    }
+    if (!a.direct) OPTX_CUDA(cudaEventRecord(g_pipe.done[j % kSlots], g_pipe.copy));
+    if (j + 1 == pieces) OPTX_CUDA(cudaEventRecord(c1, g_pipe.copy));
+    return OPTX_OK;
+  };
+  for (uint64_t j = 0; j < std::min<uint64_t>(kSlots, pieces); ++j) OPTX_TRY(queue(j));
+  if (!a.direct) {
+    for (uint64_t j = 0; j < pieces; ++j) {
+      OPTX_CUDA(cudaEventSynchronize(g_pipe.done[j % kSlots]));
+      if (touch != nullptr) touch->join();
+      const uint64_t lo = j * piece, cnt = std::min(piece, m - lo);
+      const auto pin = slot(static_cast<int>(j % kSlots));
+      std::vector<CopyCrew::Job> jobs;
+      for (int k = 0; k < 8; ++k) {
+        const size_t e = RecordArrays::elem(k);
+        jobs.push_back({static_cast<char*>(a.outs[k]) + (at + lo) * e, pin[k], cnt * e});
+      }
+      crew.copy(jobs);
+      if (j + kSlots < pieces) OPTX_TRY(queue(j + kSlots));
+    }
+  }
+  OPTX_CUDA(cudaEventSynchronize(c1));
+  return OPTX_OK;
+}
 
 // ---- one configuration as fixed shares ---------------------------------------
 // The wave kernel with one block per SM, each running an equal share of the photons
@@ -1066,6 +1194,7 @@ int optx_release_cache(void) {
   // No records call is in flight while g_event_mu (held to the end, so that
   // g_cache.rec is not in use when it is freed) and g_pipe_mu are held.
   std::lock_guard<std::mutex> elk(g_event_mu);
+  free_event_engines();
   std::vector<std::shared_ptr<TallySpace>> spaces;  // destroyed after g_mu, once unused
   {
     // Copies left queued by a records call that returned an error are drained first.
@@ -1075,12 +1204,15 @@ int optx_release_cache(void) {
       cudaStreamSynchronize(g_pipe.copy);
     }
     for (int b = 0; b < 2; ++b) {
-      if (g_pipe.dev[b]) cudaFree(g_pipe.dev[b]);
-      if (g_pipe.pin[b]) cudaFreeHost(g_pipe.pin[b]);
+      cudaFree(g_pipe.dev[b]);
       g_pipe.dev[b] = nullptr;
-      g_pipe.pin[b] = nullptr;
+      g_pipe.cap[b] = 0;
     }
-    g_pipe.cap = 0;
+    for (unsigned char*& p : g_pipe.pin) {
+      cudaFreeHost(p);
+      p = nullptr;
+    }
+    g_pipe.pin_cap = 0;
     cudaFree(g_pipe.ctrl);
     g_pipe.ctrl = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
@@ -1121,87 +1253,50 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
   // buffer sets of at most 2^22 photons each within it.
   const uint64_t cap = std::max<uint64_t>(
       1, std::min<uint64_t>({n, chunk ? chunk : (uint64_t{1} << 24), uint64_t{1} << 22}));
+  const uint64_t chunks = (n + cap - 1) / cap;
   const auto ta = std::chrono::steady_clock::now();
-  OPTX_TRY(pipe_ensure(cap));
+  OPTX_TRY(pipe_ensure(chunks > 1 ? 2 : 1, cap));
+  tm.alloc_ms = ms_since(ta);
   TallyDev none{};
   none.len = 7u;  // no histograms
-  tm.alloc_ms = ms_since(ta);
-  void* outs[8] = {out->fate, out->n_boundary, out->n_scatter, out->t, out->x, out->y, out->z, out->path};
-  bool direct = true;
-  for (void* q : outs) direct = direct && is_pinned(q);
-  const size_t elem[8] = {1, 4, 4, 4, 4, 4, 4, 4};
-  auto views = [&](int b, bool host) {
-    unsigned char* base = host ? g_pipe.pin[b] : static_cast<unsigned char*>(g_pipe.dev[b]);
+  const RecordArrays arrays(out);
+  auto dev_set = [&](int b) {
     unsigned char* fate;
     unsigned char* w[7];
-    carve(base, cap, fate, w);
-    std::array<unsigned char*, 8> v{fate, w[0], w[1], w[2], w[3], w[4], w[5], w[6]};
-    return v;
+    carve(static_cast<unsigned char*>(g_pipe.dev[b]), cap, fate, w);
+    return DevRecords{fate, reinterpret_cast<uint32_t*>(w[0]), reinterpret_cast<uint32_t*>(w[1]),
+                      reinterpret_cast<float*>(w[2]), reinterpret_cast<float*>(w[3]), reinterpret_cast<float*>(w[4]),
+                      reinterpret_cast<float*>(w[5]), reinterpret_cast<float*>(w[6])};
   };
-  const uint64_t chunks = (n + cap - 1) / cap;
-  float kms = 0.f, cms = 0.f;
-  std::unique_ptr<PageToucher> touch;  // started once the first chunk is queued
-  auto host_fill = [&](uint64_t i) {  // staging set (i % 2) -> caller arrays
-    if (touch) touch->join();
-    const uint64_t done = i * cap, m = std::min(cap, n - done);
-    auto src = views(static_cast<int>(i % 2), true);
-    std::vector<std::tuple<void*, const void*, size_t>> jobs;
-    for (int k = 0; k < 8; ++k)
-      jobs.emplace_back(static_cast<char*>(outs[k]) + done * elem[k], src[k], m * elem[k]);
-    parallel_copy(jobs);
-  };
-  for (uint64_t i = 0; i < chunks; ++i) {
+  // Chunk i's kernel into set i % 2, whose previous chunk has been copied out.
+  auto launch = [&](uint64_t i) -> int {
     const int b = static_cast<int>(i % 2);
     const uint64_t done = i * cap, m = std::min(cap, n - done);
-    auto dv = views(b, false);
-    // the device set b is free once the copy of chunk i - 2 has finished
-    if (i >= 2) OPTX_CUDA(cudaStreamWaitEvent(g_pipe.comp, g_pipe.c1[b], 0));
+    const DevRecords d = dev_set(b);
     OPTX_CUDA(cudaEventRecord(g_pipe.k0[b], g_pipe.comp));
-    const DevRecords d{dv[0], reinterpret_cast<uint32_t*>(dv[1]), reinterpret_cast<uint32_t*>(dv[2]),
-                       reinterpret_cast<float*>(dv[3]), reinterpret_cast<float*>(dv[4]),
-                       reinterpret_cast<float*>(dv[5]), reinterpret_cast<float*>(dv[6]),
-                       reinterpret_cast<float*>(dv[7])};
     OPTX_CUDA(cudaMemsetAsync(&g_pipe.ctrl[b], 0, sizeof(WaveCtrl), g_pipe.comp));
     OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &d, &g_pipe.ctrl[b], math, g_pipe.comp));
     OPTX_CUDA(cudaMemcpyAsync(&g_pipe.err[b], &g_pipe.ctrl[b].error, sizeof(unsigned), cudaMemcpyDeviceToHost,
                               g_pipe.comp));
     OPTX_CUDA(cudaEventRecord(g_pipe.k1[b], g_pipe.comp));
-    OPTX_CUDA(cudaStreamWaitEvent(g_pipe.copy, g_pipe.k1[b], 0));
-    auto hv = views(b, true);
-    for (int k = 0; k < 8; ++k) {
-      void* dst = direct ? static_cast<void*>(static_cast<char*>(outs[k]) + done * elem[k])
-                         : static_cast<void*>(hv[k]);
-      OPTX_CUDA(cudaMemcpyAsync(dst, dv[k], m * elem[k], cudaMemcpyDeviceToHost, g_pipe.copy));
-    }
-    OPTX_CUDA(cudaEventRecord(g_pipe.c1[b], g_pipe.copy));
-    if (i == 0 && !direct) {
-      std::vector<std::pair<void*, size_t>> ranges;
-      for (int k = 0; k < 8; ++k) ranges.emplace_back(outs[k], n * elem[k]);
-      touch.reset(new PageToucher(ranges));
-    }
-    if (i >= 1) {  // finish chunk i - 1 on the host while chunk i computes and copies
-      const int pb = static_cast<int>((i - 1) % 2);
-      OPTX_CUDA(cudaEventSynchronize(g_pipe.c1[pb]));
-      float ms = 0.f;
-      OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k0[pb], g_pipe.k1[pb]));
-      kms += ms;
-      OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[pb], g_pipe.c1[pb]));
-      cms += ms;
-      OPTX_TRY(run_error(g_pipe.err[pb]));
-      if (!direct) host_fill(i - 1);
-    }
+    return OPTX_OK;
+  };
+  CopyCrew crew;
+  std::unique_ptr<PageToucher> touch;  // started once the first chunk is queued
+  OPTX_TRY(launch(0));
+  if (!arrays.direct) touch.reset(new PageToucher(arrays.ranges(n)));
+  for (uint64_t i = 0; i < chunks; ++i) {
+    const int b = static_cast<int>(i % 2);
+    if (i + 1 < chunks) OPTX_TRY(launch(i + 1));  // computes while chunk i is copied out
+    const uint64_t done = i * cap, m = std::min(cap, n - done);
+    OPTX_TRY(records_out(arrays, dev_set(b), m, done, g_pipe.k1[b], g_pipe.c1[b], crew, touch.get()));
+    float ms = 0.f;
+    OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k0[b], g_pipe.k1[b]));
+    tm.kernel_ms += ms;
+    OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[b], g_pipe.c1[b]));
+    tm.d2h_ms += ms;  // kernel end to copy end per chunk (copies overlap later kernels)
+    OPTX_TRY(run_error(g_pipe.err[b]));
   }
-  const int lb = static_cast<int>((chunks - 1) % 2);
-  OPTX_CUDA(cudaEventSynchronize(g_pipe.c1[lb]));
-  float ms = 0.f;
-  OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k0[lb], g_pipe.k1[lb]));
-  kms += ms;
-  OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[lb], g_pipe.c1[lb]));
-  cms += ms;
-  OPTX_TRY(run_error(g_pipe.err[lb]));
-  if (!direct) host_fill(chunks - 1);
-  tm.kernel_ms = kms;
-  tm.d2h_ms = cms;  // kernel end to copy end per chunk (copies overlap later kernels)
   tm.total_ms = ms_since(t0);
   if (timing) *timing = tm;
   return OPTX_OK;
@@ -1929,6 +2024,62 @@ int optx_run_batch(optx_engine* e, const optx_params* events, const optx_faces* 
   return OPTX_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// Engines of the event-records calls, kept from call to call: creating one (queues,
+// tables, its graph of the forced-compaction loop) and freeing it took 2.5 ms of a 4 ms
+// call of 3e5 photons. At most kEventEngines, the newest, none with queues above
+// kEventQueueBytes; guarded by g_event_mu; freed by optx_release_cache.
+struct EventEngine {
+  int device, math, block;
+  uint32_t threshold, cadence;
+  uint64_t cap;
+  optx_engine* e;
+};
+std::vector<EventEngine>& g_event_engines = *new std::vector<EventEngine>();  // not destroyed at exit
+constexpr size_t kEventEngines = 4;
+constexpr uint64_t kEventQueueBytes = 256ull << 20;
+
+int take_event_engine(const optx_tally_config& tc, const optx_wave_config& cfg, uint64_t cap, optx_engine** out) {
+  int dev = 0;
+  OPTX_CUDA(cudaGetDevice(&dev));
+  for (size_t i = 0; i < g_event_engines.size(); ++i) {
+    const EventEngine& k = g_event_engines[i];
+    if (k.device == dev && k.math == cfg.math && k.block == cfg.block_size && k.threshold == cfg.threshold &&
+        k.cadence == cfg.cadence && k.cap == cap) {
+      *out = k.e;
+      g_event_engines.erase(g_event_engines.begin() + static_cast<std::ptrdiff_t>(i));
+      return OPTX_OK;
+    }
+  }
+  return optx_engine_create(&tc, 1, cap, &cfg, out);
+}
+
+// Keeps the engine for the next call, or frees it (after an error, or a large one).
+void give_event_engine(optx_engine* e, bool keep) {
+  int dev = 0;
+  if (!keep || 128ull * e->qcap > kEventQueueBytes || cudaGetDevice(&dev) != cudaSuccess) {
+    optx_engine_destroy(e);
+    return;
+  }
+  if (g_event_engines.size() >= kEventEngines) {
+    optx_engine_destroy(g_event_engines.front().e);
+    g_event_engines.erase(g_event_engines.begin());
+  }
+  g_event_engines.push_back({dev, e->cfg.math, e->cfg.block_size, e->cfg.threshold, e->cfg.cadence, e->max_photons, e});
+}
+
+void free_event_engines() {  // with g_event_mu held
+  for (EventEngine& k : g_event_engines) optx_engine_destroy(k.e);
+  g_event_engines.clear();
+}
+
+}  // namespace
+
+extern "C" {
+
 int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64_t n,
                            const optx_records* out, uint32_t steps_per_launch, int block_size,
                            uint64_t first_id, uint64_t chunk, int math, optx_event_stats* stats,
@@ -1960,21 +2111,27 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
   cfg.use_graph = 1;
   cfg.math = math;
   optx_engine* e = nullptr;
-  OPTX_TRY(optx_engine_create(&tc, 1, cap, &cfg, &e));
+  OPTX_TRY(take_event_engine(tc, cfg, cap, &e));
   optx_timing tm{};
   optx_event_stats st{};
   int rc = OPTX_OK;
-  {
-    std::unique_lock<std::mutex> lk(g_mu);
+  if (n > 0) {
+    std::lock_guard<std::mutex> pipe_lk(g_pipe_mu);
+    rc = pipe_ensure(0, 0);
     DevRecords d{};
-    rc = cache_records(cap, d);
-    lk.unlock();
+    if (rc == OPTX_OK) {
+      std::lock_guard<std::mutex> lk(g_mu);
+      rc = cache_records(cap, d);
+    }
+    CopyCrew crew;
+    std::unique_ptr<PageToucher> touch;
+    const RecordArrays arrays(out);
+    const optx_records dr{d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
     for (uint64_t done = 0; rc == OPTX_OK && done < n; done += cap) {
       const uint64_t m = std::min(cap, n - done);
-      const uint64_t cnt = m;
-      if ((rc = optx_engine_set_events(e, p, faces, &cnt, 1, first_id + done, nullptr)) != OPTX_OK) break;
-      const optx_records dr{d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
+      if ((rc = optx_engine_set_events(e, p, faces, &m, 1, first_id + done, nullptr)) != OPTX_OK) break;
       if ((rc = optx_engine_run_records(e, &dr, nullptr)) != OPTX_OK) break;
+      if (done == 0 && !arrays.direct) touch.reset(new PageToucher(arrays.ranges(n)));
       optx_event_stats s{};
       if ((rc = optx_engine_stats(e, &s, nullptr)) != OPTX_OK) break;
       st.launches += s.launches;
@@ -1983,13 +2140,11 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
       st.spills += s.spills;
       st.kernels_ms += s.kernels_ms;
       const auto tcp = std::chrono::steady_clock::now();
-      lk.lock();
-      rc = copy_records_d2h(out, done, d, m);
-      lk.unlock();
+      rc = records_out(arrays, d, m, done, e->ev1, g_pipe.c1[0], crew, touch.get());
       tm.d2h_ms += ms_since(tcp);
     }
   }
-  optx_engine_destroy(e);
+  give_event_engine(e, rc == OPTX_OK);
   if (rc != OPTX_OK) return rc;
   tm.kernel_ms = st.kernels_ms;
   tm.total_ms = ms_since(t0);
