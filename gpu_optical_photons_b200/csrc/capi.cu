@@ -783,7 +783,10 @@ int engine_check_ctrl(optx_engine* e, WaveCtrl& c, cudaStream_t st) {
 // pageable vectors, gpu_backend.cu:119-156, cuda_util.cuh:98-111).
 namespace {
 
-constexpr uint64_t kPiece = 1ull << 18;  // photons per staged copy (7.6 MB)
+// Photons per staged copy (15 MB): 1e6 records into the caller's arrays take 1.1 to
+// 1.3 ms with it, 1.8 with 2^18 (a piece costs the helper threads' wake-up) and 2.3
+// with 2^20 (nothing overlaps).
+constexpr uint64_t kPiece = 1ull << 19;
 constexpr int kSlots = 3;                // staging slots: copies in flight ahead of the host
 
 struct RecPipe {
@@ -868,8 +871,14 @@ bool is_pinned(const void* p) {
 // staging copies for host memory bandwidth).
 unsigned copy_threads() { return std::max(1u, std::min(8u, std::thread::hardware_concurrency())); }
 
-// memcpy of large blocks split over a few host threads, which live as long as the
-// call that owns the crew (started with its first large copy).
+// Threads for a copy of so many bytes: more than one per 2 MB get in each other's way
+// (8.7 MB into fresh pages 1.4 ms with 4, 2.0 with 8).
+unsigned copy_threads_for(size_t bytes) {
+  return std::max(1u, static_cast<unsigned>(std::min<size_t>(copy_threads(), bytes >> 21)));
+}
+
+// memcpy of large blocks split over a few host threads, started with the first large
+// copy and kept between calls (g_crew; starting them took 0.15 ms of each).
 class CopyCrew {
  public:
   struct Job {
@@ -880,11 +889,13 @@ class CopyCrew {
   void copy(const std::vector<Job>& jobs) {
     size_t total = 0;
     for (const Job& j : jobs) total += j.bytes;
-    if (total >= (2u << 20) && helpers_.empty() && !tried_) start();
-    const size_t n = helpers_.empty() || total < (2u << 20) ? 1 : helpers_.size() + 1;
+    size_t n = copy_threads_for(total);
+    if (n > 1 && !tried_) start();
+    n = std::min(n, helpers_.size() + 1);
     if (n > 1) {
       std::lock_guard<std::mutex> lk(mu_);
       jobs_ = &jobs;
+      parts_ = n;
       left_ = helpers_.size();
       ++round_;
       go_.notify_all();
@@ -927,9 +938,9 @@ class CopyCrew {
               if (stop_) return;
               seen = round_;
               jobs = jobs_;
-              n = helpers_.size() + 1;
+              n = parts_;
             }
-            part(*jobs, t, n);
+            if (t + 1 < n) part(*jobs, t, n);
             std::lock_guard<std::mutex> lk(mu_);
             if (--left_ == 0) end_.notify_one();
           }
@@ -941,10 +952,15 @@ class CopyCrew {
   std::mutex mu_;
   std::condition_variable go_, end_;
   const std::vector<Job>* jobs_ = nullptr;
-  size_t left_ = 0;
+  size_t left_ = 0, parts_ = 0;
   uint64_t round_ = 0;
   bool stop_ = false, tried_ = false;
 };
+CopyCrew* g_crew = nullptr;  // guarded by g_pipe_mu; freed by optx_release_cache, not at exit
+CopyCrew& copy_crew() {
+  if (g_crew == nullptr) g_crew = new CopyCrew();
+  return *g_crew;
+}
 
 // Fraction of the pages of [p, p + len) resident in memory (1 when unknown).
 double resident_fraction(void* p, size_t len, size_t page) {
@@ -969,7 +985,7 @@ class PageToucher {
   PageToucher(const std::vector<std::pair<void*, size_t>>& ranges) {
     size_t total = 0;
     for (auto& r : ranges) total += r.second;
-    const unsigned hw = copy_threads();
+    const unsigned hw = copy_threads_for(total);
     if (total < (8u << 20) || hw == 1) return;
     const size_t page = static_cast<size_t>(std::max(4096L, sysconf(_SC_PAGESIZE)));
     size_t res = 0;
@@ -999,8 +1015,8 @@ class PageToucher {
 // Brings the records d[0, m) to the caller's arrays from entry `at` on, once `ready`
 // has happened; c1 follows the last copy. Pinned arrays receive the DMA directly;
 // pageable ones through the staging slots, piece by piece: the host copies one piece
-// out while the next are on their way. (As one piece, 1e6 records took their kernel,
-// 0.6 ms of DMA and 1.1 ms of host copies one after another.)
+// out while the next are on their way. (Kernel, 0.6 ms of DMA and 1.1 ms of host copies
+// of 1e6 records used to follow one another.)
 struct RecordArrays {
   void* outs[8];
   bool direct;
@@ -1213,6 +1229,8 @@ int optx_release_cache(void) {
       p = nullptr;
     }
     g_pipe.pin_cap = 0;
+    delete g_crew;
+    g_crew = nullptr;
     cudaFree(g_pipe.ctrl);
     g_pipe.ctrl = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
@@ -1281,7 +1299,7 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
     OPTX_CUDA(cudaEventRecord(g_pipe.k1[b], g_pipe.comp));
     return OPTX_OK;
   };
-  CopyCrew crew;
+  CopyCrew& crew = copy_crew();
   std::unique_ptr<PageToucher> touch;  // started once the first chunk is queued
   OPTX_TRY(launch(0));
   if (!arrays.direct) touch.reset(new PageToucher(arrays.ranges(n)));
@@ -2123,7 +2141,7 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
       std::lock_guard<std::mutex> lk(g_mu);
       rc = cache_records(cap, d);
     }
-    CopyCrew crew;
+    CopyCrew& crew = copy_crew();
     std::unique_ptr<PageToucher> touch;
     const RecordArrays arrays(out);
     const optx_records dr{d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
