@@ -233,6 +233,16 @@ struct Window {
     ++made;
   }
 };
+// The stream of one of a warp's last photons: a ring of kLoneWords uniforms in shared
+// memory that the whole warp fills (wave_kernel, drain), word w at place w mod kLoneWords.
+constexpr uint32_t kLoneWords = 64u;
+struct LoneStream {
+  const float* ring;
+  uint32_t next;  // words used so far (the reference's PhiloxStream::draws())
+  template <int I>
+  __device__ __forceinline__ float uniform() const { return ring[(next + I) & (kLoneWords - 1u)]; }
+};
+
 // Words a step reads at most, and room for another block.
 constexpr uint32_t kStepWords = 5u, kWindowRoom = kWindowWords - 4u;
 
