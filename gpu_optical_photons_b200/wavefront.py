@@ -3,8 +3,8 @@
 A ``WavefrontEngine`` owns its device state queues, control block, per-event
 tallies and captured CUDA graphs. ``set_events`` uploads a batch (one or
 thousands of events with their own SimParams and photon counts); the run is
-one graph launch: a prep kernel, then a device-side while loop of persistent
-wave kernels. Event i owns photon ids ``first_id + offset_i + k``, so each
+a prep kernel and one persistent wave kernel, or, where it may need several
+waves, one graph launch with a device-side while loop of them. Event i owns photon ids ``first_id + offset_i + k``, so each
 event reproduces the reference's ``run_cpu_*(p_i, n_i, ..., first_id=offset_i)``.
 """
 from __future__ import annotations
@@ -30,7 +30,7 @@ class WaveConfig:
     math: str = "fast"
     chunk: int = 0              # consecutive photons a warp claims per grab (0 = 32 to 256 by the run's photons)
     max_gensteps: int = 0       # capacity for set_gensteps (0 = no gensteps)
-    tail_steps: int = 0         # steps in a wave before a photon may move to the next (0 = 4096)
+    tail_steps: int = 0         # steps in a wave before a photon may move to the next (0 = library's choice)
 
     @property
     def launch_block_size(self) -> int:

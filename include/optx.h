@@ -109,8 +109,8 @@ typedef struct optx_wave_config {
                             by the run's photons); results do not depend on it */
   uint32_t max_gensteps; /* capacity for optx_engine_set_gensteps, 0 = none (default) */
   uint32_t tail_steps;   /* at the end of a wave a photon moves on to the next wave only after
-                            this many steps in the wave (default 4096: in practice a warp keeps its
-                            photons until they finish); results do not depend on it */
+                            this many steps in the wave (default: a run of one wave keeps its photons
+                            until they finish, others 4096); results do not depend on it */
   uint32_t reserved;     /* must be 0 */
 } optx_wave_config;
 
