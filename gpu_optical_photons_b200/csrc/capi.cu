@@ -1079,7 +1079,7 @@ int records_out(const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t
 }
 
 // ---- one configuration as fixed shares ---------------------------------------
-// The wave kernel with one block per SM, each running an equal share of the photons
+// The wave kernel with one block per SM (shares_block), each running an equal share of the photons
 // (wave_kernel, SHARES): the same per-photon arithmetic as the history kernels
 // (bit-identical records, equal integer tallies), nothing to set up before it and no
 // state to keep after it.
@@ -1091,6 +1091,25 @@ int shares_fit(const TallyDev& td, int mode, bool& fit) {
   OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   fit = wave_smem(td, mode, false, kSharesBlock) + kSharesStaticSmem <= static_cast<size_t>(max_smem);
   return OPTX_OK;
+}
+
+// Threads per block for n photons. A run of few photons per thread lasts as long as its
+// longest histories, and those step faster the fewer warps share the SM; one of many is
+// bound by issue slots, which want every warp there is room for. Kernel times, FAST
+// tallies, 896 | 768 | 640 | 512 | 384 threads, us: cube 3e4 photons 116 | 116 | 114 |
+// 112 | 110, 2e5 200 | 203 | 193 | 190 | 191, 1e6 281 | 268 | 265 | 255 | 262, 3e6 419 |
+// 411 | 407 | 419 | 451; Lambertian 3e4 51 | 48 | 46 | 45 | 44, 3e5 93 | 91 | 88 | 91 |
+// 95, 1e6 183 | 182 | 187 | 198 | 222, 3e6 441 | 443 | 462 | 499 | 576; bar 3e4 173 |
+// 171 | 167 | 161 | 157, 3e5 280 | 264 | 271 | 266 | 265, 1e6 454 | 443 | 441 | 460 |
+// 510, 1e7 2613 | 2660 | 2781 | 3028 | 3550. (1024 threads, at 64 registers: 1 % less
+// from 1e7 photons on, but up to 6 % more below 1e6.)
+int shares_block(uint64_t n, int sms) {
+  const uint64_t per_sm = n / static_cast<uint64_t>(sms);
+  if (per_sm <= 384u) return 384;        // one photon per thread
+  if (per_sm <= 3u * 512u) return 512;   // up to three
+  if (per_sm <= 6u * 640u) return 640;   // six
+  if (per_sm <= 12u * 768u) return 768;  // twelve
+  return kSharesBlock;
 }
 
 // n <= kSharesMaxPhotons photons, added to `tally` or written to `rec`, async on st.
@@ -1112,11 +1131,12 @@ int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_
   if (rec != nullptr) a.rec = *rec;
   // A claim is a refill; fewer photons than that per warp are spread over the warps.
   const int sms = num_sms();
-  const uint64_t warps = static_cast<uint64_t>(sms) * (kSharesBlock / 32);
+  const int block = shares_block(n, sms);
+  const uint64_t warps = static_cast<uint64_t>(sms) * static_cast<uint64_t>(block / 32);
   a.chunk = static_cast<uint32_t>(std::min<uint64_t>(32u, (n + warps - 1u) / warps));
   a.tail_steps = kNoSpill;
   a.iter_cap = test_fault("watchdog") ? 1u : run_iter_cap(n, 0u, P.max_steps);
-  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, wave_smem(td, mode, false, kSharesBlock), sms, st));
+  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, block, wave_smem(td, mode, false, block), sms, st));
   return OPTX_OK;
 }
 

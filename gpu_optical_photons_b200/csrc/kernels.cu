@@ -1366,20 +1366,20 @@ cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const
 }
 
 template <int MODE>
-static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, size_t smem, int sms,
-                                      cudaStream_t st) {
+static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, int block, size_t smem,
+                                      int sms, cudaStream_t st) {
   const auto fn = wave_kernel<MODE, false, 1, false, true>;
   if (smem > kDynSmemOptIn) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  fn<<<sms, kSharesBlock, smem, st>>>(P, A, ctrl);
+  fn<<<sms, block, smem, st>>>(P, A, ctrl);
   return cudaGetLastError();
 }
-cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, size_t smem, int sms,
-                          cudaStream_t st) {
-  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, ctrl, smem, sms, st)
-                            : launch_shares_mode<kModeRecords>(P, A, ctrl, smem, sms, st);
+cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, int block, size_t smem,
+                          int sms, cudaStream_t st) {
+  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, ctrl, block, smem, sms, st)
+                            : launch_shares_mode<kModeRecords>(P, A, ctrl, block, smem, sms, st);
 }
 
 const void* sorted_prep_fn() { return reinterpret_cast<const void*>(&sorted_prep_kernel); }

@@ -171,7 +171,7 @@ inline __host__ __device__ uint32_t moment_smem_bytes(uint32_t time_bins) {
   return b <= kMomentSmemMaxBytes ? b : 0u;
 }
 
-// Fixed-share launches: one block of 28 warps (72 registers) per SM.
+// Fixed-share launches: one block per SM, of up to 28 warps (72 registers).
 constexpr int kSharesBlock = 896;
 constexpr uint64_t kSharesMaxPhotons = 0xffff0000ull;  // 32-bit cursors, with room to run past the end
 constexpr size_t kSharesStaticSmem = 1024;             // at least the kernel's static shared memory
@@ -249,7 +249,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
                           size_t smem, cudaStream_t st);                                         \
   /* The wave kernel with fixed shares of A.total photons (tally or records mode). */            \
   cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl,      \
-                            size_t smem, int sms, cudaStream_t st);                              \
+                            int block, size_t smem, int sms, cudaStream_t st);                   \
   cudaError_t launch_event_table(const unsigned long long* offsets, uint32_t n_events,           \
                                  uint32_t* table, unsigned long long total, uint32_t shift,      \
                                  cudaStream_t st);                                               \

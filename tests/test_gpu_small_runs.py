@@ -15,7 +15,10 @@ SETUPS = {"cube": P.config1, "lambert": P.config2, "bar": P.config3}
 
 # 8 x 148 x 28 warps x 64 photons = 2,121,728: where claims grow from 32 to 64 photons.
 @pytest.mark.parametrize("setup,n", [("cube", 1), ("cube", 31), ("lambert", 33), ("bar", 1000), ("lambert", 40_001),
-                                     ("lambert", 2_121_727), ("lambert", 2_121_729)])
+                                     ("lambert", 2_121_727), ("lambert", 2_121_729)]
+                         # one configuration's blocks of 384, 512, 640, 768 and 896 threads (148 SMs)
+                         + [("bar", 56_979), ("bar", 56_980), ("cube", 227_475), ("cube", 227_476),
+                            ("lambert", 568_467), ("lambert", 568_468), ("cube", 1_364_115), ("cube", 1_364_116)])
 def test_tally_equals_oracle(engine, oracle, setup, n):
     p = SETUPS[setup]()[0]
     _, flat, _ = engine.run_gpu_tally(p, TC, n, first_id=9, math="exact")
