@@ -1082,9 +1082,13 @@ int records_out(const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t
 // The wave kernel with one block per SM (shares_block), each running an equal share of the photons
 // (wave_kernel, SHARES): the same per-photon arithmetic as the history kernels
 // (bit-identical records, equal integer tallies), nothing to set up before it and no
-// state to keep after it.
+// state to keep after it. Device calls, history kernel at the same sizes | shares:
+// tally of the polished cube 1000 photons 134 | 112 us, 1.5e5 264 | 198; Lambertian 1000
+// 53 | 46, 6e4 74 | 69, 1.5e5 101 | 83; bar 1000 172 | 136, 6e4 235 | 185, 1.5e5 307 |
+// 234, 1e6 951 | 453, 1.6e7 7.97 | 4.1 ms; records the same; one photon: level.
 
-// Whether a tally's histograms fit beside the warps' pantries.
+// Whether a tally's histograms fit beside 28 warps' pantries; the history kernel takes
+// those that do not.
 int shares_fit(const TallyDev& td, int mode, bool& fit) {
   int dev = 0, max_smem = 0;
   OPTX_CUDA(cudaGetDevice(&dev));
@@ -1098,15 +1102,17 @@ int shares_fit(const TallyDev& td, int mode, bool& fit) {
 // bound by issue slots, which want every warp there is room for. Kernel times, FAST
 // tallies, 896 | 768 | 640 | 512 | 384 threads, us: cube 3e4 photons 116 | 116 | 114 |
 // 112 | 110, 2e5 200 | 203 | 193 | 190 | 191, 1e6 281 | 268 | 265 | 255 | 262, 3e6 419 |
-// 411 | 407 | 419 | 451; Lambertian 3e4 51 | 48 | 46 | 45 | 44, 3e5 93 | 91 | 88 | 91 |
-// 95, 1e6 183 | 182 | 187 | 198 | 222, 3e6 441 | 443 | 462 | 499 | 576; bar 3e4 173 |
-// 171 | 167 | 161 | 157, 3e5 280 | 264 | 271 | 266 | 265, 1e6 454 | 443 | 441 | 460 |
-// 510, 1e7 2613 | 2660 | 2781 | 3028 | 3550. (1024 threads, at 64 registers: 1 % less
-// from 1e7 photons on, but up to 6 % more below 1e6.)
+// 411 | 407 | 419 | 451; Lambertian 3e4 51 | 48 | 46 | 45 | 44, 1e5 64 | 63 | 60 | 56 |
+// 58, 3e5 93 | 91 | 88 | 91 | 95, 1e6 183 | 182 | 187 | 198 | 222, 3e6 441 | 443 | 462 |
+// 499 | 576; bar 3e4 173 | 171 | 167 | 161 | 157, 1e5 226 | 214 | 206 | 208 | 202, 3e5
+// 280 | 264 | 271 | 266 | 265, 1e6 454 | 443 | 441 | 460 | 510, 1e7 2613 | 2660 | 2781 |
+// 3028 | 3550. Two blocks of 384 are resident at once, so small device calls overlap on
+// streams (16 calls of 6e4 photons on 4 streams, Lambertian: 439 us, with 512 threads
+// 602). (1024 threads, at 64 registers: 1 % less from 1e7 photons on, but up to 6 % more
+// below 1e6.)
 int shares_block(uint64_t n, int sms) {
   const uint64_t per_sm = n / static_cast<uint64_t>(sms);
-  if (per_sm <= 384u) return 384;        // one photon per thread
-  if (per_sm <= 3u * 512u) return 512;   // up to three
+  if (per_sm <= 3u * 384u) return 384;   // up to three photons per thread
   if (per_sm <= 6u * 640u) return 640;   // six
   if (per_sm <= 12u * 768u) return 768;  // twelve
   return kSharesBlock;
@@ -1130,13 +1136,13 @@ int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_
   a.tc = td;
   if (rec != nullptr) a.rec = *rec;
   // A claim is a refill; fewer photons than that per warp are spread over the warps.
-  const int sms = num_sms();
-  const int block = shares_block(n, sms);
-  const uint64_t warps = static_cast<uint64_t>(sms) * static_cast<uint64_t>(block / 32);
+  const int grid = static_cast<int>(std::max<uint64_t>(1u, std::min<uint64_t>(n, static_cast<uint64_t>(num_sms()))));
+  const int block = shares_block(n, num_sms());
+  const uint64_t warps = static_cast<uint64_t>(grid) * static_cast<uint64_t>(block / 32);
   a.chunk = static_cast<uint32_t>(std::min<uint64_t>(32u, (n + warps - 1u) / warps));
   a.tail_steps = kNoSpill;
   a.iter_cap = test_fault("watchdog") ? 1u : run_iter_cap(n, 0u, P.max_steps);
-  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, block, wave_smem(td, mode, false, block), sms, st));
+  OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, block, wave_smem(td, mode, false, block), grid, st));
   return OPTX_OK;
 }
 
@@ -1430,21 +1436,6 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
 
 }  // extern "C"
 
-// Whether a device call's photons run as fixed shares (run_shares), when that is the
-// faster kernel: with more photons than the history kernel has resident threads
-// (its threads would run several photons each, one after another and emitting on few
-// lanes) and histograms that fit beside 28 warps' pantries. Measured, history kernel
-// against shares: device tally of the bar 1e6 951 | 547 us, 1.6e7 7.97 | 4.44 ms,
-// records of the Lambertian cube 2.5e5 166 | 109 us, 4e6 1.09 | 0.60 ms, tally with
-// 130 KB of histograms 4e6 1.67 | 0.64 ms; with one photon per thread the two are
-// level and the history kernel needs no pantry (cube 6e4 181 | 188 us).
-static int use_shares(int mode, const TallyDev& td, uint64_t n, int blocks_per_sm, int block, bool& use) {
-  use = false;
-  if (n <= static_cast<uint64_t>(std::max(blocks_per_sm, 1)) * block * num_sms() || n > kSharesMaxPhotons)
-    return OPTX_OK;
-  return shares_fit(td, mode, use);
-}
-
 extern "C" {
 
 int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t n,
@@ -1471,15 +1462,8 @@ int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t 
     dd.path += done;
     TallyDev none{};
     none.len = 7u;  // no histograms
-    bool shares = false;
-    OPTX_TRY(use_shares(kModeRecords, none, m, DISPATCH(math, history_records_blocks_per_sm, block_size), block_size,
-                        shares));
-    if (shares)
-      OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &dd, nullptr, math,
-                          static_cast<cudaStream_t>(stream)));
-    else
-      OPTX_CUDA(DISPATCH(math, launch_history_records, P, first_id + done, m, dd, block_size,
-                         static_cast<cudaStream_t>(stream)));
+    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &dd, nullptr, math,
+                        static_cast<cudaStream_t>(stream)));
     done += m;
   }
   return OPTX_OK;
@@ -1504,6 +1488,11 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
                                       " bytes of shared memory; reduce xy_bins / time_bins");
   if (n == 0) return OPTX_OK;
   const DevParams P = make_dev_params(*p, faces);
+  bool fit = false;
+  OPTX_TRY(shares_fit(td, kModeTally, fit));
+  if (fit && n <= kSharesMaxPhotons)
+    return run_shares(kModeTally, P, td, first_id, n, reinterpret_cast<unsigned long long*>(dev_tally), nullptr,
+                      nullptr, math, static_cast<cudaStream_t>(stream));
   const int bps = DISPATCH(math, history_tally_blocks_per_sm, block_size, smem);
   const uint64_t needed = (n + block_size - 1) / block_size;
   const int grid = static_cast<int>(std::max<uint64_t>(
@@ -1511,11 +1500,6 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
                                         num_sms())));
   if (n / grid >= 0xffffffffull)
     return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
-  bool shares = false;
-  OPTX_TRY(use_shares(kModeTally, td, n, bps, block_size, shares));
-  if (shares)
-    return run_shares(kModeTally, P, td, first_id, n, reinterpret_cast<unsigned long long*>(dev_tally), nullptr,
-                      nullptr, math, static_cast<cudaStream_t>(stream));
   OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n,
                      reinterpret_cast<unsigned long long*>(dev_tally), block_size, grid,
                      static_cast<cudaStream_t>(stream)));

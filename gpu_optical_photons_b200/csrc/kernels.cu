@@ -4,11 +4,11 @@
 // OPTX_NS=exact (portable math, -fmad=false) and OPTX_NS=approx (the fast
 // source with --use_fast_math). Kernels:
 //
-//  * history_records_kernel / history_tally_kernel: one thread per photon for
-//    its whole history (a thread runs its photons one after another in one
-//    loop, history_loop), the drop-in for the reference's transport_records_kernel
-//    and transport_tally_kernel (src/gpu/gpu_backend.cu:47-100 of the reference).
-//    The tally keeps fate counts and step sums in registers (no atomics) and the
+//  * history_tally_kernel: one thread per photon for its whole history (a thread
+//    runs its photons one after another in one loop, history_loop), the form of the
+//    reference's transport_tally_kernel (src/gpu/gpu_backend.cu:68-100 of the
+//    reference), for tallies whose histograms leave no room for the wave kernel's
+//    pantries. The tally keeps fate counts and step sums in registers (no atomics) and the
 //    time / hit-map histograms in block-private shared memory, flushed once per
 //    block with 64-bit global atomics: integer sums, so the result does not depend
 //    on the schedule (the property of gpu_backend.cu:68-100 and test_gpu.cpp:122-146).
@@ -118,14 +118,6 @@ __device__ __forceinline__ void history_loop(const DevParams& P, const PhiloxKey
       done(cur, s, fate);
     }
   }
-}
-
-// Blocks of up to 1024 threads (the accepted block sizes): at most 64 registers.
-__global__ void __launch_bounds__(1024, 1) history_records_kernel(const DevParams P, const __grid_constant__ PhiloxKeys K, uint64_t first_id, uint64_t n,
-                                       DevRecords out) {
-  history_loop(P, K, first_id, n, static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x,
-               static_cast<uint64_t>(gridDim.x) * blockDim.x,
-               [&](uint64_t i, const Photon& s, uint32_t fate) { store_record(out, i, s, fate); });
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
@@ -1267,27 +1259,6 @@ __global__ void __launch_bounds__(kSortThreads, MINB)
 // ---------------------------------------------------------------------------
 // Host launchers.
 
-int history_records_blocks_per_sm(int block) {
-  int bps = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, history_records_kernel, block, 0) != cudaSuccess || bps < 1)
-    bps = 1;
-  return bps;
-}
-
-cudaError_t launch_history_records(const DevParams& P, uint64_t first_id, uint64_t n,
-                                   const DevRecords& out, int block, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  // At most one wave of resident blocks: each thread runs several histories.
-  int dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int bps = history_records_blocks_per_sm(block);
-  const uint64_t grid = std::min<uint64_t>((n + block - 1) / block, static_cast<uint64_t>(bps) * sms);
-  history_records_kernel<<<static_cast<unsigned>(grid), block, 0, st>>>(P, philox_keys(P.key_lo, P.key_hi), first_id, n,
-                                                                        out);
-  return cudaGetLastError();
-}
-
 int history_tally_blocks_per_sm(int block, size_t smem) {
   int b = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, history_tally_kernel, block, smem) !=
@@ -1367,19 +1338,19 @@ cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const
 
 template <int MODE>
 static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, int block, size_t smem,
-                                      int sms, cudaStream_t st) {
+                                      int grid, cudaStream_t st) {
   const auto fn = wave_kernel<MODE, false, 1, false, true>;
   if (smem > kDynSmemOptIn) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  fn<<<sms, block, smem, st>>>(P, A, ctrl);
+  fn<<<grid, block, smem, st>>>(P, A, ctrl);
   return cudaGetLastError();
 }
 cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl, int block, size_t smem,
-                          int sms, cudaStream_t st) {
-  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, ctrl, block, smem, sms, st)
-                            : launch_shares_mode<kModeRecords>(P, A, ctrl, block, smem, sms, st);
+                          int grid, cudaStream_t st) {
+  return mode == kModeTally ? launch_shares_mode<kModeTally>(P, A, ctrl, block, smem, grid, st)
+                            : launch_shares_mode<kModeRecords>(P, A, ctrl, block, smem, grid, st);
 }
 
 const void* sorted_prep_fn() { return reinterpret_cast<const void*>(&sorted_prep_kernel); }

@@ -229,13 +229,10 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
 
 #define OPTX_DECLARE_LAUNCHERS(NS)                                                               \
   namespace NS {                                                                                 \
-  cudaError_t launch_history_records(const DevParams& P, uint64_t first_id, uint64_t n,          \
-                                     const DevRecords& out, int block, cudaStream_t st);         \
   cudaError_t launch_history_tally(const DevParams& P, const TallyDev& tc, uint64_t first_id,    \
                                    uint64_t n, unsigned long long* tally, int block, int grid,   \
                                    cudaStream_t st);                                             \
   int history_tally_blocks_per_sm(int block, size_t smem);                                       \
-  int history_records_blocks_per_sm(int block);                                                  \
   /* Wavefront: prep (reset ctrl, zero tallies) and one wave. */                                 \
   cudaError_t launch_wave_prep(const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,           \
                                cudaStream_t st);                                                 \
@@ -249,7 +246,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
                           size_t smem, cudaStream_t st);                                         \
   /* The wave kernel with fixed shares of A.total photons (tally or records mode). */            \
   cudaError_t launch_shares(int mode, const DevParams& P, const WaveArgs& A, WaveCtrl* ctrl,      \
-                            int block, size_t smem, int sms, cudaStream_t st);                   \
+                            int block, size_t smem, int grid, cudaStream_t st);                  \
   cudaError_t launch_event_table(const unsigned long long* offsets, uint32_t n_events,           \
                                  uint32_t* table, unsigned long long total, uint32_t shift,      \
                                  cudaStream_t st);                                               \

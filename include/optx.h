@@ -175,13 +175,15 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
  * optx_sorted_run are written by kernels: the record arrays n_boundary,
  * n_scatter, t, x, y, z, path must be 4-byte aligned and tallies 8-byte
  * aligned, else OPTX_ERR_INVALID_ARGUMENT before any launch. */
-/* Records of n photons into device arrays of n entries (the history kernel, or for
- * many photons the wave kernel with a fixed share of them per warp: the same values). */
+/* Records of n photons into device arrays of n entries: the wave kernel, each block
+ * running an equal share of them. block_size is checked, and sets the blocks of the
+ * history kernel where that one serves a tally. */
 int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t n,
                         uint64_t first_id, const optx_records* dev_out, int block_size, int math,
                         void* stream);
-/* The tally of n photons by the same kernels; ADDS into dev_tally (flat layout as
- * optx_run_tally). */
+/* The tally of n photons by the same kernel (by the history kernel, with the same
+ * result, when the histograms leave no room for it in shared memory or n >= 2^32 -
+ * 65535); ADDS into dev_tally (flat layout as optx_run_tally). */
 int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_tally_config* c,
                       uint64_t n, uint64_t first_id, uint64_t* dev_tally, int block_size, int math,
                       void* stream);

@@ -16,7 +16,8 @@ SETUPS = {"cube": P.config1, "lambert": P.config2, "bar": P.config3}
 # 8 x 148 x 28 warps x 64 photons = 2,121,728: where claims grow from 32 to 64 photons.
 @pytest.mark.parametrize("setup,n", [("cube", 1), ("cube", 31), ("lambert", 33), ("bar", 1000), ("lambert", 40_001),
                                      ("lambert", 2_121_727), ("lambert", 2_121_729)]
-                         # one configuration's blocks of 384, 512, 640, 768 and 896 threads (148 SMs)
+                         # one configuration's blocks of 384, 640, 768 and 896 threads (148 SMs)
+                         + [("bar", 147), ("bar", 148), ("bar", 170_643), ("bar", 170_644)]
                          + [("bar", 56_979), ("bar", 56_980), ("cube", 227_475), ("cube", 227_476),
                             ("lambert", 568_467), ("lambert", 568_468), ("cube", 1_364_115), ("cube", 1_364_116)])
 def test_tally_equals_oracle(engine, oracle, setup, n):
@@ -55,10 +56,9 @@ def test_small_ragged_batch_equals_oracle(engine, oracle, cfg):
     assert np.array_equal(got, oracle.batch_tally(arr, offs, TC, mode=oracle.PORTABLE))
 
 
-# Device calls around the sizes where they go from one photon per thread to fixed
-# shares of a warp (the resident threads of the history kernel), and tallies whose
-# histograms leave the shares no room (150 x 150 bins).
-@pytest.mark.parametrize("n,block,xy", [(1, 256, 10), (130_000, 256, 50), (152_000, 1024, 10), (152_000, 32, 100),
+# Device calls from one photon to several per thread, and tallies whose histograms
+# leave the shares no room (150 x 150 bins).
+@pytest.mark.parametrize("n,block,xy", [(1, 256, 10), (33, 32, 10), (9_473, 256, 50), (1, 256, 150), (9_473, 64, 150), (130_000, 256, 50), (152_000, 1024, 10), (152_000, 32, 100),
                                         (400_003, 256, 50), (400_003, 256, 150)])
 def test_device_calls_equal_oracle(engine, oracle, n, block, xy):
     import torch
