@@ -90,7 +90,7 @@ def parse():
     ap.add_argument("--no-other-math", action="store_true",
                     help="skip timing the same batch in the other two math modes")
     ap.add_argument("--no-history-baseline", action="store_true",
-                    help="skip the plain history-kernel baseline (one launch per event)")
+                    help="skip the baseline of one device call per event")
     ap.add_argument("--no-parity", action="store_true",
                     help="skip the parity check of the benchmarked batch against the reference CPU run")
     ap.add_argument("--no-ksweep", action="store_true",
@@ -304,7 +304,7 @@ def parity_leg(gpu_tallies, cpu_tallies, events, counts, tc, cfg, math: str, k_r
 
 
 def history_baseline(g, events, counts, tc, first_id: int, math: str, stream, reps: int = 2):
-    """The batch as the plain history kernel runs it: one optx_tally_device launch
+    """The batch as one-configuration calls run it: one optx_tally_device launch
     per event, back to back on one stream (the reference's way to process many
     events: one run_gpu_tally each), timed with CUDA events after one warm-up
     pass. Returns (photon-steps/s, ms per pass, tallies of the last pass)."""
@@ -556,7 +556,7 @@ def single_config_legs(math: str, reps: int = 3) -> dict:
     """One configuration at its specified size (single_setups(), tally mode): the
     wavefront engine (host-call settings: 7 blocks of 128 threads), the
     per-interaction sorted kernels (photons queued in HBM by pending
-    interaction, one launch per iteration) and this library's history kernel.
+    interaction, one launch per iteration) and the device call (`history_ms`).
     Median CUDA-event kernel times; the three tallies are checked equal. (The
     reference's own kernels on the same workloads are timed by the reference
     arm, `--impl reference`.)"""
@@ -604,7 +604,7 @@ def single_config_legs(math: str, reps: int = 3) -> dict:
 def ksweep_leg(math: str, n: int = 10_000_000, reps: int = 3) -> dict:
     """The wrapped-Lambertian cube with Rayleigh scattering (1e7 photons, records
     mode) as the reference's event benchmark runs it (apps/optphot_event_bench.cpp:
-    130-143): the history kernel against the wavefront engine with a forced
+    130-143): the device records call (`history_ms`) against the wavefront engine with a forced
     compaction every k steps (k = 1, 4, 8: the reference event kernel's steps
     per launch) and with none (one wave), records checked bit-identical across
     all runs. Median CUDA-event kernel times (host read-back excluded). The
@@ -926,10 +926,10 @@ def run_optx(args):
     if not args.no_history_baseline:
         hv, hms, ht = history_baseline(g, events, counts, tc, first_id, args.math, stream)
         # Same per-photon arithmetic, integer tallies: the two engines agree exactly.
-        assert np.array_equal(ht, tallies), "history and wavefront tallies differ"
+        assert np.array_equal(ht, tallies), "device-call and wavefront tallies differ"
         line["history_baseline"] = {
             "value": world * hv, "unit": UNIT, "ms_per_step": hms, "launches": len(events),
-            "what": "one history-kernel launch (optx_tally_device) per event, back to back on one "
+            "what": "one optx_tally_device launch per event, back to back on one "
                     "stream; identical tallies checked",
             "speedup_of_value": value / (world * hv)}
     if not args.no_ksweep:

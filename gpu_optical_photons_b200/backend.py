@@ -192,7 +192,7 @@ def _crec_from_torch(d) -> _lib.CRecords:
 
 def records_device(p: SimParams, n: int, first_id: int = 0, out=None, block_size: int = 256,
                    math="fast", stream=None):
-    """History kernel into torch device arrays (asynchronous on the stream)."""
+    """Records into torch device arrays (asynchronous on the stream)."""
     out = device_records(n) if out is None else out
     check_records_out(out, n)
     cp, cf = _lib.params_args(p)

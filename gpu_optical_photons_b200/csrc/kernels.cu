@@ -31,8 +31,8 @@
 //    records (events or gensteps) whose photons read their event's physics record
 //    per step; a batch whose events share their step physics (kernel argument).
 //    Batched tallies go through two per-warp shared-memory event slots.
-//    Records depend only on (seed, photon id), so they equal the history
-//    kernel's bit for bit for any block size, threshold, cadence, chunk or wave size.
+//    Records depend only on (seed, photon id), so they are the same, bit for
+//    bit, for any block size, threshold, cadence, chunk or wave size.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
 // photons fill the freed slots, and once nothing is left to emit and fewer than
 // `drain_below` photons are in flight, one last launch runs every remaining photon
 // to its end in place (the fused loop). Records depend only on (seed, photon id),
-// so they equal the history kernel's bit for bit.
+// so they equal the wave kernel's bit for bit.
 
 __device__ __forceinline__ float4 __uint_as_float4(uint4 v) {
   return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),

@@ -109,8 +109,8 @@ __device__ __forceinline__ uint4 philox10(uint4 c, uint32_t k0, uint32_t k1) {
 
 // The same with the round keys of one key made beforehand (philox_keys), in the
 // constant bank: no key additions for the batched kernels, whose photons usually
-// share a key, and for the history kernels (device tally of 1e8 bar photons 43.2 ->
-// 42.0 ms, 10 registers fewer).
+// share a key, and for the history kernel (tally of 1e8 bar photons 43.2 -> 42.0 ms,
+// 10 registers fewer).
 struct PhiloxKeys {
   uint32_t k0[10], k1[10];
 };
@@ -149,7 +149,7 @@ struct Rng {
   // Starts (draws = 0) or resumes the stream of photon `id` after `draws` words
   // (philox.hpp:117-134): blocks draws/4 and draws/4 + 1 fill the window, as two
   // independent Philox chains (instruction-level parallelism: -1 % on the batch,
-  // -3 % on the history kernels).
+  // -3 % on the history kernel).
   template <class K>
   __device__ __forceinline__ void init(uint64_t id, const K& key, uint32_t draws) {
     const uint32_t block = draws >> 2;

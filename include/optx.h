@@ -140,7 +140,7 @@ const char* optx_last_error(void);
 /* Frees the library's cached device / pinned buffers and graphs. */
 int optx_release_cache(void);
 
-/* ---- history kernel, host buffers (the reference's GPU calls) ---------- */
+/* ---- one configuration, host buffers (the reference's GPU calls) ------- */
 /* reference: RunTiming run_gpu_records(const SimParams&, uint64_t n, PhotonRecords&,
  *   int block_size = 256, uint64_t first_id = 0, uint64_t chunk = 1 << 24)
  *   (backend.hpp:88-89; gpu_backend.cu:119-156). `out` holds n entries per array. */
@@ -195,7 +195,7 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
  * scatter, a polished face, a painted face), and each warp of an iteration's
  * launch takes 32 photons of one kind, so the interaction code runs without
  * divergence between kinds. One configuration per run; the records equal the
- * history kernel's (optx_records_device) bit for bit, and the tallies
+ * device call's (optx_records_device) bit for bit, and the tallies
  * optx_tally_device's. */
 typedef struct optx_sorted optx_sorted;
 typedef struct optx_sorted_counters {
