@@ -527,7 +527,8 @@ int engine_grid(optx_engine* e, int mode, int variant, int& grid, int& block) {
   while (block > 32 && wave_smem(e->tdev, mode, batch, block) + fa.sharedSizeBytes > static_cast<size_t>(max_smem))
     block = block / 64 * 32;
   const size_t smem = wave_smem(e->tdev, mode, batch, block);
-  if (smem > kDynSmemOptIn) OPTX_CUDA(DISPATCH(math, wave_set_smem, mode, variant, minb, smem));
+  if (smem > kDynSmemOptIn)
+    OPTX_CUDA(DISPATCH(math, wave_set_smem, mode, variant, minb, static_cast<size_t>(max_smem) - fa.sharedSizeBytes));
   int bps = DISPATCH(math, wave_blocks_per_sm, mode, variant, minb, block, smem);
   if (bps <= 0) return fail(OPTX_ERR_RUNTIME, "wavefront kernel cannot be resident with this block size / tally");
   if (e->cfg.blocks_per_sm == 7) bps = std::min(bps, 7);
@@ -2511,7 +2512,9 @@ extern "C" int optx_wavefront_tally_noalloc(const optx_params* p, const optx_fac
          wave_smem(td, kModeTally, false, block) + fa.sharedSizeBytes > static_cast<size_t>(max_optin))
     block /= 2;
   const size_t smem = wave_smem(td, kModeTally, false, block);
-  if (smem > kDynSmemOptIn) OPTX_CUDA(DISPATCH(math, wave_set_smem, kModeTally, kSingle, kMinB, smem));
+  if (smem > kDynSmemOptIn)
+    OPTX_CUDA(DISPATCH(math, wave_set_smem, kModeTally, kSingle, kMinB,
+                       static_cast<size_t>(max_optin) - fa.sharedSizeBytes));
   const int bps = DISPATCH(math, wave_blocks_per_sm, kModeTally, kSingle, kMinB, block, smem);
   if (bps <= 0)
     return fail(OPTX_ERR_RUNTIME, "tally histograms need too much shared memory; reduce xy_bins / time_bins");

@@ -1272,8 +1272,8 @@ cudaError_t launch_history_tally(const DevParams& P, const TallyDev& tc, uint64_
                                  cudaStream_t st) {
   const size_t smem = static_cast<size_t>(tc.len - 7u) * sizeof(uint32_t);
   if (smem > kDynSmemOptIn) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        history_tally_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = cudaFuncSetAttribute(history_tally_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kSmemPerBlockOptIn));  // it has no static one
     if (e != cudaSuccess) return e;
   }
   history_tally_kernel<<<grid, block, smem, st>>>(P, philox_keys(P.key_lo, P.key_hi), tc, first_id, n, tally);
@@ -1325,9 +1325,9 @@ int wave_blocks_per_sm(int mode, int batch, int minb, int block, size_t smem) {
   return b;
 }
 
-cudaError_t wave_set_smem(int mode, int batch, int minb, size_t smem) {
+cudaError_t wave_set_smem(int mode, int batch, int minb, size_t most) {
   return cudaFuncSetAttribute(wave_kernel_fn(mode, batch, minb),
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
 }
 
 cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P, const WaveArgs& A,
@@ -1341,7 +1341,8 @@ static cudaError_t launch_shares_mode(const DevParams& P, const WaveArgs& A, Wav
                                       int grid, cudaStream_t st) {
   const auto fn = wave_kernel<MODE, false, 1, false, true>;
   if (smem > kDynSmemOptIn) {
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kSmemPerBlockOptIn - kSharesStaticSmem));
     if (e != cudaSuccess) return e;
   }
   fn<<<grid, block, smem, st>>>(P, A, ctrl);

@@ -122,7 +122,11 @@ constexpr uint32_t kLimitBytesPerWarp = 32u * 112u;
 // Dynamic shared memory above this needs the kernel's opt-in attribute: the
 // default limit is 48 KB minus the kernel's static shared memory (at most 1 KB
 // for the kernels here).
+// The attribute is a kernel's, shared by all threads and sizes of launch, so it is
+// always set to the most the kernel can have: set to what one launch needs, it would
+// refuse another thread's larger launch in between.
 constexpr size_t kDynSmemOptIn = 47u * 1024u;
+constexpr size_t kSmemPerBlockOptIn = 227u * 1024u;  // sm_100
 constexpr uint32_t kNoSpill = 0xffffffffu;
 constexpr unsigned kErrQueue = 1u, kErrWatchdog = 2u;
 // Sources beyond this (mm) are not kOrdinary.
@@ -240,7 +244,7 @@ static_assert(sizeof(SortCtrl) <= 1024, "sorted control block");
   /* batch: kSingle, kBatch or kBatchUniform (see WaveVariant) */                               \
   const void* wave_kernel_fn(int mode, int batch, int minb);                                     \
   int wave_blocks_per_sm(int mode, int batch, int minb, int block, size_t smem);                 \
-  cudaError_t wave_set_smem(int mode, int batch, int minb, size_t smem);                         \
+  cudaError_t wave_set_smem(int mode, int batch, int minb, size_t most);                         \
   cudaError_t launch_wave(int mode, int batch, int minb, const DevParams& P,                     \
                           const WaveArgs& A, WaveCtrl* ctrl, int grid, int block,                \
                           size_t smem, cudaStream_t st);                                         \

@@ -88,3 +88,27 @@ def test_device_calls_overlap_on_streams(engine):
     torch.cuda.synchronize()
     for o in outs:
         assert np.array_equal(o.cpu().numpy(), want)
+
+
+def test_device_calls_of_different_sizes_from_threads(engine):
+    """Launches of one kernel with different shared memory (blocks of 384 to 896 threads,
+    different histograms), issued from several threads at once, none refused."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    import torch
+    p = P.config1()[0]
+    jobs = [(n, P.TallyConfig(100, 50.0, xy)) for n in (50_000, 300_000, 900_000, 1_500_000) for xy in (10, 130, 160)]
+    want = [engine.run_gpu_tally(p, c, n, first_id=1, math="fast")[1].astype(np.int64) for n, c in jobs]
+
+    def run(job):
+        n, c = job
+        st, out = torch.cuda.Stream(), torch.zeros(c.length, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(40):
+            engine.tally_device(p, c, n, first_id=1, out=out, stream=st)
+        st.synchronize()
+        return out.cpu().numpy()
+
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        for got, w in zip(pool.map(run, jobs), want):
+            assert np.array_equal(got, 40 * w)
