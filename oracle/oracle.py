@@ -43,7 +43,7 @@ def build(with_ref: bool = True) -> None:
     """Builds the oracle (and the reference backend when its checkout is present)."""
     targets = ["all"]
     ref_dir = reference_root()
-    if with_ref and ref_dir and os.path.isdir(ref_dir):
+    if with_ref and ref_dir and os.path.isdir(os.path.join(ref_dir, "src", "cpu")):
         targets.append("ref")
     env = dict(os.environ)
     if ref_dir:
