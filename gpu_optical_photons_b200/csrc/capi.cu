@@ -1120,6 +1120,7 @@ int shares_block(uint64_t n, int sms) {
 }
 
 // n <= kSharesMaxPhotons photons, added to `tally` or written to `rec`, async on st.
+// ctrl: takes a watchdog's error word, or null for a run without iteration cap.
 int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_id, uint64_t n,
                unsigned long long* tally, const DevRecords* rec, WaveCtrl* ctrl, int math, cudaStream_t st) {
   WaveArgs a;
@@ -1142,7 +1143,7 @@ int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_
   const uint64_t warps = static_cast<uint64_t>(grid) * static_cast<uint64_t>(block / 32);
   a.chunk = static_cast<uint32_t>(std::min<uint64_t>(32u, (n + warps - 1u) / warps));
   a.tail_steps = kNoSpill;
-  a.iter_cap = test_fault("watchdog") ? 1u : run_iter_cap(n, 0u, P.max_steps);
+  a.iter_cap = ctrl == nullptr ? kNoIterCap : (test_fault("watchdog") ? 1u : run_iter_cap(n, 0u, P.max_steps));
   OPTX_CUDA(DISPATCH(math, launch_shares, mode, P, a, ctrl, block, wave_smem(td, mode, false, block), grid, st));
   return OPTX_OK;
 }

@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     const bool had = alive;
     const DevParams& P = params_of<BATCH, UNI>(P0, A, ev);
     const uint64_t id = first_id + pidx;
-    const uint32_t flags = ws.flags, cap = A.iter_cap - iters;
+    const uint32_t flags = ws.flags, cap = A.iter_cap == kNoIterCap ? kNoIterCap : A.iter_cap - iters;
     const bool shared_key = kSharedKey || A.shared_key != 0u;
     auto block = [&](uint32_t b, uint64_t of, const DevParams& Q) {
       const uint4 c = philox_counter(b, of);

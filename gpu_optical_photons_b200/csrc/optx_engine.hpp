@@ -51,7 +51,7 @@ struct WaveArgs {
   double* moments;                      // adjoint mode, optional: (time_bins + 1) x 5 FP64
                                         // per-bin (count, sum S_La, S_Ls, S_R, S_tau)
   unsigned long long graph_handle;      // cudaGraphConditionalHandle of the wave loop
-  uint32_t iter_cap;                    // watchdog: max loop iterations per warp per wave
+  uint32_t iter_cap;                    // watchdog: max loop iterations per warp per wave (kNoIterCap: none)
   uint32_t use_graph;                   // 1: the wave loop is a graph while node (set its condition)
   uint32_t wave_cap;                    // watchdog: max waves per run
   uint32_t chunk;                       // consecutive work items a warp claims per grab (>= 32)
@@ -128,6 +128,9 @@ constexpr uint32_t kLimitBytesPerWarp = 32u * 112u;
 constexpr size_t kDynSmemOptIn = 47u * 1024u;
 constexpr size_t kSmemPerBlockOptIn = 227u * 1024u;  // sm_100
 constexpr uint32_t kNoSpill = 0xffffffffu;
+// WaveArgs::iter_cap of the device calls: they have no error word to report a capped
+// run in, and their histories end at max_steps.
+constexpr uint32_t kNoIterCap = 0xffffffffu;
 constexpr unsigned kErrQueue = 1u, kErrWatchdog = 2u;
 // Sources beyond this (mm) are not kOrdinary.
 constexpr float kFarCoordinate = 0x1p40f;
