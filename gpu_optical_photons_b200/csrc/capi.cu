@@ -217,65 +217,8 @@ int num_sms() {
    : (math) == OPTX_MATH_APPROX ? approx::fn(__VA_ARGS__) \
                                 : fast::fn(__VA_ARGS__))
 
-// ---- cached device buffers (per process; the library serialises calls) ---------
-// g_cache.rec belongs to optx_run_records_event, which holds g_event_mu for its
-// whole call (its engine writes the buffer between its own g_mu sections).
-// Lock order: g_event_mu, g_pipe_mu, a tally workspace's mu, g_mu.
+// Lock order: g_event_mu (event-records calls), g_pipe_mu, a tally workspace's mu, g_mu.
 std::mutex g_event_mu;
-struct Cache {
-  void* rec = nullptr;
-  size_t rec_bytes = 0;
-  unsigned long long* tally = nullptr;
-  size_t tally_bytes = 0;
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-};
-Cache g_cache;
-
-int cache_events() {
-  if (g_cache.e0 == nullptr) {
-    OPTX_CUDA(cudaEventCreate(&g_cache.e0));
-    OPTX_CUDA(cudaEventCreate(&g_cache.e1));
-  }
-  return OPTX_OK;
-}
-
-int cache_records(size_t cap, DevRecords& d) {
-  const size_t bytes = cap * (1 + 4 + 4 + 5 * 4) + 8 * 256;
-  if (g_cache.rec_bytes < bytes) {
-    if (g_cache.rec) cudaFree(g_cache.rec);
-    g_cache.rec = nullptr;
-    g_cache.rec_bytes = 0;
-    OPTX_CUDA(cudaMalloc(&g_cache.rec, bytes));
-    g_cache.rec_bytes = bytes;
-  }
-  auto* base = static_cast<unsigned char*>(g_cache.rec);
-  size_t off = 0;
-  auto take = [&](size_t b) {
-    unsigned char* p = base + off;
-    off += (b + 255) & ~size_t(255);
-    return p;
-  };
-  d.fate = take(cap);
-  d.n_boundary = reinterpret_cast<uint32_t*>(take(cap * 4));
-  d.n_scatter = reinterpret_cast<uint32_t*>(take(cap * 4));
-  d.t = reinterpret_cast<float*>(take(cap * 4));
-  d.x = reinterpret_cast<float*>(take(cap * 4));
-  d.y = reinterpret_cast<float*>(take(cap * 4));
-  d.z = reinterpret_cast<float*>(take(cap * 4));
-  d.path = reinterpret_cast<float*>(take(cap * 4));
-  return OPTX_OK;
-}
-
-int cache_tally(size_t len) {
-  if (g_cache.tally_bytes < len * 8) {
-    if (g_cache.tally) cudaFree(g_cache.tally);
-    g_cache.tally = nullptr;
-    g_cache.tally_bytes = 0;
-    OPTX_CUDA(cudaMalloc(&g_cache.tally, len * 8));
-    g_cache.tally_bytes = len * 8;
-  }
-  return OPTX_OK;
-}
 
 int check_records(const optx_records* r) {
   if (r == nullptr || r->fate == nullptr || r->n_boundary == nullptr || r->n_scatter == nullptr ||
@@ -790,18 +733,55 @@ namespace {
 constexpr uint64_t kPiece = 1ull << 19;
 constexpr int kSlots = 3;                // staging slots: copies in flight ahead of the host
 
+// What the records calls keep on one device: buffer sets, staging slots, streams and
+// events belong to the device that was current when they were made, so a call takes
+// those of its own current device. Guarded by g_pipe_mu.
 struct RecPipe {
+  int device = -1;
   uint64_t cap[2] = {0, 0};   // photons per device buffer set
   uint64_t pin_cap = 0;       // photons per staging slot
   void* dev[2] = {nullptr, nullptr};
   unsigned char* pin[kSlots] = {};
   cudaStream_t comp = nullptr, copy = nullptr;
-  cudaEvent_t k0[2], k1[2], c1[2], done[kSlots];
+  cudaEvent_t k0[2] = {}, k1[2] = {}, c1[2] = {}, done[kSlots] = {};
   unsigned* err = nullptr;  // pinned: the run's error word per buffer set
   WaveCtrl* ctrl = nullptr;  // device: the control blocks they are read from
-  bool events = false;
 };
-RecPipe g_pipe;
+// Not destroyed at exit, when the CUDA runtime may already be gone.
+std::vector<std::unique_ptr<RecPipe>>& g_pipes = *new std::vector<std::unique_ptr<RecPipe>>();
+
+int current_pipe(RecPipe** out) {
+  int dev = 0;
+  OPTX_CUDA(cudaGetDevice(&dev));
+  for (auto& p : g_pipes)
+    if (p->device == dev) {
+      *out = p.get();
+      return OPTX_OK;
+    }
+  g_pipes.push_back(std::make_unique<RecPipe>());
+  g_pipes.back()->device = dev;
+  *out = g_pipes.back().get();
+  return OPTX_OK;
+}
+
+// Frees a pipeline, once the copies left queued by a call that returned an error are
+// through. Streams and events are left alone where that wait fails: their context is
+// gone (a device reset).
+void free_pipe(RecPipe& p) {
+  bool live = true;
+  for (cudaStream_t st : {p.comp, p.copy})
+    if (st != nullptr) live = cudaStreamSynchronize(st) == cudaSuccess && live;
+  for (void* d : p.dev) cudaFree(d);
+  for (unsigned char* h : p.pin) cudaFreeHost(h);
+  cudaFree(p.ctrl);
+  cudaFreeHost(p.err);
+  if (!live) return;
+  for (cudaStream_t st : {p.comp, p.copy})
+    if (st != nullptr) cudaStreamDestroy(st);
+  for (cudaEvent_t e : {p.k0[0], p.k0[1], p.k1[0], p.k1[1], p.c1[0], p.c1[1], p.done[0], p.done[1], p.done[2]})
+    if (e != nullptr) cudaEventDestroy(e);
+}
+static_assert(kSlots == 3, "free_pipe names the slots' events");
 
 // Structure-of-arrays views of one buffer set of `cap` photons (256-B aligned arrays).
 template <class Ptr>
@@ -817,45 +797,51 @@ void carve(unsigned char* base, uint64_t cap, Ptr& fate, Ptr (&w)[7]) {
 }
 size_t set_bytes(uint64_t cap) { return cap + 7 * ((cap * 4 + 255) & ~size_t(255)) + 256; }
 
+// A buffer set of `cap` photons as the kernels' records.
+DevRecords dev_set(const RecPipe& p, int set, uint64_t cap) {
+  unsigned char* fate;
+  unsigned char* w[7];
+  carve(static_cast<unsigned char*>(p.dev[set]), cap, fate, w);
+  return {fate, reinterpret_cast<uint32_t*>(w[0]), reinterpret_cast<uint32_t*>(w[1]), reinterpret_cast<float*>(w[2]),
+          reinterpret_cast<float*>(w[3]), reinterpret_cast<float*>(w[4]), reinterpret_cast<float*>(w[5]),
+          reinterpret_cast<float*>(w[6])};
+}
+
 // Streams and events, and `sets` device buffer sets of `cap` photons.
-int pipe_ensure(int sets, uint64_t cap) {
-  if (!g_pipe.events) {
-    OPTX_CUDA(cudaStreamCreateWithFlags(&g_pipe.comp, cudaStreamNonBlocking));
-    OPTX_CUDA(cudaStreamCreateWithFlags(&g_pipe.copy, cudaStreamNonBlocking));
-    for (int b = 0; b < 2; ++b) {
-      OPTX_CUDA(cudaEventCreate(&g_pipe.k0[b]));
-      OPTX_CUDA(cudaEventCreate(&g_pipe.k1[b]));
-      OPTX_CUDA(cudaEventCreate(&g_pipe.c1[b]));
-    }
-    for (cudaEvent_t& e : g_pipe.done) OPTX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&g_pipe.err), 2 * sizeof(unsigned),
-                            cudaHostAllocDefault));
-    g_pipe.events = true;
-  }
-  if (g_pipe.ctrl == nullptr) OPTX_CUDA(cudaMalloc(&g_pipe.ctrl, 2 * sizeof(WaveCtrl)));
+int pipe_ensure(RecPipe& p, int sets, uint64_t cap) {
+  for (cudaStream_t* st : {&p.comp, &p.copy})
+    if (*st == nullptr) OPTX_CUDA(cudaStreamCreateWithFlags(st, cudaStreamNonBlocking));
+  for (int b = 0; b < 2; ++b)
+    for (cudaEvent_t* e : {&p.k0[b], &p.k1[b], &p.c1[b]})
+      if (*e == nullptr) OPTX_CUDA(cudaEventCreate(e));
+  for (cudaEvent_t& e : p.done)
+    if (e == nullptr) OPTX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (p.err == nullptr)
+    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p.err), 2 * sizeof(unsigned), cudaHostAllocDefault));
+  if (p.ctrl == nullptr) OPTX_CUDA(cudaMalloc(&p.ctrl, 2 * sizeof(WaveCtrl)));
   for (int b = 0; b < sets; ++b) {
-    if (g_pipe.cap[b] >= cap) continue;
-    cudaFree(g_pipe.dev[b]);
-    g_pipe.dev[b] = nullptr;
-    g_pipe.cap[b] = 0;
-    OPTX_CUDA(cudaMalloc(&g_pipe.dev[b], set_bytes(cap)));
-    g_pipe.cap[b] = cap;
+    if (p.cap[b] >= cap) continue;
+    cudaFree(p.dev[b]);
+    p.dev[b] = nullptr;
+    p.cap[b] = 0;
+    OPTX_CUDA(cudaMalloc(&p.dev[b], set_bytes(cap)));
+    p.cap[b] = cap;
   }
   return OPTX_OK;
 }
 
 // Staging slots of `cap` photons, for pageable caller arrays.
-int pipe_ensure_staging(uint64_t cap) {
-  if (g_pipe.pin_cap >= cap) return OPTX_OK;
-  OPTX_CUDA(cudaStreamSynchronize(g_pipe.copy));  // no copy of an earlier, failed call still lands there
-  g_pipe.pin_cap = 0;
-  for (unsigned char*& p : g_pipe.pin) {
-    cudaFreeHost(p);
-    p = nullptr;
+int pipe_ensure_staging(RecPipe& p, uint64_t cap) {
+  if (p.pin_cap >= cap) return OPTX_OK;
+  OPTX_CUDA(cudaStreamSynchronize(p.copy));  // no copy of an earlier, failed call still lands there
+  p.pin_cap = 0;
+  for (unsigned char*& h : p.pin) {
+    cudaFreeHost(h);
+    h = nullptr;
   }
-  for (unsigned char*& p : g_pipe.pin)
-    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), set_bytes(cap), cudaHostAllocDefault));
-  g_pipe.pin_cap = cap;
+  for (unsigned char*& h : p.pin)
+    OPTX_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h), set_bytes(cap), cudaHostAllocDefault));
+  p.pin_cap = cap;
   return OPTX_OK;
 }
 
@@ -1032,17 +1018,17 @@ struct RecordArrays {
     return v;
   }
 };
-int records_out(const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t at, cudaEvent_t ready, cudaEvent_t c1,
-                CopyCrew& crew, PageToucher* touch) {
+int records_out(RecPipe& p, const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t at, cudaEvent_t ready,
+                cudaEvent_t c1, CopyCrew& crew, PageToucher* touch) {
   const void* from[8] = {d.fate, d.n_boundary, d.n_scatter, d.t, d.x, d.y, d.z, d.path};
-  OPTX_CUDA(cudaStreamWaitEvent(g_pipe.copy, ready, 0));
+  OPTX_CUDA(cudaStreamWaitEvent(p.copy, ready, 0));
   const uint64_t piece = a.direct ? m : std::min(m, kPiece);
-  if (!a.direct) OPTX_TRY(pipe_ensure_staging(piece));
+  if (!a.direct) OPTX_TRY(pipe_ensure_staging(p, piece));
   const uint64_t pieces = (m + piece - 1) / piece;
   auto slot = [&](int i) {
     unsigned char* fate;
     unsigned char* w[7];
-    carve(g_pipe.pin[i], g_pipe.pin_cap, fate, w);
+    carve(p.pin[i], p.pin_cap, fate, w);
     return std::array<unsigned char*, 8>{fate, w[0], w[1], w[2], w[3], w[4], w[5], w[6]};
   };
   auto queue = [&](uint64_t j) -> int {
@@ -1053,16 +1039,16 @@ int records_out(const RecordArrays& a, const DevRecords& d, uint64_t m, uint64_t
       const size_t e = RecordArrays::elem(k);
       void* to = a.direct ? static_cast<char*>(a.outs[k]) + (at + lo) * e : static_cast<void*>(pin[k]);
       OPTX_CUDA(cudaMemcpyAsync(to, static_cast<const char*>(from[k]) + lo * e, cnt * e, cudaMemcpyDeviceToHost,
-                                g_pipe.copy));
+                                p.copy));
     }
-    if (!a.direct) OPTX_CUDA(cudaEventRecord(g_pipe.done[j % kSlots], g_pipe.copy));
-    if (j + 1 == pieces) OPTX_CUDA(cudaEventRecord(c1, g_pipe.copy));
+    if (!a.direct) OPTX_CUDA(cudaEventRecord(p.done[j % kSlots], p.copy));
+    if (j + 1 == pieces) OPTX_CUDA(cudaEventRecord(c1, p.copy));
     return OPTX_OK;
   };
   for (uint64_t j = 0; j < std::min<uint64_t>(kSlots, pieces); ++j) OPTX_TRY(queue(j));
   if (!a.direct) {
     for (uint64_t j = 0; j < pieces; ++j) {
-      OPTX_CUDA(cudaEventSynchronize(g_pipe.done[j % kSlots]));
+      OPTX_CUDA(cudaEventSynchronize(p.done[j % kSlots]));
       if (touch != nullptr) touch->join();
       const uint64_t lo = j * piece, cnt = std::min(piece, m - lo);
       const auto pin = slot(static_cast<int>(j % kSlots));
@@ -1148,7 +1134,33 @@ int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_
   return OPTX_OK;
 }
 
-std::mutex g_pipe_mu;  // the records pipeline (g_pipe)
+// The history kernel takes the tallies whose histograms leave no room for the wave
+// kernel's pantries: one wave of resident blocks, each thread running its photons one
+// after another in one loop (history_loop). Measured on B200 at 1e7 photons: 1 wave
+// takes 1-14 % less time than 4 waves with that loop.
+constexpr uint64_t kHistoryGridWaves = 1;
+int history_smem_check(const TallyDev& td) {
+  const size_t smem = static_cast<size_t>(td.len - 7u) * 4u;
+  int dev = 0, max_smem = 0;
+  OPTX_CUDA(cudaGetDevice(&dev));
+  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (smem > static_cast<size_t>(max_smem))
+    return fail(OPTX_ERR_RUNTIME, "tally histograms need " + std::to_string(smem) +
+                                      " bytes of shared memory; reduce xy_bins / time_bins");
+  return OPTX_OK;
+}
+int history_grid(const TallyDev& td, uint64_t n, int block_size, int math, int& grid) {
+  OPTX_TRY(history_smem_check(td));
+  const int bps = DISPATCH(math, history_tally_blocks_per_sm, block_size, static_cast<size_t>(td.len - 7u) * 4u);
+  const uint64_t needed = (n + block_size - 1) / block_size;
+  grid = static_cast<int>(std::max<uint64_t>(
+      1, std::min<uint64_t>(needed, kHistoryGridWaves * static_cast<uint64_t>(std::max(bps, 1)) * num_sms())));
+  if (n / grid >= 0xffffffffull)
+    return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
+  return OPTX_OK;
+}
+
+std::mutex g_pipe_mu;  // the records pipelines (g_pipes)
 
 // Workspace of the host tally calls, one per device: [WaveCtrl][tally] on the device
 // and the pinned copy that comes back in one transfer. A call holds it for its length;
@@ -1235,41 +1247,20 @@ int optx_gpu_device_name(char* buf, size_t len) {
 const char* optx_last_error(void) { return g_err.c_str(); }
 
 int optx_release_cache(void) {
-  // No records call is in flight while g_event_mu (held to the end, so that
-  // g_cache.rec is not in use when it is freed) and g_pipe_mu are held.
+  // No records call is in flight while g_event_mu and g_pipe_mu are held.
   std::lock_guard<std::mutex> elk(g_event_mu);
   free_event_engines();
   std::vector<std::shared_ptr<TallySpace>> spaces;  // destroyed after g_mu, once unused
   {
-    // Copies left queued by a records call that returned an error are drained first.
     std::lock_guard<std::mutex> plk(g_pipe_mu);
-    if (g_pipe.events) {
-      cudaStreamSynchronize(g_pipe.comp);
-      cudaStreamSynchronize(g_pipe.copy);
-    }
-    for (int b = 0; b < 2; ++b) {
-      cudaFree(g_pipe.dev[b]);
-      g_pipe.dev[b] = nullptr;
-      g_pipe.cap[b] = 0;
-    }
-    for (unsigned char*& p : g_pipe.pin) {
-      cudaFreeHost(p);
-      p = nullptr;
-    }
-    g_pipe.pin_cap = 0;
+    for (auto& p : g_pipes) free_pipe(*p);
+    g_pipes.clear();
     delete g_crew;
     g_crew = nullptr;
-    cudaFree(g_pipe.ctrl);
-    g_pipe.ctrl = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
   }
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_cache.rec) cudaFree(g_cache.rec);
-    if (g_cache.tally) cudaFree(g_cache.tally);
-    if (g_cache.e0) cudaEventDestroy(g_cache.e0);
-    if (g_cache.e1) cudaEventDestroy(g_cache.e1);
-    g_cache = Cache{};
     spaces.swap(g_spaces);
     // After a device reset the module is loaded again, possibly elsewhere: the
     // next allocation-free call looks the scratch address up afresh.
@@ -1301,30 +1292,24 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
       1, std::min<uint64_t>({n, chunk ? chunk : (uint64_t{1} << 24), uint64_t{1} << 22}));
   const uint64_t chunks = (n + cap - 1) / cap;
   const auto ta = std::chrono::steady_clock::now();
-  OPTX_TRY(pipe_ensure(chunks > 1 ? 2 : 1, cap));
+  RecPipe* pipe = nullptr;
+  OPTX_TRY(current_pipe(&pipe));
+  OPTX_TRY(pipe_ensure(*pipe, chunks > 1 ? 2 : 1, cap));
   tm.alloc_ms = ms_since(ta);
   TallyDev none{};
   none.len = 7u;  // no histograms
   const RecordArrays arrays(out);
-  auto dev_set = [&](int b) {
-    unsigned char* fate;
-    unsigned char* w[7];
-    carve(static_cast<unsigned char*>(g_pipe.dev[b]), cap, fate, w);
-    return DevRecords{fate, reinterpret_cast<uint32_t*>(w[0]), reinterpret_cast<uint32_t*>(w[1]),
-                      reinterpret_cast<float*>(w[2]), reinterpret_cast<float*>(w[3]), reinterpret_cast<float*>(w[4]),
-                      reinterpret_cast<float*>(w[5]), reinterpret_cast<float*>(w[6])};
-  };
   // Chunk i's kernel into set i % 2, whose previous chunk has been copied out.
   auto launch = [&](uint64_t i) -> int {
     const int b = static_cast<int>(i % 2);
     const uint64_t done = i * cap, m = std::min(cap, n - done);
-    const DevRecords d = dev_set(b);
-    OPTX_CUDA(cudaEventRecord(g_pipe.k0[b], g_pipe.comp));
-    OPTX_CUDA(cudaMemsetAsync(&g_pipe.ctrl[b], 0, sizeof(WaveCtrl), g_pipe.comp));
-    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &d, &g_pipe.ctrl[b], math, g_pipe.comp));
-    OPTX_CUDA(cudaMemcpyAsync(&g_pipe.err[b], &g_pipe.ctrl[b].error, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                              g_pipe.comp));
-    OPTX_CUDA(cudaEventRecord(g_pipe.k1[b], g_pipe.comp));
+    const DevRecords d = dev_set(*pipe, b, cap);
+    OPTX_CUDA(cudaEventRecord(pipe->k0[b], pipe->comp));
+    OPTX_CUDA(cudaMemsetAsync(&pipe->ctrl[b], 0, sizeof(WaveCtrl), pipe->comp));
+    OPTX_TRY(run_shares(kModeRecords, P, none, first_id + done, m, nullptr, &d, &pipe->ctrl[b], math, pipe->comp));
+    OPTX_CUDA(cudaMemcpyAsync(&pipe->err[b], &pipe->ctrl[b].error, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                              pipe->comp));
+    OPTX_CUDA(cudaEventRecord(pipe->k1[b], pipe->comp));
     return OPTX_OK;
   };
   CopyCrew& crew = copy_crew();
@@ -1335,23 +1320,18 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
     const int b = static_cast<int>(i % 2);
     if (i + 1 < chunks) OPTX_TRY(launch(i + 1));  // computes while chunk i is copied out
     const uint64_t done = i * cap, m = std::min(cap, n - done);
-    OPTX_TRY(records_out(arrays, dev_set(b), m, done, g_pipe.k1[b], g_pipe.c1[b], crew, touch.get()));
+    OPTX_TRY(records_out(*pipe, arrays, dev_set(*pipe, b, cap), m, done, pipe->k1[b], pipe->c1[b], crew, touch.get()));
     float ms = 0.f;
-    OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k0[b], g_pipe.k1[b]));
+    OPTX_CUDA(cudaEventElapsedTime(&ms, pipe->k0[b], pipe->k1[b]));
     tm.kernel_ms += ms;
-    OPTX_CUDA(cudaEventElapsedTime(&ms, g_pipe.k1[b], g_pipe.c1[b]));
+    OPTX_CUDA(cudaEventElapsedTime(&ms, pipe->k1[b], pipe->c1[b]));
     tm.d2h_ms += ms;  // kernel end to copy end per chunk (copies overlap later kernels)
-    OPTX_TRY(run_error(g_pipe.err[b]));
+    OPTX_TRY(run_error(pipe->err[b]));
   }
   tm.total_ms = ms_since(t0);
   if (timing) *timing = tm;
   return OPTX_OK;
 }
-
-// History tally grid: one wave of resident blocks, each thread running its
-// photons one after another in one loop (history_loop). Measured on B200 at 1e7
-// photons: 1 wave takes 1-14 % less time than 4 waves with that loop.
-constexpr uint64_t kHistoryGridWaves = 1;
 
 int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tally_config* c,
                    uint64_t n, uint64_t* tally_out, int block_size, uint64_t first_id, int math,
@@ -1367,78 +1347,42 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
   const auto t0 = std::chrono::steady_clock::now();
   bool fit = false;
   OPTX_TRY(shares_fit(td, kModeTally, fit));
+  int grid = 0;  // of the history kernel
+  if (!fit) OPTX_TRY(history_grid(td, n, block_size, math, grid));
+  std::shared_ptr<TallySpace> space;
+  OPTX_TRY(tally_space(space));
+  std::lock_guard<std::mutex> slk(space->mu);
+  OPTX_TRY(tally_space_ensure(*space, td.len));
+  tm.alloc_ms = ms_since(t0);
+  const DevParams P = make_dev_params(*p, faces);
+  const size_t bytes = kTallySpaceHead + 8ull * td.len;
+  auto* ctrl = reinterpret_cast<WaveCtrl*>(space->dev);
+  auto* tally = reinterpret_cast<unsigned long long*>(space->dev + kTallySpaceHead);
+  OPTX_CUDA(cudaMemsetAsync(space->dev, 0, bytes, nullptr));
+  OPTX_CUDA(cudaEventRecord(space->e0, nullptr));
   if (fit) {
-    std::shared_ptr<TallySpace> space;
-    OPTX_TRY(tally_space(space));
-    std::lock_guard<std::mutex> slk(space->mu);
-    OPTX_TRY(tally_space_ensure(*space, td.len));
-    tm.alloc_ms = ms_since(t0);
-    const DevParams P = make_dev_params(*p, faces);
-    const size_t bytes = kTallySpaceHead + 8ull * td.len;
-    auto* ctrl = reinterpret_cast<WaveCtrl*>(space->dev);
-    auto* tally = reinterpret_cast<unsigned long long*>(space->dev + kTallySpaceHead);
-    OPTX_CUDA(cudaMemsetAsync(space->dev, 0, bytes, nullptr));
-    OPTX_CUDA(cudaEventRecord(space->e0, nullptr));
     for (uint64_t done = 0; done < n;) {  // one launch, but for more photons than its cursors count
       const uint64_t m = std::min(n - done, kSharesMaxPhotons);
       OPTX_TRY(run_shares(kModeTally, P, td, first_id + done, m, tally, nullptr, ctrl, math, nullptr));
       done += m;
     }
-    OPTX_CUDA(cudaEventRecord(space->e1, nullptr));
-    const auto tc = std::chrono::steady_clock::now();
-    OPTX_CUDA(cudaMemcpyAsync(space->host, space->dev, bytes, cudaMemcpyDeviceToHost, nullptr));
-    OPTX_CUDA(cudaStreamSynchronize(nullptr));
-    float kms = 0.f;
-    OPTX_CUDA(cudaEventElapsedTime(&kms, space->e0, space->e1));
-    OPTX_TRY(run_error(reinterpret_cast<const WaveCtrl*>(space->host)->error));
-    std::memcpy(tally_out, space->host + kTallySpaceHead, 8ull * td.len);
-    tm.kernel_ms = kms;
-    tm.d2h_ms = ms_since(tc);
-    tm.total_ms = ms_since(t0);
-    if (timing) *timing = tm;
-    return OPTX_OK;
+  } else if (n > 0) {
+    OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n, tally, block_size, grid, nullptr));
   }
-  // The history kernel: the wave kernel's pantries do not fit beside these histograms
-  // in shared memory.
-  std::lock_guard<std::mutex> lk(g_mu);
-  OPTX_TRY(cache_events());
-  const DevParams P = make_dev_params(*p, faces);
-  const size_t smem = static_cast<size_t>(td.len - 7u) * 4u;
-  int dev = 0, max_smem = 0;
-  OPTX_CUDA(cudaGetDevice(&dev));
-  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (smem > static_cast<size_t>(max_smem))
-    return fail(OPTX_ERR_RUNTIME, "tally histograms need " + std::to_string(smem) +
-                                      " bytes of shared memory; reduce xy_bins / time_bins");
-  const int bps = DISPATCH(math, history_tally_blocks_per_sm, block_size, smem);
-  const uint64_t needed = (n + block_size - 1) / block_size;
-  const int grid = static_cast<int>(std::max<uint64_t>(
-      1, std::min<uint64_t>(needed, kHistoryGridWaves * static_cast<uint64_t>(std::max(bps, 1)) *
-                                        num_sms())));
-  if (n / grid >= 0xffffffffull)
-    return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
-  const auto ta = std::chrono::steady_clock::now();
-  OPTX_TRY(cache_tally(td.len));
-  OPTX_CUDA(cudaMemset(g_cache.tally, 0, td.len * 8ull));
-  tm.alloc_ms = ms_since(ta);
-  OPTX_CUDA(cudaEventRecord(g_cache.e0, 0));
-  if (n > 0) OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n, g_cache.tally, block_size, grid, nullptr));
-  OPTX_CUDA(cudaEventRecord(g_cache.e1, 0));
-  OPTX_CUDA(cudaEventSynchronize(g_cache.e1));
-  float ms = 0.f;
-  OPTX_CUDA(cudaEventElapsedTime(&ms, g_cache.e0, g_cache.e1));
-  tm.kernel_ms = ms;
+  OPTX_CUDA(cudaEventRecord(space->e1, nullptr));
   const auto tc = std::chrono::steady_clock::now();
-  OPTX_CUDA(cudaMemcpy(tally_out, g_cache.tally, td.len * 8ull, cudaMemcpyDeviceToHost));
+  OPTX_CUDA(cudaMemcpyAsync(space->host, space->dev, bytes, cudaMemcpyDeviceToHost, nullptr));
+  OPTX_CUDA(cudaStreamSynchronize(nullptr));
+  float kms = 0.f;
+  OPTX_CUDA(cudaEventElapsedTime(&kms, space->e0, space->e1));
+  OPTX_TRY(run_error(reinterpret_cast<const WaveCtrl*>(space->host)->error));
+  std::memcpy(tally_out, space->host + kTallySpaceHead, 8ull * td.len);
+  tm.kernel_ms = kms;
   tm.d2h_ms = ms_since(tc);
   tm.total_ms = ms_since(t0);
   if (timing) *timing = tm;
   return OPTX_OK;
 }
-
-}  // extern "C"
-
-extern "C" {
 
 int optx_records_device(const optx_params* p, const optx_faces* faces, uint64_t n,
                         uint64_t first_id, const optx_records* dev_out, int block_size, int math,
@@ -1481,13 +1425,7 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
   OPTX_TRY(make_tally_dev(c, td));
   OPTX_TRY(check_dev_tally(dev_tally));
   OPTX_TRY(ensure_device());
-  const size_t smem = static_cast<size_t>(td.len - 7u) * 4u;
-  int dev = 0, max_smem = 0;
-  OPTX_CUDA(cudaGetDevice(&dev));
-  OPTX_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (smem > static_cast<size_t>(max_smem))
-    return fail(OPTX_ERR_RUNTIME, "tally histograms need " + std::to_string(smem) +
-                                      " bytes of shared memory; reduce xy_bins / time_bins");
+  OPTX_TRY(history_smem_check(td));
   if (n == 0) return OPTX_OK;
   const DevParams P = make_dev_params(*p, faces);
   bool fit = false;
@@ -1495,13 +1433,8 @@ int optx_tally_device(const optx_params* p, const optx_faces* faces, const optx_
   if (fit && n <= kSharesMaxPhotons)
     return run_shares(kModeTally, P, td, first_id, n, reinterpret_cast<unsigned long long*>(dev_tally), nullptr,
                       nullptr, math, static_cast<cudaStream_t>(stream));
-  const int bps = DISPATCH(math, history_tally_blocks_per_sm, block_size, smem);
-  const uint64_t needed = (n + block_size - 1) / block_size;
-  const int grid = static_cast<int>(std::max<uint64_t>(
-      1, std::min<uint64_t>(needed, kHistoryGridWaves * static_cast<uint64_t>(std::max(bps, 1)) *
-                                        num_sms())));
-  if (n / grid >= 0xffffffffull)
-    return fail(OPTX_ERR_RUNTIME, "too many photons for one tally launch; split the run");
+  int grid = 0;
+  OPTX_TRY(history_grid(td, n, block_size, math, grid));
   OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n,
                      reinterpret_cast<unsigned long long*>(dev_tally), block_size, grid,
                      static_cast<cudaStream_t>(stream)));
@@ -2115,7 +2048,7 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
   OPTX_TRY(check_math(math));
   if (n > 0) OPTX_TRY(check_records(out));
   OPTX_TRY(ensure_device());
-  std::lock_guard<std::mutex> event_lk(g_event_mu);  // g_cache.rec is in use until the end
+  std::lock_guard<std::mutex> event_lk(g_event_mu);
   const auto t0 = std::chrono::steady_clock::now();
   const uint64_t cap = std::max<uint64_t>(1, std::min<uint64_t>({n, chunk ? chunk : (uint64_t{1} << 24), uint64_t{1} << 31}));
   optx_tally_config tc{1u, 1.0f, 1u};
@@ -2141,12 +2074,11 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
   int rc = OPTX_OK;
   if (n > 0) {
     std::lock_guard<std::mutex> pipe_lk(g_pipe_mu);
-    rc = pipe_ensure(0, 0);
+    RecPipe* pipe = nullptr;
     DevRecords d{};
-    if (rc == OPTX_OK) {
-      std::lock_guard<std::mutex> lk(g_mu);
-      rc = cache_records(cap, d);
-    }
+    rc = current_pipe(&pipe);
+    if (rc == OPTX_OK) rc = pipe_ensure(*pipe, 1, cap);
+    if (rc == OPTX_OK) d = dev_set(*pipe, 0, cap);
     CopyCrew& crew = copy_crew();
     std::unique_ptr<PageToucher> touch;
     const RecordArrays arrays(out);
@@ -2164,7 +2096,7 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
       st.spills += s.spills;
       st.kernels_ms += s.kernels_ms;
       const auto tcp = std::chrono::steady_clock::now();
-      rc = records_out(arrays, d, m, done, e->ev1, g_pipe.c1[0], crew, touch.get());
+      rc = records_out(*pipe, arrays, d, m, done, e->ev1, pipe->c1[0], crew, touch.get());
       tm.d2h_ms += ms_since(tcp);
     }
   }

@@ -1,0 +1,109 @@
+// Checks of the library's host code on a fake CUDA runtime (fake_cudart.hpp):
+// `host_check NAME` runs one, prints what is wrong and exits non-zero then. Built and
+// run by tests/test_host_calls.py.
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "../../include/optx.h"
+#include "fake_cudart.hpp"
+
+namespace {
+
+int bad = 0;
+void expect(bool ok, const std::string& what) {
+  if (ok) return;
+  std::printf("%s (%s)\n", what.c_str(), optx_last_error());
+  ++bad;
+}
+
+optx_params cube() {
+  optx_params p{};
+  p.hx = p.hy = p.hz = 25.0f;
+  p.n_scint = 1.63f;
+  p.n_det = 1.5f;
+  p.n_out = 1.0f;
+  p.abs_length = 2000.0f;
+  p.scat_length = 500.0f;
+  p.tau = 4.0f;
+  p.max_steps = 10000;
+  p.seed = 12345;
+  return p;
+}
+
+struct Records {
+  std::vector<uint8_t> fate;
+  std::vector<uint32_t> nb, ns;
+  std::vector<float> t, x, y, z, path;
+  explicit Records(uint64_t n) : fate(n), nb(n), ns(n), t(n), x(n), y(n), z(n), path(n) {}
+  optx_records c() { return {fate.data(), nb.data(), ns.data(), t.data(), x.data(), y.data(), z.data(), path.data()}; }
+  bool right(uint64_t first_id) const {
+    for (uint64_t i = 0; i < fate.size(); ++i) {
+      const uint64_t id = first_id + i;
+      const float f = static_cast<float>(fake::word(id) >> 8);
+      if (fate[i] != fake::fate(id) || nb[i] != fake::word(id) || ns[i] != fake::word(id + 1) || t[i] != f ||
+          x[i] != static_cast<float>((fake::word(id) >> 8) + 1) || path[i] != static_cast<float>((fake::word(id) >> 8) + 4))
+        return false;
+    }
+    return true;
+  }
+};
+
+void records_call(const std::string& what, uint64_t n, uint64_t first_id) {
+  const optx_params p = cube();
+  Records r(n);
+  const optx_records c = r.c();
+  expect(optx_run_records(&p, nullptr, n, &c, 256, first_id, 0, OPTX_MATH_FAST, nullptr) == OPTX_OK, what + ": records");
+  expect(r.right(first_id), what + ": record values");
+}
+void event_call(const std::string& what, uint64_t n, uint64_t first_id, uint32_t k = 8) {
+  const optx_params p = cube();
+  Records r(n);
+  const optx_records c = r.c();
+  expect(optx_run_records_event(&p, nullptr, n, &c, k, 256, first_id, 0, OPTX_MATH_FAST, nullptr, nullptr) == OPTX_OK,
+         what + ": event records");
+  expect(r.right(first_id), what + ": event record values");
+}
+void tally_call(const std::string& what, uint32_t xy) {
+  const optx_params p = cube();
+  const optx_tally_config c{100, 50.0f, xy};
+  std::vector<uint64_t> t(5 + 101 + xy * xy + 2);
+  expect(optx_run_tally(&p, nullptr, &c, 1000, t.data(), 256, 3, OPTX_MATH_FAST, nullptr) == OPTX_OK, what + ": tally");
+  expect(t[0] == 1000, what + ": tally values");
+}
+
+// Host calls made with another current device than earlier ones use that device's own
+// buffers, streams and events.
+void devices() {
+  for (int d : {0, 1, 0, 1}) {
+    fake::current = d;
+    const std::string at = "device " + std::to_string(d);
+    records_call(at, 5000, 77);
+    event_call(at, 5000, 78);
+    tally_call(at, 10);
+    tally_call(at + ", wide", 230);
+  }
+  expect(fake::faults == 0, "launches with another device's memory");
+  optx_release_cache();
+  expect(fake::device_bytes() == 0, "device memory left after optx_release_cache");
+  fake::current = 0;
+  records_call("after the release", 5000, 79);
+}
+
+const struct {
+  const char* name;
+  void (*run)();
+} kChecks[] = {{"devices", devices}};
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  for (const auto& c : kChecks)
+    if (argc == 2 && std::strcmp(argv[1], c.name) == 0) {
+      c.run();
+      return bad != 0;
+    }
+  std::printf("usage: host_check NAME\n");
+  return 2;
+}
