@@ -735,7 +735,7 @@ constexpr int kSlots = 3;                // staging slots: copies in flight ahea
 
 // What the records calls keep on one device: buffer sets, staging slots, streams and
 // events belong to the device that was current when they were made, so a call takes
-// those of its own current device. Guarded by g_pipe_mu.
+// those of its own current device.
 struct RecPipe {
   int device = -1;
   uint64_t cap[2] = {0, 0};   // photons per device buffer set
@@ -747,20 +747,23 @@ struct RecPipe {
   unsigned* err = nullptr;  // pinned: the run's error word per buffer set
   WaveCtrl* ctrl = nullptr;  // device: the control blocks they are read from
 };
-// Not destroyed at exit, when the CUDA runtime may already be gone.
-std::vector<std::unique_ptr<RecPipe>>& g_pipes = *new std::vector<std::unique_ptr<RecPipe>>();
+using RecPipes = std::vector<std::unique_ptr<RecPipe>>;
+// Of optx_run_records, guarded by g_pipe_mu, and of optx_run_records_event, guarded by
+// g_event_mu: calls of the two kinds run side by side. Not destroyed at exit, when the
+// CUDA runtime may already be gone.
+RecPipes &g_pipes = *new RecPipes(), &g_event_pipes = *new RecPipes();
 
-int current_pipe(RecPipe** out) {
+int current_pipe(RecPipes& pipes, RecPipe** out) {
   int dev = 0;
   OPTX_CUDA(cudaGetDevice(&dev));
-  for (auto& p : g_pipes)
+  for (auto& p : pipes)
     if (p->device == dev) {
       *out = p.get();
       return OPTX_OK;
     }
-  g_pipes.push_back(std::make_unique<RecPipe>());
-  g_pipes.back()->device = dev;
-  *out = g_pipes.back().get();
+  pipes.push_back(std::make_unique<RecPipe>());
+  pipes.back()->device = dev;
+  *out = pipes.back().get();
   return OPTX_OK;
 }
 
@@ -877,7 +880,9 @@ class CopyCrew {
     size_t total = 0;
     for (const Job& j : jobs) total += j.bytes;
     size_t n = copy_threads_for(total);
-    if (n > 1 && !tried_) start();
+    if (n == 1) return part(jobs, 0, 1);
+    std::lock_guard<std::mutex> one(use_);  // the helpers do one caller's copy at a time
+    if (!tried_) start();
     n = std::min(n, helpers_.size() + 1);
     if (n > 1) {
       std::lock_guard<std::mutex> lk(mu_);
@@ -936,15 +941,19 @@ class CopyCrew {
     }
   }
   std::vector<std::thread> helpers_;
-  std::mutex mu_;
+  std::mutex use_, mu_;
   std::condition_variable go_, end_;
   const std::vector<Job>* jobs_ = nullptr;
   size_t left_ = 0, parts_ = 0;
   uint64_t round_ = 0;
   bool stop_ = false, tried_ = false;
 };
-CopyCrew* g_crew = nullptr;  // guarded by g_pipe_mu; freed by optx_release_cache, not at exit
+// Freed by optx_release_cache (with g_event_mu and g_pipe_mu held: no call uses it then),
+// not at exit.
+CopyCrew* g_crew = nullptr;
+std::mutex g_crew_mu;
 CopyCrew& copy_crew() {
+  std::lock_guard<std::mutex> lk(g_crew_mu);
   if (g_crew == nullptr) g_crew = new CopyCrew();
   return *g_crew;
 }
@@ -1160,7 +1169,7 @@ int history_grid(const TallyDev& td, uint64_t n, int block_size, int math, int& 
   return OPTX_OK;
 }
 
-std::mutex g_pipe_mu;  // the records pipelines (g_pipes)
+std::mutex g_pipe_mu;  // records calls (g_pipes)
 
 // Workspace of the host tally calls, one per device: [WaveCtrl][tally] on the device
 // and the pinned copy that comes back in one transfer. A call holds it for its length;
@@ -1253,8 +1262,10 @@ int optx_release_cache(void) {
   std::vector<std::shared_ptr<TallySpace>> spaces;  // destroyed after g_mu, once unused
   {
     std::lock_guard<std::mutex> plk(g_pipe_mu);
-    for (auto& p : g_pipes) free_pipe(*p);
-    g_pipes.clear();
+    for (RecPipes* pipes : {&g_pipes, &g_event_pipes}) {
+      for (auto& p : *pipes) free_pipe(*p);
+      pipes->clear();
+    }
     delete g_crew;
     g_crew = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
@@ -1293,7 +1304,7 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
   const uint64_t chunks = (n + cap - 1) / cap;
   const auto ta = std::chrono::steady_clock::now();
   RecPipe* pipe = nullptr;
-  OPTX_TRY(current_pipe(&pipe));
+  OPTX_TRY(current_pipe(g_pipes, &pipe));
   OPTX_TRY(pipe_ensure(*pipe, chunks > 1 ? 2 : 1, cap));
   tm.alloc_ms = ms_since(ta);
   TallyDev none{};
@@ -2073,10 +2084,9 @@ int optx_run_records_event(const optx_params* p, const optx_faces* faces, uint64
   optx_event_stats st{};
   int rc = OPTX_OK;
   if (n > 0) {
-    std::lock_guard<std::mutex> pipe_lk(g_pipe_mu);
     RecPipe* pipe = nullptr;
     DevRecords d{};
-    rc = current_pipe(&pipe);
+    rc = current_pipe(g_event_pipes, &pipe);
     if (rc == OPTX_OK) rc = pipe_ensure(*pipe, 1, cap);
     if (rc == OPTX_OK) d = dev_set(*pipe, 0, cap);
     CopyCrew& crew = copy_crew();

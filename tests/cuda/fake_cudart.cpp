@@ -332,7 +332,7 @@ namespace optx {
     const DevRecords& r = a.rec;                                                                                      \
     const cudaError_t e = launchable(st, {c, a.tally, r.fate, r.n_boundary, r.n_scatter, r.t, r.x, r.y, r.z, r.path}); \
     if (e != cudaSuccess) return e;                                                                                   \
-    if (on_shares) on_shares();                                                                                       \
+    if (const auto f = on_shares) f();                                                                                \
     if (r.fate != nullptr) write_records(r, a.first_id, 0, a.total);                                                  \
     if (a.tally != nullptr) a.tally[0] += a.total;                                                                    \
     return cudaSuccess;                                                                                               \

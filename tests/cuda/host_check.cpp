@@ -1,9 +1,12 @@
 // Checks of the library's host code on a fake CUDA runtime (fake_cudart.hpp):
 // `host_check NAME` runs one, prints what is wrong and exits non-zero then. Built and
 // run by tests/test_host_calls.py.
+#include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/optx.h"
@@ -91,10 +94,31 @@ void devices() {
   records_call("after the release", 5000, 79);
 }
 
+// A records call and an event-records call on two threads do not wait for each other.
+void overlap() {
+  std::promise<void> started, event_done;
+  bool waited = false;
+  std::future<void> done = event_done.get_future();
+  fake::on_shares = [&] {  // the records call's kernel, under way until the event call is through
+    fake::on_shares = nullptr;
+    started.set_value();
+    waited = done.wait_for(std::chrono::seconds(5)) == std::future_status::timeout;
+  };
+  std::thread records([] { records_call("thread", 1200000, 5); });
+  started.get_future().wait();
+  event_call("main", 1200000, 9);  // large enough for the copy helpers, which both use
+  event_done.set_value();
+  records.join();
+  expect(!waited, "the event-records call waited for the records call");
+  std::thread again([] { records_call("thread", 1200000, 6); });
+  event_call("main", 1200000, 10);
+  again.join();
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}};
 
 }  // namespace
 
