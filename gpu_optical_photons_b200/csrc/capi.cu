@@ -410,9 +410,8 @@ struct optx_engine {
     int batch;  // WaveVariant
     int grid, block;
     size_t smem;
-    DevParams P0;
-    WaveArgs args;  // graph_handle and use_graph zero
     cudaGraph_t graph;
+    cudaGraphNode_t prep, wave;
     cudaGraphExec_t exec;
     cudaGraphConditionalHandle handle;
   };
@@ -571,17 +570,41 @@ WaveArgs engine_args(const optx_engine* e, int mode, int warps, const DevRecords
   return a;
 }
 
+// The graph of a run that may take several waves, with the run's parameters in its
+// kernel nodes: prep (reset the control block, zero the tallies), then
+// while (active) { wave }. One executable graph serves all runs of a mode and variant;
+// a run sets its parameters on it (runs already queued keep theirs), 1 us, where
+// instantiating a graph for new photons, seeds or pointers took 0.25 ms a run (batch of
+// 256 events, 5e5 photons, in waves of at least 64 steps: 0.62 ms with new ids, 0.36 with
+// the same).
 int engine_graph(optx_engine* e, int mode, int batch, int grid, int block, const WaveArgs& args,
                  optx_engine::Graph** out) {
   const size_t smem = wave_smem(e->tdev, mode, batch != kSingle, block);
-  const DevParams P0 = batch == kBatch ? DevParams{} : e->P0;
+  const int math = e->cfg.math;
+  DevParams P0 = batch == kBatch ? DevParams{} : e->P0;
+  WaveArgs a = args;
+  a.use_graph = 1u;
+  WaveCtrl* c_ptr = e->d_ctrl;
+  void* prep_args[] = {&a, &c_ptr};
+  cudaKernelNodeParams kp{};
+  kp.func = const_cast<void*>(DISPATCH(math, wave_prep_fn));
+  kp.gridDim = dim3(std::max(1, std::min(grid, 4 * e->n_sm)));
+  kp.blockDim = dim3(256);
+  kp.kernelParams = prep_args;
+  void* wave_args[] = {&P0, &a, &c_ptr};
+  cudaKernelNodeParams wp{};
+  wp.func = const_cast<void*>(DISPATCH(math, wave_kernel_fn, mode, batch, engine_minb(e)));
+  wp.gridDim = dim3(grid);
+  wp.blockDim = dim3(block);
+  wp.sharedMemBytes = static_cast<unsigned>(smem);
+  wp.kernelParams = wave_args;
   for (auto& g : e->graphs) {
-    if (g.mode == mode && g.batch == batch && g.grid == grid && g.block == block &&
-        g.smem == smem && std::memcmp(&g.P0, &P0, sizeof(P0)) == 0 &&
-        std::memcmp(&g.args, &args, sizeof(args)) == 0) {
-      *out = &g;
-      return OPTX_OK;
-    }
+    if (g.mode != mode || g.batch != batch || g.grid != grid || g.block != block || g.smem != smem) continue;
+    a.graph_handle = g.handle;
+    OPTX_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, g.prep, &kp));
+    OPTX_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, g.wave, &wp));
+    *out = &g;
+    return OPTX_OK;
   }
   optx_engine::Graph g{};
   g.mode = mode;
@@ -589,49 +612,19 @@ int engine_graph(optx_engine* e, int mode, int batch, int grid, int block, const
   g.grid = grid;
   g.block = block;
   g.smem = smem;
-  g.P0 = P0;
-  g.args = args;
-  const int math = e->cfg.math;
   OPTX_CUDA(cudaGraphCreate(&g.graph, 0));
   OPTX_CUDA(cudaGraphConditionalHandleCreate(&g.handle, g.graph, 1u, cudaGraphCondAssignDefault));
-  WaveArgs a = args;
   a.graph_handle = g.handle;
-  a.use_graph = 1u;
-
-  // prep: reset the control block, zero the tallies
-  cudaKernelNodeParams kp{};
-  WaveCtrl* c_ptr = e->d_ctrl;
-  void* prep_args[] = {&a, &c_ptr};
-  kp.func = const_cast<void*>(DISPATCH(math, wave_prep_fn));
-  kp.gridDim = dim3(std::max(1, std::min(grid, 4 * e->n_sm)));
-  kp.blockDim = dim3(256);
-  kp.sharedMemBytes = 0;
-  kp.kernelParams = prep_args;
-  cudaGraphNode_t n_prep;
-  OPTX_CUDA(cudaGraphAddKernelNode(&n_prep, g.graph, nullptr, 0, &kp));
-
-  // while (active) { wave }
+  OPTX_CUDA(cudaGraphAddKernelNode(&g.prep, g.graph, nullptr, 0, &kp));
   cudaGraphNodeParams cp{};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = g.handle;
   cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
   cudaGraphNode_t n_while;
-  OPTX_CUDA(cudaGraphAddNode(&n_while, g.graph, &n_prep, 1, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-
-  DevParams p_copy = P0;
-  void* wave_args[] = {&p_copy, &a, &c_ptr};
-  cudaKernelNodeParams wp{};
-  wp.func = const_cast<void*>(DISPATCH(math, wave_kernel_fn, mode, batch, engine_minb(e)));
-  wp.gridDim = dim3(grid);
-  wp.blockDim = dim3(block);
-  wp.sharedMemBytes = static_cast<unsigned>(smem);
-  wp.kernelParams = wave_args;
-  cudaGraphNode_t n_wave;
-  OPTX_CUDA(cudaGraphAddKernelNode(&n_wave, body, nullptr, 0, &wp));
+  OPTX_CUDA(cudaGraphAddNode(&n_while, g.graph, &g.prep, 1, &cp));
+  OPTX_CUDA(cudaGraphAddKernelNode(&g.wave, cp.conditional.phGraph_out[0], nullptr, 0, &wp));
   OPTX_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
-  // A graph bakes its run's arguments in; keep a few.
   constexpr size_t kMaxGraphs = 8;
   if (e->graphs.size() >= kMaxGraphs) {
     cudaGraphExecDestroy(e->graphs.front().exec);

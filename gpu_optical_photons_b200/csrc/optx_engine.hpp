@@ -21,7 +21,7 @@ struct TallyDev {
 
 // Wavefront run description, a kernel parameter: the kernels read it through the
 // constant bank (from device memory each use was a dependent load, and each run an
-// upload), and a graph holds the arguments that it was made for.
+// upload).
 struct WaveArgs {
   const DevParams* params;              // records: events, or gensteps (1 entry when not batched)
   const DevParams* phys;                // physics per event (= params unless gensteps)

@@ -115,10 +115,44 @@ void overlap() {
   again.join();
 }
 
+// An engine that runs in several waves makes one graph, whatever its runs cover, and
+// each run is launched with its own parameters.
+void graphs() {
+  const optx_tally_config tc{100, 50.0f, 10};
+  optx_wave_config cfg{};
+  cfg.cadence = 8;
+  optx_engine* e = nullptr;
+  expect(optx_engine_create(&tc, 4, 100000, &cfg, &e) == OPTX_OK, "create");
+  std::vector<optx_params> ev(4, cube());
+  for (uint32_t i = 0; i < 20; ++i) {
+    for (uint32_t k = 0; k < 4; ++k) ev[k].seed = 100 * i + k, ev[k].abs_length = 100.0f + static_cast<float>(i + k);
+    const std::vector<uint64_t> counts{100 + i, 7, 0, 1000 - i};
+    expect(optx_engine_set_events(e, ev.data(), nullptr, counts.data(), 4, 1000 * i, nullptr) == OPTX_OK, "upload");
+    expect(optx_engine_run_tally(e, nullptr) == OPTX_OK, "run");
+    const optx::WaveArgs& a = fake::runs.back().args;
+    expect(fake::runs.size() == 2 * i + 1 && a.first_id == 1000 * i && a.item_lo == 0 && a.total == 1107 && a.keep_tally == 0,
+           "a run's arguments");
+    expect(optx_engine_run_tally_range(e, 50, 60 + i, 1, nullptr) == OPTX_OK, "range");
+    const optx::WaveArgs& r = fake::runs.back().args;
+    expect(r.item_lo == 50 && r.total == 60 + i && r.keep_tally == 1, "a range's arguments");
+  }
+  expect(fake::instantiations == 1, "graphs of the batch: " + std::to_string(fake::instantiations));
+  for (uint32_t i = 0; i < 20; ++i) {  // one configuration: the physics is a parameter too
+    optx_params p = cube();
+    p.seed = i;
+    const uint64_t n = 500 + i;
+    expect(optx_engine_set_events(e, &p, nullptr, &n, 1, i, nullptr) == OPTX_OK, "upload");
+    expect(optx_engine_run_tally(e, nullptr) == OPTX_OK, "run");
+    expect(fake::runs.back().p0.key_lo == i && fake::runs.back().args.total == n, "a run's physics");
+  }
+  expect(fake::instantiations == 2, "graphs: " + std::to_string(fake::instantiations));
+  optx_engine_destroy(e);
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}};
 
 }  // namespace
 
