@@ -1991,8 +1991,8 @@ namespace {
 
 // Engines of the event-records calls, kept from call to call: creating one (queues,
 // tables, its graph of the forced-compaction loop) and freeing it took 2.5 ms of a 4 ms
-// call of 3e5 photons. At most kEventEngines, the newest, none with queues above
-// kEventQueueBytes; guarded by g_event_mu; freed by optx_release_cache.
+// call of 3e5 photons. At most kEventEngines, the newest, with queues of at most
+// kEventQueueBytes together; guarded by g_event_mu; freed by optx_release_cache.
 struct EventEngine {
   int device, math, block;
   uint32_t threshold, cadence;
@@ -2025,7 +2025,11 @@ void give_event_engine(optx_engine* e, bool keep) {
     optx_engine_destroy(e);
     return;
   }
-  if (g_event_engines.size() >= kEventEngines) {
+  const auto queue_bytes = [](const optx_engine* x) { return 128ull * x->qcap; };
+  uint64_t total = queue_bytes(e);
+  for (const EventEngine& k : g_event_engines) total += queue_bytes(k.e);
+  while (!g_event_engines.empty() && (g_event_engines.size() >= kEventEngines || total > kEventQueueBytes)) {
+    total -= queue_bytes(g_event_engines.front().e);
     optx_engine_destroy(g_event_engines.front().e);
     g_event_engines.erase(g_event_engines.begin());
   }

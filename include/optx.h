@@ -137,7 +137,10 @@ int optx_gpu_available(void);
 /* reference: std::string gpu_device_name() (backend.hpp:85) */
 int optx_gpu_device_name(char* buf, size_t len);
 const char* optx_last_error(void);
-/* Frees the library's cached device / pinned buffers and graphs. */
+/* Frees what the library keeps between calls: the device and pinned buffers of the host
+ * calls (sized for the largest so far), the engines of optx_run_records_event (at most
+ * four, with queues of at most 256 MB together) with their graphs, and the helper
+ * threads of the copies into pageable arrays (at most seven). */
 int optx_release_cache(void);
 
 /* ---- one configuration, host buffers (the reference's GPU calls) ------- */

@@ -149,10 +149,23 @@ void graphs() {
   optx_engine_destroy(e);
 }
 
+// What event-records calls of several kinds keep on the device stays bounded.
+void kept() {
+  constexpr uint64_t n = 2000000;
+  for (uint32_t k : {2, 4, 8, 16, 32}) {
+    event_call("cadence " + std::to_string(k), n, k, k);
+    // 256 MB of queues, the call's 29 bytes per photon, and a few MB of tables
+    expect(fake::device_bytes() <= (256ull << 20) + 30 * n + (4ull << 20),
+           "device memory kept: " + std::to_string(fake::device_bytes() >> 20) + " MB");
+  }
+  optx_release_cache();
+  expect(fake::device_bytes() == 0, "device memory left after optx_release_cache");
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}};
 
 }  // namespace
 
