@@ -2003,7 +2003,18 @@ std::vector<EventEngine>& g_event_engines = *new std::vector<EventEngine>();  //
 constexpr size_t kEventEngines = 4;
 constexpr uint64_t kEventQueueBytes = 256ull << 20;
 
-int take_event_engine(const optx_tally_config& tc, const optx_wave_config& cfg, uint64_t cap, optx_engine** out) {
+// Photons that an engine for calls of `cap` holds: the next power of two from 2^16 on, so
+// that calls of similar sizes use one engine, where its queues may be kept at all; a
+// larger one is made to measure. Records and statistics do not depend on it: the queues
+// hold all photons of the call either way, up to the 2^23 that they hold at most.
+uint64_t event_capacity(uint64_t cap) {
+  uint64_t c = 1ull << 16;
+  while (c < cap) c <<= 1;
+  return 128ull * c <= kEventQueueBytes ? c : cap;
+}
+
+int take_event_engine(const optx_tally_config& tc, const optx_wave_config& cfg, uint64_t photons, optx_engine** out) {
+  const uint64_t cap = event_capacity(photons);
   int dev = 0;
   OPTX_CUDA(cudaGetDevice(&dev));
   for (size_t i = 0; i < g_event_engines.size(); ++i) {
@@ -2015,7 +2026,8 @@ int take_event_engine(const optx_tally_config& tc, const optx_wave_config& cfg, 
       return OPTX_OK;
     }
   }
-  return optx_engine_create(&tc, 1, cap, &cfg, out);
+  const int rc = optx_engine_create(&tc, 1, cap, &cfg, out);
+  return rc == OPTX_ERR_CUDA && cap != photons ? optx_engine_create(&tc, 1, photons, &cfg, out) : rc;
 }
 
 // Keeps the engine for the next call, or frees it (after an error, or a large one).

@@ -162,10 +162,18 @@ void kept() {
   expect(fake::device_bytes() == 0, "device memory left after optx_release_cache");
 }
 
+// Event-records calls of similar sizes use one kept engine.
+void sizes() {
+  event_call("first", 130000, 1);
+  const int before = fake::mallocs;
+  for (uint64_t n : {129999, 120001, 100000, 70007}) event_call("size " + std::to_string(n), n, n);
+  expect(fake::mallocs == before, "allocations by calls of other sizes: " + std::to_string(fake::mallocs - before));
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}};
 
 }  // namespace
 
