@@ -981,14 +981,17 @@ class PageToucher {
     for (auto& r : ranges)
       res += static_cast<size_t>(resident_fraction(r.first, r.second, page) * static_cast<double>(r.second));
     if (res * 2 >= total) return;
-    for (unsigned t = 0; t < hw; ++t) {
-      th_.emplace_back([ranges, t, hw, page] {
-        for (auto& r : ranges) {
-          volatile char* q = static_cast<volatile char*>(r.first);
-          const size_t lo = r.second * t / hw, hi = r.second * (t + 1) / hw;
-          for (size_t off = lo; off < hi; off += page) q[off] = 0;
-        }
-      });
+    try {
+      for (unsigned t = 0; t < hw; ++t) {
+        th_.emplace_back([ranges, t, hw, page] {
+          for (auto& r : ranges) {
+            volatile char* q = static_cast<volatile char*>(r.first);
+            const size_t lo = r.second * t / hw, hi = r.second * (t + 1) / hw;
+            for (size_t off = lo; off < hi; off += page) q[off] = 0;
+          }
+        });
+      }
+    } catch (const std::exception&) {  // no more threads: the other pages fault in during the copies
     }
   }
   void join() {

@@ -1,6 +1,7 @@
 // Checks of the library's host code on a fake CUDA runtime (fake_cudart.hpp):
 // `host_check NAME` runs one, prints what is wrong and exits non-zero then. Built and
 // run by tests/test_host_calls.py.
+#include <cerrno>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -9,10 +10,16 @@
 #include <thread>
 #include <vector>
 
+#include <dlfcn.h>
+#include <pthread.h>
+#include <sys/mman.h>
+
 #include "../../include/optx.h"
 #include "fake_cudart.hpp"
 
 namespace {
+
+bool threads_fail = false;  // pthread_create (below) refuses
 
 int bad = 0;
 void expect(bool ok, const std::string& what) {
@@ -170,12 +177,37 @@ void sizes() {
   expect(fake::mallocs == before, "allocations by calls of other sizes: " + std::to_string(fake::mallocs - before));
 }
 
+// Records calls into fresh pages where no thread can be started: as with them, slower.
+void threads() {
+  constexpr uint64_t n = 1000000;
+  threads_fail = true;
+  for (bool event : {true, false}) {
+    std::vector<void*> a;
+    for (int k = 0; k < 8; ++k)
+      a.push_back(mmap(nullptr, (k ? 4 : 1) * n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+    const auto f = [&](int k) { return static_cast<float*>(a[static_cast<size_t>(k)]); };
+    const optx_records c{static_cast<uint8_t*>(a[0]), static_cast<uint32_t*>(a[1]), static_cast<uint32_t*>(a[2]), f(3), f(4),
+                         f(5), f(6), f(7)};
+    const optx_params p = cube();
+    expect((event ? optx_run_records_event(&p, nullptr, n, &c, 8, 256, 3, 0, OPTX_MATH_FAST, nullptr, nullptr)
+                  : optx_run_records(&p, nullptr, n, &c, 256, 3, 0, OPTX_MATH_FAST, nullptr)) == OPTX_OK, "records");
+    for (uint64_t i = 0; i < n; ++i)
+      if (c.fate[i] != fake::fate(3 + i) || c.n_scatter[i] != fake::word(4 + i)) return expect(false, "record values");
+  }
+  threads_fail = false;
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}};
 
 }  // namespace
+
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* attr, void* (*run)(void*), void* arg) noexcept {
+  static const auto real = reinterpret_cast<decltype(&pthread_create)>(dlsym(RTLD_NEXT, "pthread_create"));
+  return threads_fail ? EAGAIN : real(t, attr, run, arg);
+}
 
 int main(int argc, char** argv) {
   for (const auto& c : kChecks)
