@@ -891,6 +891,8 @@ class CopyCrew {
       end_.wait(lk, [&] { return left_ == 0; });
     }
   }
+  // A forked child has its parent's crew without the threads: nothing to end or join.
+  bool forked() const { return owner_ != getpid(); }
   ~CopyCrew() {
     {
       std::lock_guard<std::mutex> lk(mu_);
@@ -933,6 +935,7 @@ class CopyCrew {
     } catch (const std::exception&) {  // no more threads: those that started do the copies
     }
   }
+  const pid_t owner_ = getpid();
   std::vector<std::thread> helpers_;
   std::mutex use_, mu_;
   std::condition_variable go_, end_;
@@ -1262,7 +1265,7 @@ int optx_release_cache(void) {
       for (auto& p : *pipes) free_pipe(*p);
       pipes->clear();
     }
-    delete g_crew;
+    if (g_crew != nullptr && !g_crew->forked()) delete g_crew;
     g_crew = nullptr;
     cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
   }

@@ -13,6 +13,8 @@
 #include <dlfcn.h>
 #include <pthread.h>
 #include <sys/mman.h>
+#include <sys/wait.h>
+#include <unistd.h>
 
 #include "../../include/optx.h"
 #include "fake_cudart.hpp"
@@ -197,10 +199,26 @@ void threads() {
   threads_fail = false;
 }
 
+// optx_release_cache in a forked child returns, although the copies' helper threads are
+// its parent's.
+void forked() {
+  records_call("parent", 1200000, 5);
+  const pid_t child = fork();
+  if (child == 0) {
+    alarm(10);
+    _exit(optx_release_cache());
+  }
+  int status = 0;
+  waitpid(child, &status, 0);
+  expect(WIFEXITED(status) && WEXITSTATUS(status) == 0, "the child's release");
+  records_call("parent", 1200000, 6);
+  optx_release_cache();
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}};
 
 }  // namespace
 
