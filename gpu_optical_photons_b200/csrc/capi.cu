@@ -1267,7 +1267,6 @@ int optx_release_cache(void) {
     }
     if (g_crew != nullptr && !g_crew->forked()) delete g_crew;
     g_crew = nullptr;
-    cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
   }
   {
     std::lock_guard<std::mutex> lk(g_mu);
@@ -1277,6 +1276,7 @@ int optx_release_cache(void) {
     noalloc_forget_addresses();
   }
   spaces.clear();  // one still used by a call is destroyed when that call ends
+  cudaGetLastError();  // release reports nothing; a stale error must not reach the next call
   return OPTX_OK;
 }
 

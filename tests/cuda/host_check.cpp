@@ -215,10 +215,25 @@ void forked() {
   optx_release_cache();
 }
 
+// A release whose frees fail (after a device reset) leaves no error behind: launches ask
+// for the last one and would report it.
+void stale() {
+  records_call("before", 5000, 1);
+  event_call("before", 5000, 2);
+  tally_call("before", 10);
+  fake::frees_fail = true;
+  expect(optx_release_cache() == OPTX_OK, "release");
+  fake::frees_fail = false;
+  expect(!fake::stale_error(), "the release left an error");
+  records_call("after", 5000, 3);
+  event_call("after", 5000, 4);
+  tally_call("after", 10);
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}, {"stale", stale}};
 
 }  // namespace
 
