@@ -421,11 +421,10 @@ struct optx_engine {
 namespace {
 
 // Dynamic shared memory of a block of `block` threads: its warps', then the block's
-// histograms (tally) or bin weights and moment table (adjoint).
+// histograms (tally) or moment table (score moments).
 size_t wave_extra(const TallyDev& t, int mode, bool batch) {
   if (mode == kModeTally) return batch ? 0u : static_cast<size_t>(t.len - 7u) * 4u;
-  if (mode == kModeAdjoint || mode == kModeMoments)
-    return static_cast<size_t>(t.time_bins + 1u) * 8u + (mode == kModeMoments ? moment_smem_bytes(t.time_bins) : 0u);
+  if (mode == kModeMoments) return moment_smem_bytes(t.time_bins);
   return 0u;
 }
 size_t wave_smem(const TallyDev& t, int mode, bool batch, int block) {
@@ -433,11 +432,13 @@ size_t wave_smem(const TallyDev& t, int mode, bool batch, int block) {
          wave_extra(t, mode, batch);
 }
 // What counts against the device's shared memory per block when a tally is accepted
-// or refused (kLimitBytesPerWarp).
+// or refused (kLimitBytesPerWarp; replays count their bin weights, which were staged
+// in shared memory).
 size_t wave_smem_limit(const TallyDev& t, int mode, bool batch, int block) {
   const size_t fixed = (mode == kModeTally ? 96u : (mode == kModeRecords ? 80u : 608u)) + (batch ? (mode == kModeTally ? 272u : 256u) : 0u);
   const size_t slots = mode == kModeTally && batch ? kSlotCounterBytesPerWarp + slot_bin_bytes_per_warp(t.len - 7u) : 0u;
-  return static_cast<size_t>(block / 32) * (kLimitBytesPerWarp + slots) + wave_extra(t, mode, batch) + fixed;
+  const size_t weights = mode == kModeAdjoint || mode == kModeMoments ? static_cast<size_t>(t.time_bins + 1u) * 8u : 0u;
+  return static_cast<size_t>(block / 32) * (kLimitBytesPerWarp + slots) + wave_extra(t, mode, batch) + weights + fixed;
 }
 
 // Register-budget variant of the wave kernel: 2, 3 or 4 blocks of 256 threads

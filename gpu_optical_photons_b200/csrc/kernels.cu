@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   const uint32_t nwarps = blockDim.x >> 5;
   // [per warp (wave_warp_bytes): ring windows | pantry | batched: bookkeeping | batched
   //  tally: 2 x 8 u32 slot counters, then 2 x n_bins u32 bins when n_bins <=
-  //  kSlotBins][block histograms (tally), bin weights (adjoint)]
+  //  kSlotBins][block histograms (tally), moment table (score moments, if moments_smem)]
   constexpr bool kSlots = BATCH && MODE == kModeTally;
   constexpr bool kAdj = MODE == kModeAdjoint || MODE == kModeMoments;  // replay modes
   constexpr bool kLaneCounts = MODE == kModeTally && !BATCH;
@@ -321,8 +321,7 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
   uint32_t* s_book = reinterpret_cast<uint32_t*>(pantry + 32u * kEntry);
   unsigned char* extra = smem_raw + nwarps * warp_bytes;
   uint32_t* s_hist = reinterpret_cast<uint32_t*>(extra);
-  double* s_w = reinterpret_cast<double*>(extra);
-  double* s_mom = s_w + (A.tc.time_bins + 1u);  // adjoint, moments_smem: [time_bins + 1][5]
+  double* s_mom = reinterpret_cast<double*>(extra);  // [time_bins + 1][5]
   uint32_t* s_evc = s_book + kBookWords;
   __shared__ double s_red[4][16];
 
@@ -378,12 +377,8 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
       for (uint32_t b = lane; b < 2u * n_bins; b += 32u) s_sb[b] = 0u;
     }
   }
-  if (kAdj) {
-    const double* wb = A.w_bin;
-    for (uint32_t b = threadIdx.x; b <= tc.time_bins; b += blockDim.x) s_w[b] = wb ? wb[b] : 0.0;
-    if (MODE == kModeMoments && A.moments_smem) {
-      for (uint32_t i = threadIdx.x; i < 5u * (tc.time_bins + 1u); i += blockDim.x) s_mom[i] = 0.0;
-    }
+  if (MODE == kModeMoments && A.moments_smem) {
+    for (uint32_t i = threadIdx.x; i < 5u * (tc.time_bins + 1u); i += blockDim.x) s_mom[i] = 0.0;
   }
   __syncthreads();
 
@@ -505,7 +500,9 @@ __global__ void __launch_bounds__(wave_max_threads<MINB>(), MINB)
     } else {  // adjoint: score terms of detected photons (see WaveArgs)
       if (fate == kDetected) {
         const uint32_t tb = time_bin(s.t, tc.tscale, tc.time_bins);
-        const double w = s_w[tb] + A.w_det;
+        // From device memory: staged in shared memory, the weights of a long window left
+        // the warps no room.
+        const double w = (A.w_bin != nullptr ? __ldg(A.w_bin + tb) : 0.0) + A.w_det;
         double* M = MODE == kModeMoments ? A.moments : nullptr;
         if (w != 0.0 || M != nullptr) {
           const double path = s.path;
