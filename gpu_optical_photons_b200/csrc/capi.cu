@@ -1148,6 +1148,11 @@ int run_shares(int mode, const DevParams& P, const TallyDev& td, uint64_t first_
 // after another in one loop (history_loop). Measured on B200 at 1e7 photons: 1 wave
 // takes 1-14 % less time than 4 waves with that loop.
 constexpr uint64_t kHistoryGridWaves = 1;
+// The host call's blocks have at least this many threads: one block per SM is resident
+// beside such histograms, so a smaller one leaves the SM idle. Host calls, 184 x 184
+// bins, blocks of 32 | 64 | 128 | 256 threads, ms: Lambertian cube 3e6 photons 7.4 | 3.9 |
+// 2.1 | 1.3, 3e5 1.06 | 0.64 | 0.41 | 0.31; polished cube 3e6 5.2 | 3.0 | 1.8 | 1.3.
+constexpr int kHostHistoryBlock = 256;
 int history_smem_check(const TallyDev& td) {
   const size_t smem = static_cast<size_t>(td.len - 7u) * 4u;
   int dev = 0, max_smem = 0;
@@ -1359,7 +1364,8 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
   bool fit = false;
   OPTX_TRY(shares_fit(td, kModeTally, fit));
   int grid = 0;  // of the history kernel
-  if (!fit) OPTX_TRY(history_grid(td, n, block_size, math, grid));
+  const int block = std::max(block_size, kHostHistoryBlock);
+  if (!fit) OPTX_TRY(history_grid(td, n, block, math, grid));
   std::shared_ptr<TallySpace> space;
   OPTX_TRY(tally_space(space));
   std::lock_guard<std::mutex> slk(space->mu);
@@ -1378,7 +1384,7 @@ int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tal
       done += m;
     }
   } else if (n > 0) {
-    OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n, tally, block_size, grid, nullptr));
+    OPTX_CUDA(DISPATCH(math, launch_history_tally, P, td, first_id, n, tally, block, grid, nullptr));
   }
   OPTX_CUDA(cudaEventRecord(space->e1, nullptr));
   const auto tc = std::chrono::steady_clock::now();

@@ -18,7 +18,7 @@ namespace fake {
 int devices = 2;
 thread_local int current = 0;
 bool frees_fail = false;
-int faults = 0, mallocs = 0, instantiations = 0;
+int faults = 0, mallocs = 0, instantiations = 0, history_block = 0;
 std::function<void()> on_shares;
 std::vector<Run> runs;
 
@@ -313,7 +313,8 @@ namespace optx {
   namespace NS {                                                                                                      \
   int history_tally_blocks_per_sm(int, size_t) { return 1; }                                                          \
   cudaError_t launch_history_tally(const DevParams&, const TallyDev&, uint64_t, uint64_t n, unsigned long long* t,    \
-                                   int, int, cudaStream_t st) {                                                       \
+                                   int block, int, cudaStream_t st) {                                                 \
+    history_block = block;                                                                                            \
     const cudaError_t e = launchable(st, {t});                                                                        \
     if (e == cudaSuccess) t[0] += n;                                                                                  \
     return e;                                                                                                         \

@@ -19,6 +19,7 @@ extern thread_local int current;    // the calling thread's current device
 extern bool frees_fail;             // cudaFree and friends fail, as after a device reset
 extern int faults;                  // launches given another device's memory
 extern int mallocs, instantiations; // calls so far
+extern int history_block;           // threads per block of the last history_tally_kernel
 size_t device_bytes();              // device memory allocated now
 bool stale_error();                 // what the next cudaGetLastError would return is an error
 

@@ -77,11 +77,11 @@ void event_call(const std::string& what, uint64_t n, uint64_t first_id, uint32_t
          what + ": event records");
   expect(r.right(first_id), what + ": event record values");
 }
-void tally_call(const std::string& what, uint32_t xy) {
+void tally_call(const std::string& what, uint32_t xy, int block = 256) {
   const optx_params p = cube();
   const optx_tally_config c{100, 50.0f, xy};
   std::vector<uint64_t> t(5 + 101 + xy * xy + 2);
-  expect(optx_run_tally(&p, nullptr, &c, 1000, t.data(), 256, 3, OPTX_MATH_FAST, nullptr) == OPTX_OK, what + ": tally");
+  expect(optx_run_tally(&p, nullptr, &c, 1000, t.data(), block, 3, OPTX_MATH_FAST, nullptr) == OPTX_OK, what + ": tally");
   expect(t[0] == 1000, what + ": tally values");
 }
 
@@ -230,10 +230,18 @@ void stale() {
   tally_call("after", 10);
 }
 
+// Host tallies with wide histograms fill the SMs whatever block size is asked for.
+void wide_blocks() {
+  for (int block : {32, 64, 128, 256, 512, 1024}) {
+    tally_call("block " + std::to_string(block), 200, block);
+    expect(fake::history_block >= 256 && fake::history_block >= block, "threads: " + std::to_string(fake::history_block));
+  }
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}, {"stale", stale}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}, {"stale", stale}, {"wide_blocks", wide_blocks}};
 
 }  // namespace
 

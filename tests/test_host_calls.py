@@ -14,12 +14,14 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 def host_check(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("host") / "host_check")
     src = [os.path.join(HERE, "cuda", f) for f in ("host_check.cpp", "fake_cudart.cpp")]
-    subprocess.run([B.nvcc()] + B.ARCH + ["-O1", "-std=c++17", "-cudart", "none", "-x", "cu", "-I", B.CSRC, "-I", B.INCLUDE]
+    subprocess.run([B.nvcc()] + B.ARCH + ["-O1", "-std=c++17", "-cudart", "none", "-x", "cu", "-I", B.CSRC,
+                                          "-I", B.INCLUDE]
                    + src + [os.path.join(B.CSRC, "capi.cu"), "-o", exe, "-lpthread", "-ldl"], check=True)
     return exe
 
 
-@pytest.mark.parametrize("check", ["devices", "overlap", "graphs", "kept", "sizes", "threads", "forked", "stale"])
+@pytest.mark.parametrize("check", ["devices", "overlap", "graphs", "kept", "sizes", "threads", "forked", "stale",
+                                   "wide_blocks"])
 def test_host_code(host_check, check):
     out = subprocess.run([host_check, check], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
