@@ -238,10 +238,35 @@ void wide_blocks() {
   }
 }
 
+// Which tallies run the history kernel: histograms that do not fit beside 28 warps'
+// pantries (100 time bins: from 184 x 184 hit-map bins on), and device calls of more
+// photons than the wave kernel's cursors count.
+void routes() {
+  const optx_params p = cube();
+  uint64_t* t = nullptr;
+  expect(cudaMalloc(reinterpret_cast<void**>(&t), 8 * 60000) == cudaSuccess, "malloc");
+  const auto device = [&](uint32_t xy, uint64_t n) {
+    const optx_tally_config c{100, 50.0f, xy};
+    fake::history_block = 0;
+    t[0] = 0;
+    expect(optx_tally_device(&p, nullptr, &c, n, 0, t, 64, OPTX_MATH_FAST, nullptr) == OPTX_OK && t[0] == n, "device tally");
+    return fake::history_block == 64;
+  };
+  for (uint32_t xy : {10, 170, 183, 184, 200, 236}) {
+    fake::history_block = 0;
+    tally_call(std::to_string(xy) + " bins", xy);
+    expect((fake::history_block != 0) == (xy >= 184), "route of the host tally, " + std::to_string(xy));
+    expect(device(xy, 1000) == (xy >= 184), "route of the device tally, " + std::to_string(xy));
+  }
+  expect(!device(10, optx::kSharesMaxPhotons), "route of 2^32 - 65536 photons");
+  expect(device(10, optx::kSharesMaxPhotons + 1), "route of 2^32 - 65535 photons");
+  cudaFree(t);
+}
+
 const struct {
   const char* name;
   void (*run)();
-} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}, {"stale", stale}, {"wide_blocks", wide_blocks}};
+} kChecks[] = {{"devices", devices}, {"overlap", overlap}, {"graphs", graphs}, {"kept", kept}, {"sizes", sizes}, {"threads", threads}, {"forked", forked}, {"stale", stale}, {"wide_blocks", wide_blocks}, {"routes", routes}};
 
 }  // namespace
 

@@ -21,7 +21,7 @@ def host_check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("check", ["devices", "overlap", "graphs", "kept", "sizes", "threads", "forked", "stale",
-                                   "wide_blocks"])
+                                   "wide_blocks", "routes"])
 def test_host_code(host_check, check):
     out = subprocess.run([host_check, check], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
