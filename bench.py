@@ -5,7 +5,7 @@ to [1e2, 1e6]; 66,481,565 photons, ~2.8e8 photon-steps), per-event absorption
 length, reflectivity, refractive index and scattering length, point sources
 uniform in a 50 mm cube, Lambertian faces, per-event tallies (100 arrival-time
 bins over 0-50 ns + overflow, 10x10 hit map). A step is one run of the whole
-batch: one CUDA-graph launch of the persistent wavefront engine.
+batch: one run of the persistent wavefront engine (two launches).
 
   value  photon-steps/s with the event table resident on the device
   e2e    photon-steps/s through the C ABI call optx_run_batch with pinned host
@@ -94,7 +94,7 @@ def parse():
     ap.add_argument("--no-parity", action="store_true",
                     help="skip the parity check of the benchmarked batch against the reference CPU run")
     ap.add_argument("--no-ksweep", action="store_true",
-                    help="skip the history vs forced-compaction (k = 1, 4, 8) records leg")
+                    help="skip the one-launch vs forced-compaction (k = 1, 4, 8) records leg")
     ap.add_argument("--no-reference-gpu", action="store_true",
                     help="reference arm: skip the reference's own GPU kernels (CPU value only)")
     ap.add_argument("--events", type=int, default=4096)
@@ -554,7 +554,7 @@ def _ev_ms(fn, reps: int) -> float:
 
 def single_config_legs(math: str, reps: int = 3) -> dict:
     """One configuration at its specified size (single_setups(), tally mode): the
-    wavefront engine (host-call settings: 7 blocks of 128 threads), the
+    wavefront engine (7 blocks of 128 threads per SM), the
     per-interaction sorted kernels (photons queued in HBM by pending
     interaction, one launch per iteration) and the device call (`history_ms`).
     Median CUDA-event kernel times; the three tallies are checked equal. (The

@@ -1,7 +1,8 @@
 """Command-line runner (the role of the reference's apps/optphot_main.cpp and
-apps/optphot_event_bench.cpp): runs one configuration through the history or
-the wavefront kernel (or the per-interaction sorted kernels, or gensteps through
-the wavefront engine) and prints a JSON line with timings and tallies summary.
+apps/optphot_event_bench.cpp): runs one configuration through the library's host
+calls (`history`, the reference's names) or the wavefront engine (or the
+per-interaction sorted kernels, or gensteps through the wavefront engine) and
+prints a JSON line with timings and tallies summary.
 
     python -m gpu_optical_photons_b200.cli --config config2 --engine wave --n 1e7
     python -m gpu_optical_photons_b200.cli --config config2 --engine sorted --n 1e7

@@ -1,11 +1,11 @@
 """The wavefront engine (optx_engine_* of include/optx.h) and batched events.
 
 A ``WavefrontEngine`` owns its device state queues, control block, per-event
-tallies and captured CUDA graphs. ``set_events`` uploads a batch (one or
-thousands of events with their own SimParams and photon counts); the run is
-a prep kernel and one persistent wave kernel, or, where it may need several
-waves, one graph launch with a device-side while loop of them. Event i owns photon ids ``first_id + offset_i + k``, so each
-event reproduces the reference's ``run_cpu_*(p_i, n_i, ..., first_id=offset_i)``.
+tallies and CUDA graphs. ``set_events`` uploads a batch (one or thousands of
+events with their own SimParams and photon counts); the run is a prep kernel and
+one persistent wave kernel, or, where it may need several waves, one graph launch
+with a device-side while loop of them. Event i owns photon ids ``first_id +
+offset_i + k``, so each event reproduces the reference's ``run_cpu_*(p_i, n_i, ..., first_id=offset_i)``.
 """
 from __future__ import annotations
 
@@ -153,7 +153,7 @@ class WavefrontEngine:
         self.counts = None  # known on the device only
 
     def run_gensteps(self, events, gensteps, first_id: int = 0):
-        """One-shot host-buffer genstep run: upload, graph launch, D2H per-event tallies."""
+        """One-shot host-buffer genstep run: upload, run, D2H per-event tallies."""
         from .gensteps import as_gensteps
         arr, faces = _events_c(events)
         g = as_gensteps(gensteps)
@@ -211,7 +211,7 @@ class WavefrontEngine:
         return st.as_dict()
 
     def run_batch(self, events, counts, first_id: int = 0):
-        """One-shot host-buffer run: H2D table, graph launch, D2H tallies."""
+        """One-shot host-buffer run: H2D table, run, D2H tallies."""
         arr, faces = _events_c(events)
         cnt = _counts_c(counts, len(arr))
         out = np.zeros((len(events), self.tally_config.length), np.uint64)

@@ -155,7 +155,8 @@ int optx_run_records(const optx_params* p, const optx_faces* faces, uint64_t n,
  *   gpu_backend.cu:158-212). tally_out: flat u64 array of
  *   5 + time_bins + 1 + xy_bins^2 + 2 entries = [fate counts | arrival-time histogram
  *   (last bin overflow) | hit map, row-major iy*xy_bins+ix | sum n_boundary | sum n_scatter];
- *   it is overwritten. */
+ *   it is overwritten. Where the history kernel serves it (see optx_tally_device) its
+ *   blocks have block_size threads, at least 256. */
 int optx_run_tally(const optx_params* p, const optx_faces* faces, const optx_tally_config* c,
                    uint64_t n, uint64_t* tally_out, int block_size, uint64_t first_id, int math,
                    optx_timing* timing);
@@ -237,7 +238,7 @@ int optx_sorted_run(optx_sorted* s, const optx_params* p, const optx_faces* face
  * OPTX_ERR_WATCHDOG when the run failed. */
 int optx_sorted_stats(optx_sorted* s, optx_sorted_counters* stats, void* stream);
 
-/* ---- wavefront engine (extension: persistent, graph-captured, batched) -- */
+/* ---- wavefront engine (extension: persistent, batched) ------------------ */
 typedef struct optx_engine optx_engine;
 /* An engine for up to max_events events and max_photons photons per run. The
  * tally layout is per event as in optx_run_tally. */
@@ -341,15 +342,15 @@ int optx_engine_tally_ptr(optx_engine* e, uint64_t** dev_ptr, uint64_t* len_per_
 int optx_engine_get_tallies(optx_engine* e, uint64_t* host_out, void* stream);
 /* Statistics of the last run (synchronises `stream`). */
 int optx_engine_stats(optx_engine* e, optx_event_stats* stats, void* stream);
-/* One-shot batched run with host buffers: H2D of the event table, one graph
- * launch, D2H of the per-event tallies (host_tallies: n_events x tally length),
+/* One-shot batched run with host buffers: H2D of the event table, the run,
+ * D2H of the per-event tallies (host_tallies: n_events x tally length),
  * with one wait for the run. On an error return host_tallies is unspecified. */
 int optx_run_batch(optx_engine* e, const optx_params* events, const optx_faces* faces,
                    const uint64_t* counts, uint32_t n_events, uint64_t first_id,
                    uint64_t* host_tallies, optx_event_stats* stats, optx_timing* timing);
 
-/* One-shot genstep run with host buffers (extension): set_gensteps, one graph
- * launch, D2H of the per-event tallies (host_tallies: n_events x tally length),
+/* One-shot genstep run with host buffers (extension): set_gensteps, the run,
+ * D2H of the per-event tallies (host_tallies: n_events x tally length),
  * with one wait for the run. On an error return host_tallies is unspecified. */
 int optx_run_gensteps(optx_engine* e, const optx_params* events, const optx_faces* faces,
                       uint32_t n_events, const optx_genstep* gensteps, uint32_t n_gensteps,

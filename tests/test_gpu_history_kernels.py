@@ -1,12 +1,10 @@
-"""The plain history kernels themselves against the oracle and the reference's
-golden outputs, through the device calls that launch them and nothing else:
-optx_records_device (history_records_kernel, one thread per photon, the drop-in
-for the reference's transport_records_kernel, src/gpu/gpu_backend.cu:47-52) and
-optx_tally_device (history_tally_kernel, the drop-in for transport_tally_kernel,
-gpu_backend.cu:56-100). The host calls optx_run_records / optx_run_tally run the
-wavefront engine, so these are the only tests that pin the history kernels
-without going through another GPU path. Modelled on the reference's
-tests/test_gpu.cpp:77-146."""
+"""The device calls against the oracle and the reference's golden outputs:
+optx_records_device (the drop-in for the reference's transport_records_kernel,
+src/gpu/gpu_backend.cu:47-52) and optx_tally_device (the drop-in for
+transport_tally_kernel, gpu_backend.cu:56-100). The names here date from the
+history kernels that these calls launched; every call in this file now runs the
+wave kernel. history_tally_kernel, which serves wider histograms, is pinned by
+test_gpu_wide_tallies.py. Modelled on the reference's tests/test_gpu.cpp:77-146."""
 import numpy as np
 import pytest
 
@@ -33,7 +31,7 @@ PARITY = {
 
 
 def history_records(engine, p, n, first_id, math, block_size=256):
-    """history_records_kernel only: optx_records_device into device arrays."""
+    """optx_records_device into device arrays."""
     import torch
     d = engine.records_device(p, n, first_id=first_id, math=math, block_size=block_size)
     torch.cuda.synchronize()
@@ -41,7 +39,7 @@ def history_records(engine, p, n, first_id, math, block_size=256):
 
 
 def history_tally(engine, p, c, n, first_id, math, block_size=256):
-    """history_tally_kernel only: optx_tally_device into a zeroed device tally."""
+    """optx_tally_device into a zeroed device tally."""
     t = engine.tally_device(p, c, n, first_id=first_id, math=math, block_size=block_size)
     return t.cpu().numpy().astype(np.uint64)
 

@@ -56,8 +56,8 @@ def test_small_ragged_batch_equals_oracle(engine, oracle, cfg):
     assert np.array_equal(got, oracle.batch_tally(arr, offs, TC, mode=oracle.PORTABLE))
 
 
-# Device calls from one photon to several per thread, and tallies whose histograms
-# leave the shares no room (150 x 150 bins).
+# Device calls from one photon to several per thread (tallies whose histograms leave the
+# wave kernel no room: test_gpu_wide_tallies.py).
 @pytest.mark.parametrize("n,block,xy", [(1, 256, 10), (33, 32, 10), (9_473, 256, 50), (1, 256, 150), (9_473, 64, 150), (130_000, 256, 50), (152_000, 1024, 10), (152_000, 32, 100),
                                         (400_003, 256, 50), (400_003, 256, 150)])
 def test_device_calls_equal_oracle(engine, oracle, n, block, xy):
